@@ -8,17 +8,22 @@
 //     BRDF of getRadiance (cudaGather.cu:84-90) is paid once per AVPL instead of once per pair.
 //   * The receiver's Lambertian BRDF is constant per pixel and is applied once in the epilogue.
 //   * A block owns a 16 x (16*PX) pixel tile; AVPL records are staged chunk by chunk into shared
-//     memory with bulk asynchronous copies (cp.async.bulk, no multicast) on an mbarrier ring and
-//     read back as broadcast 128-bit loads, each reused for PX pixels per thread.
+//     memory with bulk asynchronous copies (cp.async.bulk, no multicast) on an mbarrier.
+//   * The default and the all-FP64 precision (no or cone antiradiance) test each staged record once
+//     against the tile's bounds and evaluate only the records that can add something to it
+//     (gather_bf_culled_kernel, pair_cull.cuh); the other precisions and the disk variant evaluate
+//     every pair (gather_bf_kernel).
 //   * Radiance and antiradiance go to separate compensated sums (per-chunk FP32 partials folded
 //     into Kahan sums, or per-term Kahan) and are combined in FP64.
 // General path (specular materials or geometry-term limits): one thread per pixel evaluating the
 // full f_r on both sides of every pair.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
 #include "arc_internal.h"
 #include "device_common.cuh"
+#include "pair_cull.cuh"
 #include "pair_math.cuh"
 
 namespace arc {
@@ -57,9 +62,9 @@ struct BfArgs {
     uint32_t* err;
     // general path (raw SoA)
     ArcAvplsGpuParam soa;
-    // packed path over a compacted pixel list (nullptr: rectangular tiles)
-    const int* pixel_list;
-    const int* pixel_count;
+    // culled path: the AVPLs split over gridDim.z segments, each block's sums of one segment here
+    // (NULL with one segment): [tile][segment][6][pixels of a tile]
+    double* partial;
 };
 
 // ---------------------------------------------------------------------------------------
@@ -102,21 +107,6 @@ __global__ void pack_bf_records(ArcAvplsGpuParam a, const MaterialRecord* mats, 
     d[1] = r[1];
     d[2] = r[2];
     d[3] = r[3];
-}
-
-// The same records interleaved by AVPL pair: float pair * 32 + 2 f + h holds field f of AVPL
-// 2 pair + h; an odd count is padded with a zero record (it contributes exactly 0).
-__global__ void pack_bf_pairs(ArcAvplsGpuParam a, const MaterialRecord* mats, int32_t num_mats, float* rec,
-                              uint32_t* err) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.numAvpls + (a.numAvpls & 1)) return;
-    float4 r[4] = {make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0),
-                   make_float4(0, 0, 0, 0)};
-    if (i < a.numAvpls) bf_record(a, mats, num_mats, i, err, r);
-    const float* f = reinterpret_cast<const float*>(r);
-    float* d = rec + (i >> 1) * 32 + (i & 1);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) d[2 * q] = f[q];
 }
 
 // PREC: 0 = chunk partials folded into Kahan sums, 1 = per-term Kahan, 2 = naive FP32, 3 = FP64.
@@ -314,239 +304,332 @@ __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
     }
 }
 
-// Surface pixels of the G-buffer, compacted into a list (order within a warp arbitrary), for the
-// list form of the packed kernel; every other pixel gets here the outputs the gather gives a pixel
-// without a surface (0, w = 1).  Bad material indices are reported as the gather kernels do.
-__global__ void bf_compact_pixels(BfArgs k, int* list, int* count) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    const int lane = threadIdx.x & 31;
-    bool valid = x < k.width;
-    if (valid) {
-        const int m = (int)k.gnrm[(int64_t)y * k.gpitch + x].w;
-        if (m <= 0 || m >= k.num_mats) {
-            if (m != 0) set_error(k.err, ARC_DEVERR_BAD_MATERIAL);
-            valid = false;
+// A pixel's outputs from its FP64 sums (radiance 0..2, antiradiance 3..5): receiver BRDF, signed
+// combine; 0 without a surface (material 0).
+__device__ __forceinline__ void write_pixel(const BfArgs& k, int x, int y, int mat, const double* S) {
+    double rad[3] = {0, 0, 0}, ar[3] = {0, 0, 0}, res[3] = {0, 0, 0};
+    if (mat > 0) {
+        const float4 d = k.mats[mat].diffuse_exp;
+        const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            rad[c] = (double)kd[c] * S[c];
+            ar[c] = (double)kd[c] * S[3 + c];
+            res[c] = rad[c] - ar[c];
         }
     }
-    const unsigned vm = __ballot_sync(0xffffffffu, valid);
-    int base = 0;
-    if (vm) {
-        const int leader = __ffs(vm) - 1;
-        if (lane == leader) base = atomicAdd(count, __popc(vm));
-        base = __shfl_sync(0xffffffffu, base, leader);
-    }
-    if (valid) {
-        list[base + __popc(vm & ((1u << lane) - 1u))] = y * k.width + x;
-    } else if (x < k.width) {
-        const int64_t o = (int64_t)y * k.opitch + x;
-        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-        if (k.out_res) k.out_res[o] = z;
-        if (k.out_rad) k.out_rad[o] = z;
-        if (k.out_ar) k.out_ar[o] = z;
-        if (k.out_res64) k.out_res64[3 * o] = k.out_res64[3 * o + 1] = k.out_res64[3 * o + 2] = 0.0;
-        if (k.out_ar64) k.out_ar64[3 * o] = k.out_ar64[3 * o + 1] = k.out_ar64[3 * o + 2] = 0.0;
-    }
+    const int64_t o = (int64_t)y * k.opitch + x;
+    if (k.out_res) k.out_res[o] = make_float4((float)res[0], (float)res[1], (float)res[2], 1.0f);
+    if (k.out_rad) k.out_rad[o] = make_float4((float)rad[0], (float)rad[1], (float)rad[2], 1.0f);
+    if (k.out_ar) k.out_ar[o] = make_float4((float)ar[0], (float)ar[1], (float)ar[2], 1.0f);
+    if (k.out_res64)
+        for (int c = 0; c < 3; ++c) k.out_res64[3 * o + c] = res[c];
+    if (k.out_ar64)
+        for (int c = 0; c < 3; ++c) k.out_ar64[3 * o + c] = ar[c];
 }
 
 // ---------------------------------------------------------------------------------------
-// Packed FP32x2 variant of the default path (per-chunk partials folded into Kahan sums, no or cone
-// antiradiance).  Records come from pack_bf_pairs, so one 16-byte shared load brings two fields of
-// two AVPLs, and each thread evaluates two AVPLs per step for each of its PX pixels with
-// add/mul/fma.rn.f32x2 (sm_100).  Same terms as pair_terms; within a chunk the even and odd AVPLs
-// are summed apart and added before the chunk's Kahan step.
+// Culled form of the default precision (T = float: packed FP32x2, per-chunk FP32 partials folded
+// into FP64 sums) and of the all-FP64 precision (T = double), no or cone antiradiance.
+//
+// A block owns a 16 x 16 PX pixel tile and one segment (blockIdx.z) of the AVPLs.  Per chunk of
+// staged records: each thread tests one record against the tile's bounds (record_need), the kept
+// ones go in AVPL order into a radiance list and a cone list, the next chunk's copy is issued, and
+// every thread runs its PX pixels over the two lists.  The sums of several segments are added in
+// FP64 by bf_combine_segments.
 // ---------------------------------------------------------------------------------------
-// LIST: the block takes kThreads * PX consecutive entries of the compacted list of surface pixels
-// (bf_compact_pixels) instead of a 16 x 16 PX rectangle.
-template <int AR, int PX, bool LIST>
-__global__ void __launch_bounds__(kThreads) gather_bf_packed_kernel(BfArgs k) {
+// staged records | the two lists | FP32: the threads' FP64 sums (their registers hold the pixels and
+// the pair loop's operands instead) | mbarrier
+template <typename T, int PX>
+constexpr int culled_smem(int chunk) {
+    return chunk * 64 + 2 * chunk * (int)(kPairFloats / 2 * sizeof(T)) +
+           (sizeof(T) == 4 ? 6 * PX * kThreads * (int)sizeof(double) : 0) + 8;
+}
+
+// Three resident blocks of up to two pixels per thread hide the pair loop's latencies (24 warps)
+template <int AR, typename T, int PX, bool RAD>
+__global__ void __launch_bounds__(kThreads, PX <= 2 ? 3 : 1) gather_bf_culled_kernel(BfArgs k) {
+    constexpr bool kDouble = sizeof(T) == 8;
+    constexpr int kW = kThreads / 32;
     extern __shared__ __align__(128) unsigned char smem[];
-    float* stage = reinterpret_cast<float*>(smem);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)kStages * k.chunk * 64);
+    float4* stage = reinterpret_cast<float4*>(smem);
+    T* list_r = reinterpret_cast<T*>(smem + (size_t)k.chunk * 64);
+    T* list_a = list_r + (size_t)k.chunk * (kPairFloats / 2);
+    double* fsum = reinterpret_cast<double*>(list_a + (size_t)k.chunk * (kPairFloats / 2)) + threadIdx.x;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(list_a + (size_t)k.chunk * (kPairFloats / 2)) +
+                    (kDouble ? 0 : 6 * PX * kThreads);
+    __shared__ PixelBounds sb[kW];
+    __shared__ int s_cnt[2][2][kW];
 
-    const int tid = threadIdx.x;
-    const int tx = tid % kTileW, ty = tid / kTileW;
-    const int rows = kThreads / kTileW;  // 16
-    const int64_t lbase = (int64_t)blockIdx.x * kThreads * PX;
-    int list_n = 0;
-    if (LIST) {
-        list_n = *k.pixel_count;
-        if (lbase >= list_n) return;  // uniform: before any barrier
-    }
-    // pixel j of this thread
-    auto pixel_xy = [&](int j, int& px_, int& py_) {
-        if (LIST) {
-            const int64_t e = lbase + (int64_t)j * kThreads + tid;
-            const int idx = e < list_n ? k.pixel_list[e] : -1;
-            px_ = idx >= 0 ? idx % k.width : k.width;  // past the image: no pixel
-            py_ = idx >= 0 ? idx / k.width : 0;
-        } else {
-            px_ = blockIdx.x * kTileW + tx;
-            py_ = blockIdx.y * rows * PX + ty + j * rows;
-        }
-    };
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int x = blockIdx.x * kTileW + tid % kTileW;
+    const int y0 = blockIdx.y * (kThreads / kTileW) * PX + tid / kTileW;
+    constexpr int rows = kThreads / kTileW;
 
-    const int npad = k.n + (k.n & 1);  // records incl. the zero pad; k.chunk is even
-    const int nchunks = (npad + k.chunk - 1) / k.chunk;
-    if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) mbar_init(&bars[s], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-        for (int c = 0; c < kStages && c < nchunks; ++c) {
-            const int cnt = min(k.chunk, npad - c * k.chunk);
-            mbar_arrive_expect_tx(&bars[c], (uint32_t)cnt * 64u);
-            bulk_g2s(stage + (size_t)c * k.chunk * 16, k.records + (size_t)c * k.chunk * 4, (uint32_t)cnt * 64u,
-                     &bars[c]);
-        }
-    }
-
-    uint64_t PXc[PX], PYc[PX], PZc[PX], NXc[PX], NYc[PX], NZc[PX];
-    float sc[PX][6], ss[PX][6];
-    bool valid[PX];
-    int mat[PX];
+    T px_[PX], py_[PX], pz_[PX], nx_[PX], ny_[PX], nz_[PX];
+    int mat[PX];  // 0: no surface
+    PixelBounds b;
+    b.clear();
+    bool any = false;
 #pragma unroll
     for (int j = 0; j < PX; ++j) {
-        int x, y;
-        pixel_xy(j, x, y);
-        valid[j] = (x < k.width && y < k.height);
-        mat[j] = 0;
+        const int y = y0 + j * rows;
+        const bool in = x < k.width && y < k.height;
         float4 gp = make_float4(0, 0, 0, 0), gn = make_float4(0, 0, 0, 0);
-        if (valid[j]) {
+        if (in) {
             gp = k.gpos[(int64_t)y * k.gpitch + x];
             gn = k.gnrm[(int64_t)y * k.gpitch + x];
-            mat[j] = (int)gn.w;
-            if (mat[j] <= 0 || mat[j] >= k.num_mats) {
-                if (mat[j] != 0) set_error(k.err, ARC_DEVERR_BAD_MATERIAL);
-                valid[j] = false;
-            }
         }
-        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-        if (valid[j]) {
-            const float l = rsqrtf(gn.x * gn.x + gn.y * gn.y + gn.z * gn.z);
-            nx = gn.x * l;
-            ny = gn.y * l;
-            nz = gn.z * l;
+        mat[j] = (int)gn.w;
+        if (mat[j] <= 0 || mat[j] >= k.num_mats) {
+            if (mat[j] != 0) set_error(k.err, ARC_DEVERR_BAD_MATERIAL);
+            mat[j] = 0;
         }
-        PXc[j] = f2(-gp.x, -gp.x);
-        PYc[j] = f2(-gp.y, -gp.y);
-        PZc[j] = f2(-gp.z, -gp.z);
-        NXc[j] = f2(nx, nx);
-        NYc[j] = f2(ny, ny);
-        NZc[j] = f2(nz, nz);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) sc[j][c] = ss[j][c] = 0.0f;
+        nx_[j] = ny_[j] = nz_[j] = (T)0;
+        px_[j] = gp.x;
+        py_[j] = gp.y;
+        pz_[j] = gp.z;
+        if (mat[j]) {
+            const T l = rsqrt_t<T>((T)gn.x * gn.x + (T)gn.y * gn.y + (T)gn.z * gn.z);
+            nx_[j] = gn.x * l;
+            ny_[j] = gn.y * l;
+            nz_[j] = gn.z * l;
+            any = true;
+            if constexpr (kDouble)
+                b.add(gp.x, gp.y, gp.z, __double2float_rd(nx_[j]), __double2float_rd(ny_[j]),
+                      __double2float_rd(nz_[j]), __double2float_ru(nx_[j]), __double2float_ru(ny_[j]),
+                      __double2float_ru(nz_[j]));
+            else
+                b.add(gp.x, gp.y, gp.z, nx_[j], ny_[j], nz_[j], nx_[j], ny_[j], nz_[j]);
+        }
     }
-    const float cos_thr = k.pc.cos_thr, eps = k.pc.eps, inv_clamp2 = k.pc.inv_clamp2;
-    // distance floor folded into the FMA chain: l2 + 1e-30 equals max(l2, 1e-30) for l2 above ~1e-23
-    const uint64_t kTiny2 = f2(1e-30f, 1e-30f);
+    const bool live = __syncthreads_or(any) != 0;
 
-    bool ok = true;
-    int fail_c = -1;  // first chunk whose wait gave up
-    for (int c = 0; c < nchunks; ++c) {
-        const int s = c % kStages;
-        const uint32_t parity = (uint32_t)((c / kStages) & 1);
-        if (ok) {
-            ok = mbar_wait_bounded(&bars[s], parity, k.err);
-            if (!ok) fail_c = c;
+    double sum[PX][6];  // T = double; the FP32 form keeps its sums at fsum[(6 j + c) * kThreads]
+#pragma unroll
+    for (int j = 0; j < PX; ++j)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            sum[j][c] = 0.0;
+            if (!kDouble) fsum[(6 * j + c) * kThreads] = 0.0;
         }
-        if (ok) {
-            const int pairs = min(k.chunk, npad - c * k.chunk) >> 1;
-            const float* st = stage + (size_t)s * k.chunk * 16;
-            uint64_t acc[PX][6];
+    // adds a chunk's packed partial (even and odd list entries) to sum c of pixel j
+    auto fold = [&](int j, int c, uint64_t acc) {
+        float lo, hi;
+        f2_split(acc, lo, hi);
+        fsum[(6 * j + c) * kThreads] += (double)(lo + hi);
+    };
+    if (live) {
+        // this segment's chunks
+        const int nchunks = (k.n + k.chunk - 1) / k.chunk;
+        const int c0 = (int)((int64_t)nchunks * blockIdx.z / gridDim.z),
+                  c1 = (int)((int64_t)nchunks * (blockIdx.z + 1) / gridDim.z);
+        auto copy_chunk = [&](int c) {
+            const uint32_t bytes = (uint32_t)min(k.chunk, k.n - c * k.chunk) * 64u;
+            mbar_arrive_expect_tx(bar, bytes);
+            bulk_g2s(stage, k.records + (size_t)c * k.chunk * 4, bytes, bar);
+        };
+        if (tid == 0) {
+            mbar_init(bar, 1);
+            fence_mbar_init();
+        }
+        b.reduce_warp();
+        if (lane == 0) sb[w] = b;
+        __syncthreads();
+        if (tid == 0 && c0 < c1) copy_chunk(c0);
+        if (w == 0) {
+            b = sb[lane & (kW - 1)];
+            b.reduce_warp();
+            if (lane == 0) sb[0] = b;
+        }
+        __syncthreads();
+        const float cos_thr = k.pc.cos_thr, eps = k.pc.eps, inv_clamp2 = k.pc.inv_clamp2;
+        // distance floor folded into the FMA chain: l2 + 1e-30 equals max(l2, 1e-30) for l2 above ~1e-23
+        const uint64_t tiny2 = f2(1e-30f, 1e-30f);
+        PixelPair pp[PX];
+        if constexpr (!kDouble) {
 #pragma unroll
-            for (int j = 0; j < PX; ++j)
+            for (int j = 0; j < PX; ++j) pp[j] = pixel_pair(px_[j], py_[j], pz_[j], nx_[j], ny_[j], nz_[j]);
+        }
+        for (int c = c0; c < c1; ++c) {
+            const bool ok = mbar_wait_bounded(bar, (uint32_t)((c - c0) & 1), k.err);
+            const int cnt = min(k.chunk, k.n - c * k.chunk);
+            int nr = 0, na = 0;  // list lengths so far
+            bool all_ok = true;
+            for (int base = 0; base < cnt; base += kThreads) {
+                const int i = base + tid, turn = (base / kThreads) & 1;
+                RecordNeed need{false, false};
+                float4 q0, q1, q2, q3;
+                if (ok && i < cnt) {
+                    q0 = stage[4 * i];
+                    q1 = stage[4 * i + 1];
+                    q2 = stage[4 * i + 2];
+                    q3 = stage[4 * i + 3];
+                    need = record_need<AR == ARC_AR_CONE>(sb[0], q0, q1, q2, q3, cos_thr);
+                    if (!RAD) need.radiance = false;
+                }
+                const unsigned mr = __ballot_sync(0xffffffffu, need.radiance);
+                const unsigned ma = __ballot_sync(0xffffffffu, need.cone);
+                if (lane == 0) {
+                    s_cnt[turn][0][w] = __popc(mr);
+                    s_cnt[turn][1][w] = __popc(ma);
+                }
+                // also: every thread is done with the lists of the chunk before
+                all_ok = __syncthreads_and(ok) != 0;
+                if (!all_ok) break;
+                int er = nr + __popc(mr & ((1u << lane) - 1u)), ea = na + __popc(ma & ((1u << lane) - 1u));
 #pragma unroll
-                for (int q = 0; q < 6; ++q) acc[j][q] = 0;  // packed zeros
+                for (int q = 0; q < kW; ++q) {
+                    const int r = s_cnt[turn][0][q], a = s_cnt[turn][1][q];
+                    if (q < w) {
+                        er += r;
+                        ea += a;
+                    }
+                    nr += r;
+                    na += a;
+                }
+                if constexpr (kDouble) {
+                    if (need.radiance) {
+                        T* d = list_r + (size_t)er * (kPairFloats / 2);
+                        d[0] = q0.x; d[1] = q0.y; d[2] = q0.z;
+                        d[3] = q0.w; d[4] = q1.x; d[5] = q1.y;
+                        d[6] = q2.y; d[7] = q2.z; d[8] = q2.w;
+                    }
+                    if (need.cone) {
+                        T* d = list_a + (size_t)ea * (kPairFloats / 2);
+                        d[0] = q0.x; d[1] = q0.y; d[2] = q0.z;
+                        d[3] = q1.z; d[4] = q1.w; d[5] = q2.x;
+                        d[6] = q3.x; d[7] = q3.y; d[8] = q3.z;
+                    }
+                } else {
+                    if (need.radiance)
+                        put_entry(list_r, er, q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q2.y, q2.z, q2.w);
+                    if (need.cone) put_entry(list_a, ea, q0.x, q0.y, q0.z, q1.z, q1.w, q2.x, q3.x, q3.y, q3.z);
+                }
+            }
+            if (!all_ok) {  // the copy gave up: one more bounded wait for it before the block exits
+                if (tid == 0) drain_ring_bounded(bar, 1, c - c0, c1 - c0, k.err);
+                break;
+            }
+            if constexpr (!kDouble) {  // an odd list ends with a zero record, which adds exactly 0
+                if (tid == 0 && (nr & 1)) put_entry(list_r, nr, 0, 0, 0, 0, 0, 0, 0, 0, 0);
+                if (tid == 32 && (na & 1)) put_entry(list_a, na, 0, 0, 0, 0, 0, 0, 0, 0, 0);
+            }
+            __syncthreads();  // lists complete, staged records no longer read
+            if (tid == 0 && c + 1 < c1) {
+                fence_proxy_async_smem();
+                copy_chunk(c + 1);
+            }
+            if constexpr (kDouble) {
+                const T clampi = (T)inv_clamp2;
 #pragma unroll 2
-            for (int pr = 0; pr < pairs; ++pr) {
-                const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(st + pr * 32);
-                const ulonglong2 f01 = s2[0], f23 = s2[1], f45 = s2[2], f89 = s2[4], f1011 = s2[5];
+                for (int i = 0; i < nr; ++i) {
+                    const T* d = list_r + (size_t)i * (kPairFloats / 2);
 #pragma unroll
-                for (int j = 0; j < PX; ++j) {
-                    const uint64_t dx = f2_add(f01.x, PXc[j]), dy = f2_add(f01.y, PYc[j]), dz = f2_add(f23.x, PZc[j]);
-                    const uint64_t l2 = f2_fma(dz, dz, f2_fma(dy, dy, f2_fma(dx, dx, kTiny2)));  // >= 1e-30
-                    float l2a, l2b;
-                    f2_split(l2, l2a, l2b);
-                    const uint64_t r = f2(rsqrtf(l2a), rsqrtf(l2b));
-                    const uint64_t c1 = f2_mul(f2_fma(NZc[j], dz, f2_fma(NYc[j], dy, f2_mul(NXc[j], dx))), r);
-                    const uint64_t c2n = f2_mul(f2_fma(f45.y, dz, f2_fma(f45.x, dy, f2_mul(f23.y, dx))), r);
-                    float c1a, c1b, c2a, c2b, rra, rrb, ia, ib;
-                    f2_split(c1, c1a, c1b);
-                    f2_split(c2n, c2a, c2b);
-                    f2_split(f2_mul(r, r), rra, rrb);
-                    const uint64_t inv = f2(fminf(rra, inv_clamp2), fminf(rrb, inv_clamp2));
-                    // c1 / max(d^2, clamp^2): the radiance term's receiver factor and the cone term itself
-                    f2_split(f2_mul(c1, inv), ia, ib);
-                    const uint64_t g = f2_mul(f2(fmaxf(ia, 0.0f), fmaxf(ib, 0.0f)), f2(fmaxf(-c2a, 0.0f), fmaxf(-c2b, 0.0f)));
-                    acc[j][0] = f2_fma(f89.y, g, acc[j][0]);
-                    acc[j][1] = f2_fma(f1011.x, g, acc[j][1]);
-                    acc[j][2] = f2_fma(f1011.y, g, acc[j][2]);
-                    if (AR == ARC_AR_CONE) {
-                        const ulonglong2 f67 = s2[3], f1213 = s2[6], f1415 = s2[7];
-                        const uint64_t wdr = f2_mul(f2_fma(f89.x, dz, f2_fma(f67.y, dy, f2_mul(f67.x, dx))), r);
-                        float wa, wb;
-                        f2_split(wdr, wa, wb);
-                        const uint64_t ga = f2((-wa > cos_thr && c1a > eps) ? ia : 0.0f,
-                                               (-wb > cos_thr && c1b > eps) ? ib : 0.0f);
-                        acc[j][3] = f2_fma(f1213.x, ga, acc[j][3]);
-                        acc[j][4] = f2_fma(f1213.y, ga, acc[j][4]);
-                        acc[j][5] = f2_fma(f1415.x, ga, acc[j][5]);
+                    for (int j = 0; j < PX; ++j) {
+                        const T dx = d[0] - px_[j], dy = d[1] - py_[j], dz = d[2] - pz_[j];
+                        T l2 = dx * dx + dy * dy + dz * dz;
+                        l2 = l2 > (T)1e-30 ? l2 : (T)1e-30;
+                        const T inv = (T)1 / l2;
+                        const T a = (nx_[j] * dx + ny_[j] * dy + nz_[j] * dz) * inv;
+                        const T e = -(d[3] * dx + d[4] * dy + d[5] * dz) * (inv < clampi ? inv : clampi);
+                        const T g = (a > (T)0 ? a : (T)0) * (e > (T)0 ? e : (T)0);
+                        sum[j][0] += d[6] * g;
+                        sum[j][1] += d[7] * g;
+                        sum[j][2] += d[8] * g;
                     }
                 }
-            }
+                if (AR == ARC_AR_CONE) {
+                    for (int i = 0; i < na; ++i) {
+                        const T* d = list_a + (size_t)i * (kPairFloats / 2);
 #pragma unroll
-            for (int j = 0; j < PX; ++j)
-#pragma unroll
-                for (int q = 0; q < 6; ++q) {
-                    float lo, hi;
-                    f2_split(acc[j][q], lo, hi);
-                    kahan_add(ss[j][q], sc[j][q], lo + hi);
+                        for (int j = 0; j < PX; ++j) {
+                            const T dx = d[0] - px_[j], dy = d[1] - py_[j], dz = d[2] - pz_[j];
+                            T l2 = dx * dx + dy * dy + dz * dz;
+                            l2 = l2 > (T)1e-30 ? l2 : (T)1e-30;
+                            const T r = rsqrt(l2);
+                            const T a = (nx_[j] * dx + ny_[j] * dy + nz_[j] * dz) * r;
+                            const T cw = -(d[3] * dx + d[4] * dy + d[5] * dz) * r;
+                            const T rr = r * r;
+                            if (cw > (T)cos_thr && a > (T)eps) {
+                                const T ga = a * (rr < clampi ? rr : clampi);
+                                sum[j][3] += d[6] * ga;
+                                sum[j][4] += d[7] * ga;
+                                sum[j][5] += d[8] * ga;
+                            }
+                        }
+                    }
                 }
-        }
-        __syncthreads();  // every thread is done reading stage s before it is refilled
-        if (tid == 0 && ok && c + kStages < nchunks) {
-            fence_proxy_async_smem();
-            const int cn = c + kStages;
-            const int cnt = min(k.chunk, npad - cn * k.chunk);
-            mbar_arrive_expect_tx(&bars[s], (uint32_t)cnt * 64u);
-            bulk_g2s(stage + (size_t)s * k.chunk * 16, k.records + (size_t)cn * k.chunk * 4, (uint32_t)cnt * 64u,
-                     &bars[s]);
+            } else {
+                if (RAD) {
+                    uint64_t acc[PX][3] = {};  // packed zeros
+#pragma unroll 2
+                    for (int pr = 0; 2 * pr < nr; ++pr)
+#pragma unroll
+                        for (int j = 0; j < PX; ++j)
+                            radiance_pair(list_r + pr * kPairFloats, pp[j], inv_clamp2, tiny2, acc[j][0], acc[j][1],
+                                          acc[j][2]);
+#pragma unroll
+                    for (int j = 0; j < PX; ++j)
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) fold(j, q, acc[j][q]);
+                }
+                if (AR == ARC_AR_CONE && na > 0) {
+                    uint64_t acc[PX][3] = {};
+#pragma unroll 1
+                    for (int pr = 0; 2 * pr < na; ++pr)
+#pragma unroll
+                        for (int j = 0; j < PX; ++j)
+                            cone_pair(list_a + pr * kPairFloats, pp[j], cos_thr, eps, inv_clamp2, tiny2, acc[j][0],
+                                      acc[j][1], acc[j][2]);
+#pragma unroll
+                    for (int j = 0; j < PX; ++j)
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) fold(j, 3 + q, acc[j][q]);
+                }
+            }
         }
     }
-    // the copies the ring still has in flight after a wait gave up (only thread 0 issues them)
-    if (tid == 0 && fail_c >= 0) drain_ring_bounded(bars, kStages, fail_c, nchunks, k.err);
 
-    // epilogue: receiver BRDF, FP64 signed combine, stores
 #pragma unroll
     for (int j = 0; j < PX; ++j) {
-        int x, y;
-        pixel_xy(j, x, y);
+        double S[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) S[c] = kDouble ? sum[j][c] : fsum[(6 * j + c) * kThreads];
+        if (k.partial) {
+            double* d = k.partial + (((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * gridDim.z + blockIdx.z) * 6 *
+                                        (kThreads * PX) + j * kThreads + tid;
+            if (live)  // (a tile without surface pixels is written by bf_combine_segments alone)
+#pragma unroll
+                for (int c = 0; c < 6; ++c) d[c * (kThreads * PX)] = S[c];
+        } else {
+            const int y = y0 + j * rows;
+            if (x < k.width && y < k.height) write_pixel(k, x, y, mat[j], S);
+        }
+    }
+}
+
+// The segments' sums of every pixel added in segment order, and the outputs; the grid of
+// gather_bf_culled_kernel without its segments.
+template <int PX>
+__global__ void __launch_bounds__(kThreads) bf_combine_segments(BfArgs k, int segments) {
+    const int tid = threadIdx.x;
+    const int x = blockIdx.x * kTileW + tid % kTileW;
+#pragma unroll
+    for (int j = 0; j < PX; ++j) {
+        const int y = (blockIdx.y * PX + j) * (kThreads / kTileW) + tid / kTileW;
         if (x >= k.width || y >= k.height) continue;
-        double rad[3] = {0, 0, 0}, ar[3] = {0, 0, 0}, res[3] = {0, 0, 0};
-        if (valid[j]) {
-            const float4 d = k.mats[mat[j]].diffuse_exp;
-            const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
-            for (int c = 0; c < 3; ++c) {
-                rad[c] = (double)kd[c] * ((double)ss[j][c] - (double)sc[j][c]);
-                ar[c] = (double)kd[c] * ((double)ss[j][3 + c] - (double)sc[j][3 + c]);
-                res[c] = rad[c] - ar[c];
-            }
+        int m = (int)k.gnrm[(int64_t)y * k.gpitch + x].w;
+        if (m < 0 || m >= k.num_mats) m = 0;
+        double S[6] = {0, 0, 0, 0, 0, 0};
+        if (m > 0) {
+            const double* d = k.partial + ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * segments * 6 *
+                                              (kThreads * PX) + j * kThreads + tid;
+            for (int s = 0; s < segments; ++s)
+#pragma unroll
+                for (int c = 0; c < 6; ++c) S[c] += d[(s * 6 + c) * (kThreads * PX)];
         }
-        const int64_t o = (int64_t)y * k.opitch + x;
-        if (k.out_res) k.out_res[o] = make_float4((float)res[0], (float)res[1], (float)res[2], 1.0f);
-        if (k.out_rad) k.out_rad[o] = make_float4((float)rad[0], (float)rad[1], (float)rad[2], 1.0f);
-        if (k.out_ar) k.out_ar[o] = make_float4((float)ar[0], (float)ar[1], (float)ar[2], 1.0f);
-        if (k.out_res64) {
-            k.out_res64[3 * o + 0] = res[0];
-            k.out_res64[3 * o + 1] = res[1];
-            k.out_res64[3 * o + 2] = res[2];
-        }
-        if (k.out_ar64) {
-            k.out_ar64[3 * o + 0] = ar[0];
-            k.out_ar64[3 * o + 1] = ar[1];
-            k.out_ar64[3 * o + 2] = ar[2];
-        }
+        write_pixel(k, x, y, m, S);
     }
 }
 
@@ -696,6 +779,13 @@ constexpr TileShape kTileShapes[] = {{1, 128}, {2, 128}, {2, 256}, {4, 128}, {4,
                                      {4, 64},  {1, 512}, {2, 512}, {4, 512}, {1, 1024}, {2, 1024}};
 constexpr int kNumTileShapes = sizeof(kTileShapes) / sizeof(kTileShapes[0]);
 constexpr int kDefaultTileShape = 2;
+constexpr int kFp64Chunk = 256;
+// Segments of the culled gather: enough blocks for several waves of resident ones (a grid of one
+// partial wave leaves SMs idle), each segment at least kMinChunks chunks long (a block's set-up --
+// pixel loads, tile bounds -- costs about a chunk), partial sums within kPartialBytes.
+constexpr int kBlocksPerSm = 24;
+constexpr int kMinChunks = 2;
+constexpr int64_t kPartialBytes = (int64_t)1 << 30;
 
 template <int AR, int PREC, int PX, bool RAD = true>
 arc_status launch_fast(const BfArgs& a, cudaStream_t st) {
@@ -715,59 +805,86 @@ arc_status launch_fast_px(const BfArgs& a, int px, cudaStream_t st) {
     return launch_fast<AR, PREC, 4>(a, st);
 }
 
-template <int AR>
-arc_status launch_fast_prec(const BfArgs& a, int prec, int px, cudaStream_t st) {
-    switch (prec) {
-        case 0: return launch_fast_px<AR, 0>(a, px, st);
-        case 1: return launch_fast_px<AR, 1>(a, px, st);
-        case 2: return launch_fast_px<AR, 2>(a, px, st);
-        default: return launch_fast<AR, 3, 1>(a, st);
-    }
+// the culled kernel serves the default and the all-FP64 precision with no or cone antiradiance
+bool use_culled(const ArcGatherParams& p) {
+    return p.ar_kind != ARC_AR_DISK && (p.precision == ARC_PREC_KAHAN || p.precision == ARC_PREC_FP64);
 }
 
-// the packed kernel serves the default precision with no or cone antiradiance
-bool use_packed(const ArcGatherParams& p) { return p.precision == ARC_PREC_KAHAN && p.ar_kind != ARC_AR_DISK; }
+dim3 tile_grid(const BfArgs& a, int px) {
+    return dim3((a.width + kTileW - 1) / kTileW, (a.height + 16 * px - 1) / (16 * px));
+}
 
-template <int AR, int PX>
-arc_status launch_packed(const BfArgs& a, cudaStream_t st) {
-    const size_t smem = (size_t)kStages * a.chunk * 64 + kStages * sizeof(uint64_t);
-    if (a.pixel_list) {  // one block per kThreads * PX listed pixels; blocks past the count return
-        auto fn = gather_bf_packed_kernel<AR, PX, true>;
-        if (smem > 48 * 1024)
-            ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int64_t pixels = (int64_t)a.width * a.height;
-        fn<<<(unsigned)((pixels + kThreads * PX - 1) / (kThreads * PX)), kThreads, smem, st>>>(a);
-    } else {
-        auto fn = gather_bf_packed_kernel<AR, PX, false>;
-        if (smem > 48 * 1024)
-            ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        dim3 grid((a.width + kTileW - 1) / kTileW, (a.height + 16 * PX - 1) / (16 * PX));
-        fn<<<grid, kThreads, smem, st>>>(a);
-    }
+template <int AR, typename T, int PX, bool RAD>
+arc_status launch_culled_kernel(const BfArgs& a, int segments, cudaStream_t st) {
+    const int smem = culled_smem<T, PX>(a.chunk);
+    auto fn = gather_bf_culled_kernel<AR, T, PX, RAD>;
+    ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    dim3 grid = tile_grid(a, PX);
+    grid.z = (unsigned)segments;
+    fn<<<grid, kThreads, smem, st>>>(a);
     ARC_TRY_CUDA(cudaGetLastError());
+    if (a.partial) {
+        bf_combine_segments<PX><<<tile_grid(a, PX), kThreads, 0, st>>>(a, segments);
+        ARC_TRY_CUDA(cudaGetLastError());
+    }
     return ARC_OK;
 }
 
-template <int AR>
-arc_status launch_packed_px(const BfArgs& a, int px, cudaStream_t st) {
-    if (px == 1) return launch_packed<AR, 1>(a, st);
-    if (px == 2) return launch_packed<AR, 2>(a, st);
-    return launch_packed<AR, 4>(a, st);
+template <int AR, bool RAD>
+arc_status launch_culled_px(const BfArgs& a, int px, int segments, cudaStream_t st) {
+    if (px == 1) return launch_culled_kernel<AR, float, 1, RAD>(a, segments, st);
+    if (px == 2) return launch_culled_kernel<AR, float, 2, RAD>(a, segments, st);
+    return launch_culled_kernel<AR, float, 4, RAD>(a, segments, st);
 }
 
-// dispatch of the fast path (records packed by pack_bf_pairs when use_packed(p), else by
-// pack_bf_records)
+// A culled gather: its pixels per thread and AVPLs per chunk, and how many segments the AVPLs are
+// split into.
+struct CulledPlan {
+    int px, chunk, segments;
+};
+
+CulledPlan culled_plan(const BfArgs& a, const ArcGatherParams& p, int shape, int sm_count) {
+    CulledPlan c{kTileShapes[shape >= 0 ? shape : kDefaultTileShape].px,
+                 kTileShapes[shape >= 0 ? shape : kDefaultTileShape].chunk, 1};
+    if (p.precision == ARC_PREC_FP64) c = CulledPlan{1, kFp64Chunk, 1};
+    const dim3 g = tile_grid(a, c.px);
+    const int64_t tiles = (int64_t)g.x * g.y;
+    const int64_t want = ((int64_t)sm_count * kBlocksPerSm + tiles - 1) / tiles;
+    const int64_t chunks = (a.n + c.chunk - 1) / c.chunk;
+    const int64_t room = kPartialBytes / (tiles * 6 * kThreads * c.px * (int64_t)sizeof(double));
+    c.segments = (int)std::max<int64_t>(1, std::min(std::min(want, chunks / kMinChunks), room));
+    return c;
+}
+
+// dispatch of the culled path (a.records packed); a.partial: room for plan.segments, or NULL with one
+arc_status launch_culled(BfArgs a, const ArcGatherParams& p, const CulledPlan& c, cudaStream_t st) {
+    a.chunk = c.chunk;
+    if (p.precision == ARC_PREC_FP64)
+        return p.ar_kind == ARC_AR_NONE ? launch_culled_kernel<0, double, 1, true>(a, c.segments, st)
+                                        : launch_culled_kernel<2, double, 1, true>(a, c.segments, st);
+    return p.ar_kind == ARC_AR_NONE ? launch_culled_px<0, true>(a, c.px, c.segments, st)
+                                    : launch_culled_px<2, true>(a, c.px, c.segments, st);
+}
+
+template <int AR>
+arc_status launch_fast_prec(const BfArgs& a, int prec, int px, cudaStream_t st) {
+    return prec == ARC_PREC_KAHAN_STRICT ? launch_fast_px<AR, 1>(a, px, st) : launch_fast_px<AR, 2>(a, px, st);
+}
+
+// dispatch of the kernel that evaluates every pair
 arc_status launch_fast_path(const BfArgs& a, const ArcGatherParams& p, int px, cudaStream_t st) {
-    if (use_packed(p)) return p.ar_kind == ARC_AR_NONE ? launch_packed_px<0>(a, px, st) : launch_packed_px<2>(a, px, st);
-    switch (p.ar_kind) {
-        case 0: return launch_fast_prec<0>(a, p.precision, px, st);
-        case 1: return launch_fast_prec<1>(a, p.precision, px, st);
-        default: return launch_fast_prec<2>(a, p.precision, px, st);
+    if (p.ar_kind == ARC_AR_DISK) {
+        if (p.precision == ARC_PREC_KAHAN) return launch_fast_px<1, 0>(a, px, st);
+        if (p.precision == ARC_PREC_FP64) return launch_fast<1, 3, 1>(a, st);
+        return launch_fast_prec<1>(a, p.precision, px, st);
     }
+    return p.ar_kind == ARC_AR_NONE ? launch_fast_prec<0>(a, p.precision, px, st)
+                                    : launch_fast_prec<2>(a, p.precision, px, st);
 }
 
 BfArgs make_args(arc_context* ctx, const GatherLaunch& g);
-arc_status pack_records(arc_context* ctx, const GatherLaunch& g, BfArgs& a, bool pairs);
+arc_status pack_records(arc_context* ctx, const GatherLaunch& g, BfArgs& a);
+arc_status run_culled(arc_context* ctx, BfArgs& a, const ArcGatherParams& p, int shape, bool rad);
 
 }  // namespace
 
@@ -809,23 +926,11 @@ arc_status launch_gather_bruteforce(arc_context* ctx, const GatherLaunch& g) {
         ARC_TRY_CUDA(cudaGetLastError());
         return ARC_OK;
     }
-    ARC_TRY(pack_records(ctx, g, a, use_packed(p)));
-    const int shape = p.tile_config >= 0 ? p.tile_config : (ctx->bf_tile_config >= 0 ? ctx->bf_tile_config : kDefaultTileShape);
-    const TileShape ts = kTileShapes[shape];
+    ARC_TRY(pack_records(ctx, g, a));
+    const int chosen = p.tile_config >= 0 ? p.tile_config : ctx->bf_tile_config;
+    if (use_culled(p)) return run_culled(ctx, a, p, chosen, true);
+    const TileShape ts = kTileShapes[chosen >= 0 ? chosen : kDefaultTileShape];
     a.chunk = ts.chunk;
-    if (use_packed(p)) {  // only surface pixels are gathered
-        int *list = nullptr, *count = nullptr;
-        ARC_TRY(ctx->arena.get("bf_pixel_list", sizeof(int) * (size_t)gb.width * gb.height,
-                               reinterpret_cast<void**>(&list)));
-        ARC_TRY(ctx->arena.get("bf_pixel_count", sizeof(int), reinterpret_cast<void**>(&count)));
-        ARC_TRY_CUDA(cudaMemsetAsync(count, 0, sizeof(int), st));
-        stage_begin(ctx, "bf_pixels");
-        bf_compact_pixels<<<dim3((gb.width + 255) / 256, gb.height), 256, 0, st>>>(a, list, count);
-        stage_end(ctx, 1);
-        ARC_TRY_CUDA(cudaGetLastError());
-        a.pixel_list = list;
-        a.pixel_count = count;
-    }
     stage_begin(ctx, "bf_gather");
     const arc_status s = launch_fast_path(a, p, ts.px, st);
     stage_end(ctx, 1);
@@ -855,11 +960,15 @@ arc_status launch_antiradiance_only(arc_context* ctx, const GatherLaunch& g, dou
     a.out_res64 = nullptr;
     a.out_ar64 = ar64;
     cudaStream_t st = ctx->stream;
-    ARC_TRY(pack_records(ctx, g, a, false));
+    ARC_TRY(pack_records(ctx, g, a));
+    if (p.ar_kind == ARC_AR_CONE) {
+        ArcGatherParams q = p;
+        q.precision = ARC_PREC_KAHAN;
+        return run_culled(ctx, a, q, -1, false);
+    }
     a.chunk = kTileShapes[kDefaultTileShape].chunk;
     stage_begin(ctx, "bf_antiradiance");
-    const arc_status s = p.ar_kind == ARC_AR_DISK ? launch_fast<ARC_AR_DISK, 0, 2, false>(a, st)
-                                                  : launch_fast<ARC_AR_CONE, 0, 2, false>(a, st);
+    const arc_status s = launch_fast<ARC_AR_DISK, 0, 2, false>(a, st);
     stage_end(ctx, 1);
     return s;
 }
@@ -905,22 +1014,32 @@ BfArgs make_args(arc_context* ctx, const GatherLaunch& g) {
 }
 
 // Pack the AVPL records into the context arena.
-arc_status pack_records(arc_context* ctx, const GatherLaunch& g, BfArgs& a, bool pairs) {
-    float4* rec = nullptr;
-    ARC_TRY(ctx->arena.get("bf_records", (size_t)(a.n + 1) * 64, reinterpret_cast<void**>(&rec)));
-    if (a.n > 0) {
-        stage_begin(ctx, "bf_pack");
-        if (pairs)
-            pack_bf_pairs<<<(a.n + 1 + 255) / 256, 256, 0, ctx->stream>>>(
-                *g.avpls, ctx->d_materials, ctx->num_materials, reinterpret_cast<float*>(rec), ctx->d_error);
-        else
-            pack_bf_records<<<(a.n + 255) / 256, 256, 0, ctx->stream>>>(*g.avpls, ctx->d_materials,
-                                                                         ctx->num_materials, rec, ctx->d_error);
-        stage_end(ctx, 1);
-        ARC_TRY_CUDA(cudaGetLastError());
-    }
+arc_status pack_records(arc_context* ctx, const GatherLaunch& g, BfArgs& a) {
+    const float4* rec = nullptr;
+    ARC_TRY(launch_pack_records(ctx, g.avpls, &rec));
     a.records = rec;
     return ARC_OK;
+}
+
+// The culled gather on the context's stream (rad: radiance and antiradiance; else the cone
+// antiradiance alone), its partial sums in the context arena.
+arc_status run_culled(arc_context* ctx, BfArgs& a, const ArcGatherParams& p, int shape, bool rad) {
+    const CulledPlan c = culled_plan(a, p, shape, ctx->sm_count);
+    if (c.segments > 1) {
+        const dim3 g = tile_grid(a, c.px);
+        ARC_TRY(ctx->arena.get("bf_partial", (size_t)g.x * g.y * c.segments * 6 * kThreads * c.px * sizeof(double),
+                               reinterpret_cast<void**>(&a.partial)));
+    }
+    stage_begin(ctx, rad ? "bf_gather" : "bf_antiradiance");
+    arc_status s;
+    if (rad) {
+        s = launch_culled(a, p, c, ctx->stream);
+    } else {
+        a.chunk = c.chunk;
+        s = launch_culled_px<ARC_AR_CONE, false>(a, c.px, c.segments, ctx->stream);
+    }
+    stage_end(ctx, a.partial ? 2 : 1);
+    return s;
 }
 
 }  // namespace
@@ -1111,17 +1230,18 @@ extern "C" arc_status arc_gather_bruteforce_noalloc(void* cuda_stream, const Arc
         ARC_TRY_CUDA(cudaGetLastError());
     } else {
         if (a.n > 0) {
-            // an odd count's zero pad record still fits: the scratch holds kNoAllocMaxAvpls (even)
-            if (use_packed(p))
-                pack_bf_pairs<<<(a.n + 1 + 255) / 256, 256, 0, st>>>(*avpls, mats, num_materials,
-                                                                    reinterpret_cast<float*>(records), err);
-            else
-                pack_bf_records<<<(a.n + 255) / 256, 256, 0, st>>>(*avpls, mats, num_materials, records, err);
+            pack_bf_records<<<(a.n + 255) / 256, 256, 0, st>>>(*avpls, mats, num_materials, records, err);
             ARC_TRY_CUDA(cudaGetLastError());
         }
-        const TileShape ts = kTileShapes[p.tile_config < 0 ? kDefaultTileShape : p.tile_config];
-        a.chunk = ts.chunk;
-        ARC_TRY(launch_fast_path(a, p, ts.px, st));
+        if (use_culled(p)) {  // one segment: there is no room for partial sums
+            CulledPlan c = culled_plan(a, p, p.tile_config, 1);
+            c.segments = 1;
+            ARC_TRY(launch_culled(a, p, c, st));
+        } else {
+            const TileShape ts = kTileShapes[p.tile_config < 0 ? kDefaultTileShape : p.tile_config];
+            a.chunk = ts.chunk;
+            ARC_TRY(launch_fast_path(a, p, ts.px, st));
+        }
     }
     if (device_error_word) {
         uint32_t w = 0;
