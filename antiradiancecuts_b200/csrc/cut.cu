@@ -800,6 +800,17 @@ __global__ void combine_kernel(const double* rad64, const double* ar64, int widt
 
 }  // namespace
 
+arc_status launch_combine(arc_context* ctx, const double* rad64, const double* ar64, int width, int height,
+                          const ArcOutputView* out) {
+    stage_begin(ctx, "combine");
+    combine_kernel<<<dim3((width + 31) / 32, (height + 7) / 8), dim3(32, 8), 0, ctx->stream>>>(
+        rad64, ar64, width, height, reinterpret_cast<float4*>(out->result),
+        reinterpret_cast<float4*>(out->antiradiance), out->result_fp64, out->pitch);
+    stage_end(ctx, 1);
+    ARC_TRY_CUDA(cudaGetLastError());
+    return ARC_OK;
+}
+
 arc_status launch_tile_setup(arc_context* ctx, const arc_lbvh* bvh, const ArcGBufferView* gb, const ArcGatherParams* gp,
                              const ArcCutParams* cp, float4** info_out, float4** extra_out) {
     const int W = gb->width, H = gb->height;
@@ -885,14 +896,7 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
             GatherLaunch g{avpls, gb, cam, gp, out};
             ARC_TRY(launch_antiradiance_only(ctx, g, ar64));
         }
-        dim3 cg((W + 31) / 32, (H + 7) / 8);
-        stage_begin(ctx, "combine");
-        combine_kernel<<<cg, dim3(32, 8), 0, st>>>(rad64, ar64, W, H, reinterpret_cast<float4*>(out->result),
-                                                  reinterpret_cast<float4*>(out->antiradiance), out->result_fp64,
-                                                  out->pitch);
-        stage_end(ctx, 1);
-        ARC_TRY_CUDA(cudaGetLastError());
-        return ARC_OK;
+        return launch_combine(ctx, rad64, ar64, W, H, out);
     }
 
     // tile cuts

@@ -1,0 +1,291 @@
+// Disk antiradiance of every AVPL at every pixel (getAntiradiance, cudaGather.cu:97-144), with the
+// AVPLs culled per block of pixels.
+//
+// A pair contributes only when the AVPL's ray p_a + s w (s > 0) passes within the disk radius of the
+// pixel, the AVPL lies in front of the pixel and the pixel behind the AVPL: a handful of AVPLs per
+// pixel.  A block owns a pixel tile and walks the AVPLs in order, kStep at a time:
+//   1. each thread tests AVPLs' rays against the tile's bounding sphere grown by the radius, and the
+//      block compacts the survivors in AVPL order;
+//   2. each warp tests survivors, one per lane, against its own pixels' sphere and their position and
+//      normal boxes, and stages the records that remain;
+//   3. every lane evaluates those for its pixels with the terms of pair_terms, in AVPL order, with one
+//      compensated sum per channel.
+// The tests drop a pair only when pair_terms is certain to give 0 (their margins exceed its rounding),
+// so the sums are those over every AVPL.  The work left is the ray tests, 20 operations per (tile,
+// AVPL) instead of 45 per (pixel, AVPL).
+#include <cfloat>
+
+#include "arc_internal.h"
+#include "device_common.cuh"
+#include "pair_cull.cuh"
+#include "pair_math.cuh"
+
+namespace arc {
+namespace {
+
+constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr int kPerThread = 4;                     // rays tested per thread and step
+constexpr int kStep = kThreads * kPerThread;      // AVPLs per step
+static_assert(kPerThread * kWarps == 32, "one lane per (pass, warp) count in the block's prefix sum");
+
+// 32 x 32 tiles when they make at least this many blocks per SM, else 16 x 16
+constexpr int64_t kBigTilesPerSm = 4;
+
+struct DiskArgs {
+    const float4* records;  // 4 float4 per AVPL (launch_pack_records)
+    const float4* rays;     // 2 float4 per AVPL: {p, > 0 when it can contribute}, {w / |w|, 0}
+    int n;
+    const float4* gpos;
+    const float4* gnrm;
+    int64_t gpitch;
+    int width, height;
+    const MaterialRecord* mats;
+    int num_mats;
+    PairConsts pc;
+    float radius;
+    float disk_scale;
+    bool clustered;   // surface pixels as the clustered pass has them (normal.w > 0)
+    float4* out_ar;
+    double* out_ar64; // 3 per pixel
+    int64_t opitch;
+    uint32_t* err;
+};
+
+// The rays of the packed records.  An AVPL without antiradiance or without a direction adds 0 to
+// every pixel; one with a non-finite antiradiance is kept.
+__global__ void disk_rays(const float4* records, int n, float4* rays) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 q0 = records[4 * (size_t)i], q1 = records[4 * (size_t)i + 1], q2 = records[4 * (size_t)i + 2],
+                 q3 = records[4 * (size_t)i + 3];
+    const float la = fabsf(q3.x) + fabsf(q3.y) + fabsf(q3.z);
+    const bool never = la == 0.0f || (la <= FLT_MAX && q1.z == 0.0f && q1.w == 0.0f && q2.x == 0.0f);
+    rays[2 * (size_t)i] = make_float4(q0.x, q0.y, q0.z, never ? 0.0f : 1.0f);
+    rays[2 * (size_t)i + 1] = make_float4(q1.z * q3.w, q1.w * q3.w, q2.x * q3.w, 0.0f);
+}
+
+// Whether the ray from r0 along the unit vector r1 can pass within `radius` of a point of the sphere
+// (c, rho); the margin covers the rounding of the hit point in pair_terms (a few ulp of the distance).
+__device__ __forceinline__ bool ray_near(float4 r0, float4 r1, float cx, float cy, float cz, float rho) {
+    const float vx = cx - r0.x, vy = cy - r0.y, vz = cz - r0.z;
+    const float s = fmaxf(0.0f, vx * r1.x + vy * r1.y + vz * r1.z);
+    const float hx = vx - s * r1.x, hy = vy - s * r1.y, hz = vz - s * r1.z;
+    const float reach = rho + 1e-4f * (rho + s + fabsf(vx) + fabsf(vy) + fabsf(vz));
+    return !(hx * hx + hy * hy + hz * hz > reach * reach);
+}
+
+// PX = 1: 16 x 16 pixel tiles, 8 x 4 pixels per warp; PX = 4: 32 x 32 tiles, 16 x 8 per warp.
+template <int PX>
+__global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
+    constexpr int kSide = PX == 1 ? 16 : 32, kSub = PX == 1 ? 1 : 2;
+    __shared__ float4 s_rec[kWarps][32 * 4];
+    __shared__ int s_list[kStep];
+    __shared__ int s_cnt[32];
+    __shared__ PixelBounds s_box[kWarps];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int xb = blockIdx.x * kSide + (w & 1) * 8 * kSub + (lane & 7);
+    const int yb = blockIdx.y * kSide + (w >> 1) * 4 * kSub + (lane >> 3);
+
+    Pixel<float> px[PX];
+    int mat[PX];  // 0: nothing to gather
+    PixelBounds box;
+    box.clear();
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < PX; ++j) {
+        const int x = xb + (j % kSub) * 8, y = yb + (j / kSub) * 4;
+        float4 gp = make_float4(0, 0, 0, 0), gn = make_float4(0, 0, 0, 0);
+        if (x < a.width && y < a.height) {
+            gp = a.gpos[(int64_t)y * a.gpitch + x];
+            gn = a.gnrm[(int64_t)y * a.gpitch + x];
+        }
+        mat[j] = (int)gn.w;
+        if (mat[j] <= 0 || mat[j] >= a.num_mats) {
+            if (a.clustered ? gn.w > 0.0f : mat[j] != 0) set_error(a.err, ARC_DEVERR_BAD_MATERIAL);
+            mat[j] = 0;
+        }
+        const float l = mat[j] ? rsqrtf(gn.x * gn.x + gn.y * gn.y + gn.z * gn.z) : 0.0f;
+        px[j].px = gp.x;
+        px[j].py = gp.y;
+        px[j].pz = gp.z;
+        px[j].nx = gn.x * l;
+        px[j].ny = gn.y * l;
+        px[j].nz = gn.z * l;
+        if (mat[j]) {
+            any = true;
+            box.add(gp.x, gp.y, gp.z, px[j].nx, px[j].ny, px[j].nz, px[j].nx, px[j].ny, px[j].nz);
+        }
+    }
+    float sum[PX][3], comp[PX][3];
+#pragma unroll
+    for (int j = 0; j < PX; ++j)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sum[j][c] = comp[j][c] = 0.0f;
+
+    const bool warp_live = __any_sync(0xffffffffu, any);
+    if (__syncthreads_or(any)) {
+        box.reduce_warp();
+        if (lane == 0) s_box[w] = box;
+        __syncthreads();
+        PixelBounds tb = s_box[0];
+        for (int q = 1; q < kWarps; ++q) tb.merge(s_box[q]);
+        // bounding spheres of the tile and of the warp, grown by the disk radius
+        auto sphere = [&](const PixelBounds& b, float& cx, float& cy, float& cz) {
+            cx = 0.5f * (b.pmin[0] + b.pmax[0]);
+            cy = 0.5f * (b.pmin[1] + b.pmax[1]);
+            cz = 0.5f * (b.pmin[2] + b.pmax[2]);
+            const float ex = b.pmax[0] - b.pmin[0], ey = b.pmax[1] - b.pmin[1], ez = b.pmax[2] - b.pmin[2];
+            return 0.5001f * sqrtf(ex * ex + ey * ey + ez * ez) + a.radius;
+        };
+        float tcx, tcy, tcz, wcx, wcy, wcz;
+        const float trho = sphere(tb, tcx, tcy, tcz);
+        const float wrho = sphere(box, wcx, wcy, wcz);
+        float4* rec = s_rec[w];
+        for (int base = 0; base < a.n; base += kStep) {
+            unsigned m[kPerThread];
+#pragma unroll
+            for (int u = 0; u < kPerThread; ++u) {
+                const int i = base + u * kThreads + tid;
+                bool near = false;
+                if (i < a.n) {
+                    const float4 r0 = a.rays[2 * (size_t)i], r1 = a.rays[2 * (size_t)i + 1];
+                    near = r0.w != 0.0f && ray_near(r0, r1, tcx, tcy, tcz, trho);
+                }
+                m[u] = __ballot_sync(0xffffffffu, near);
+                if (lane == 0) s_cnt[u * kWarps + w] = __popc(m[u]);
+            }
+            __syncthreads();  // the counts; and every warp is done with the list of the step before
+            int incl = s_cnt[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int excl = incl - s_cnt[lane];
+            const int count = __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+            for (int u = 0; u < kPerThread; ++u) {
+                const int first = __shfl_sync(0xffffffffu, excl, u * kWarps + w);
+                if (m[u] >> lane & 1u) s_list[first + __popc(m[u] & ((1u << lane) - 1u))] = base + u * kThreads + tid;
+            }
+            __syncthreads();
+            if (!warp_live) continue;
+            for (int k = 0; k < count; k += 32) {
+                float4 q0, q1, q2, q3;
+                bool keep = false;
+                if (k + lane < count) {
+                    const int i = s_list[k + lane];
+                    const float4* q = a.records + 4 * (size_t)i;
+                    q0 = q[0];
+                    q1 = q[1];
+                    q2 = q[2];
+                    q3 = q[3];
+                    keep = ray_near(q0, make_float4(q1.z * q3.w, q1.w * q3.w, q2.x * q3.w, 0.0f), wcx, wcy, wcz, wrho);
+                    if (keep) {
+                        const float p[3] = {q0.x, q0.y, q0.z}, n[3] = {q0.w, q1.x, q1.y};
+                        float recv[3], back[3];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            const float lo = p[d] - box.pmax[d], hi = p[d] - box.pmin[d];
+                            recv[d] = fmaxf(fmaxf(box.nmin[d] * lo, box.nmin[d] * hi),
+                                            fmaxf(box.nmax[d] * lo, box.nmax[d] * hi));
+                            back[d] = fmaxf(n[d] * lo, n[d] * hi);
+                        }
+                        // accepted pairs have n.d > 0 (t = -n.d / w.n > 0 with w.n < 0) and n_a.d > 0
+                        keep = !(dot_never_positive(recv[0], recv[1], recv[2]) ||
+                                 dot_never_positive(back[0], back[1], back[2]));
+                    }
+                    keep = keep || !(fabsf(q3.x) + fabsf(q3.y) + fabsf(q3.z) <= FLT_MAX);
+                }
+                const unsigned mk = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    float4* d = rec + 4 * __popc(mk & ((1u << lane) - 1u));
+                    d[0] = q0;
+                    d[1] = q1;
+                    d[2] = q2;
+                    d[3] = q3;
+                }
+                __syncwarp();
+                const int kept = __popc(mk);
+                for (int i = 0; i < kept; ++i) {
+                    const float4 r0 = rec[4 * i], r1 = rec[4 * i + 1], r2 = rec[4 * i + 2], r3 = rec[4 * i + 3];
+#pragma unroll
+                    for (int j = 0; j < PX; ++j) {
+                        float g, ga;
+                        pair_terms<ARC_AR_DISK, float>(r0, r1, r2, r3, px[j], a.pc, g, ga);
+                        // (0 times a non-finite antiradiance is added too, except by the clustered pass)
+                        const float x = r3.x * ga, y = r3.y * ga, z = r3.z * ga;
+                        if (ga != 0.0f || (!a.clustered && !(x == 0.0f && y == 0.0f && z == 0.0f))) {
+                            kahan_add(sum[j][0], comp[j][0], x);
+                            kahan_add(sum[j][1], comp[j][1], y);
+                            kahan_add(sum[j][2], comp[j][2], z);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+
+#pragma unroll
+    for (int j = 0; j < PX; ++j) {
+        const int x = xb + (j % kSub) * 8, y = yb + (j / kSub) * 4;
+        if (x >= a.width || y >= a.height) continue;
+        double ar[3] = {0.0, 0.0, 0.0};
+        if (mat[j] > 0) {
+            const float4 d = a.mats[mat[j]].diffuse_exp;
+            const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
+            for (int c = 0; c < 3; ++c)
+                ar[c] = (double)kd[c] * (double)a.disk_scale * ((double)sum[j][c] - (double)comp[j][c]);
+        }
+        const int64_t o = (int64_t)y * a.opitch + x;
+        if (a.out_ar) a.out_ar[o] = make_float4((float)ar[0], (float)ar[1], (float)ar[2], 1.0f);
+        if (a.out_ar64)
+            for (int c = 0; c < 3; ++c) a.out_ar64[3 * o + c] = ar[c];
+    }
+}
+
+}  // namespace
+
+arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* avpls, const ArcGBufferView* gb,
+                                    const ArcGatherParams* gp, bool clustered, float* out_ar, double* out_ar64,
+                                    int64_t opitch) {
+    const float4* records = nullptr;
+    ARC_TRY(launch_pack_records(ctx, avpls, &records));
+    DiskArgs a{};
+    a.records = records;
+    a.n = avpls->numAvpls;
+    float4* rays = nullptr;
+    ARC_TRY(ctx->arena.get("disk_rays", (size_t)(a.n + 1) * 2 * sizeof(float4), reinterpret_cast<void**>(&rays)));
+    a.rays = rays;
+    a.gpos = reinterpret_cast<const float4*>(gb->position);
+    a.gnrm = reinterpret_cast<const float4*>(gb->normal);
+    a.gpitch = gb->pitch;
+    a.width = gb->width;
+    a.height = gb->height;
+    a.mats = ctx->d_materials;
+    a.num_mats = ctx->num_materials;
+    a.pc.eps = 0.001f;
+    a.pc.inv_clamp2 = gp->dist_clamp > 0.0f ? 1.0f / (gp->dist_clamp * gp->dist_clamp) : INFINITY;
+    a.pc.disk_r2 = gp->disk_radius * gp->disk_radius;
+    a.radius = gp->disk_radius;
+    a.disk_scale = gp->disk_radius > 0.0f ? 1.0f / (kPi * gp->disk_radius * gp->disk_radius) : 0.0f;
+    a.clustered = clustered;
+    a.out_ar = reinterpret_cast<float4*>(out_ar);
+    a.out_ar64 = out_ar64;
+    a.opitch = opitch;
+    a.err = ctx->d_error;
+    cudaStream_t st = ctx->stream;
+    stage_begin(ctx, "disk_antiradiance");
+    if (a.n > 0) disk_rays<<<(a.n + 255) / 256, 256, 0, st>>>(records, a.n, rays);
+    const dim3 big((a.width + 31) / 32, (a.height + 31) / 32), small((a.width + 15) / 16, (a.height + 15) / 16);
+    if ((int64_t)big.x * big.y >= kBigTilesPerSm * ctx->sm_count)
+        disk_antiradiance<4><<<big, kThreads, 0, st>>>(a);
+    else
+        disk_antiradiance<1><<<small, kThreads, 0, st>>>(a);
+    stage_end(ctx, a.n > 0 ? 2 : 1);
+    ARC_TRY_CUDA(cudaGetLastError());
+    return ARC_OK;
+}
+
+}  // namespace arc

@@ -11,8 +11,9 @@
 //     memory with bulk asynchronous copies (cp.async.bulk, no multicast) on an mbarrier.
 //   * The default and the all-FP64 precision (no or cone antiradiance) test each staged record once
 //     against the tile's bounds and evaluate only the records that can add something to it
-//     (gather_bf_culled_kernel, pair_cull.cuh); the other precisions and the disk variant evaluate
-//     every pair (gather_bf_kernel).
+//     (gather_bf_culled_kernel, pair_cull.cuh), and the default precision's disk antiradiance is a
+//     culled pass of its own (disk_ar.cu); the other precisions, and every disk gather of the
+//     allocation-free entry point, evaluate every pair (gather_bf_kernel).
 //   * Radiance and antiradiance go to separate compensated sums (per-chunk FP32 partials folded
 //     into Kahan sums, or per-term Kahan) and are combined in FP64.
 // General path (specular materials or geometry-term limits): one thread per pixel evaluating the
@@ -110,8 +111,7 @@ __global__ void pack_bf_records(ArcAvplsGpuParam a, const MaterialRecord* mats, 
 }
 
 // PREC: 0 = chunk partials folded into Kahan sums, 1 = per-term Kahan, 2 = naive FP32, 3 = FP64.
-// RAD = false skips the radiance sums (antiradiance-only pass of the solid-angle cut path).
-template <int AR, int PREC, int PX, bool RAD = true>
+template <int AR, int PREC, int PX>
 __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
     using T = typename std::conditional<PREC == 3, double, float>::type;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -197,22 +197,18 @@ __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
                     T g, ga;
                     pair_terms<AR, T>(q0, q1, q2, q3, pix[j], k.pc, g, ga);
                     if (PREC == 1) {
-                        if (RAD) {
-                            kahan_add(ss[j][0], sc[j][0], (float)(q2.y * g));
-                            kahan_add(ss[j][1], sc[j][1], (float)(q2.z * g));
-                            kahan_add(ss[j][2], sc[j][2], (float)(q2.w * g));
-                        }
+                        kahan_add(ss[j][0], sc[j][0], (float)(q2.y * g));
+                        kahan_add(ss[j][1], sc[j][1], (float)(q2.z * g));
+                        kahan_add(ss[j][2], sc[j][2], (float)(q2.w * g));
                         if (AR != ARC_AR_NONE) {
                             kahan_add(ss[j][3], sc[j][3], (float)(q3.x * ga));
                             kahan_add(ss[j][4], sc[j][4], (float)(q3.y * ga));
                             kahan_add(ss[j][5], sc[j][5], (float)(q3.z * ga));
                         }
                     } else {
-                        if (RAD) {
-                            pix[j].r0 += (T)q2.y * g;
-                            pix[j].r1 += (T)q2.z * g;
-                            pix[j].r2 += (T)q2.w * g;
-                        }
+                        pix[j].r0 += (T)q2.y * g;
+                        pix[j].r1 += (T)q2.z * g;
+                        pix[j].r2 += (T)q2.w * g;
                         if (AR != ARC_AR_NONE) {
                             pix[j].a0 += (T)q3.x * ga;
                             pix[j].a1 += (T)q3.y * ga;
@@ -295,11 +291,6 @@ __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
             k.out_res64[3 * o + 0] = res[0];
             k.out_res64[3 * o + 1] = res[1];
             k.out_res64[3 * o + 2] = res[2];
-        }
-        if (k.out_ar64) {
-            k.out_ar64[3 * o + 0] = ar[0];
-            k.out_ar64[3 * o + 1] = ar[1];
-            k.out_ar64[3 * o + 2] = ar[2];
         }
     }
 }
@@ -787,10 +778,10 @@ constexpr int kBlocksPerSm = 24;
 constexpr int kMinChunks = 2;
 constexpr int64_t kPartialBytes = (int64_t)1 << 30;
 
-template <int AR, int PREC, int PX, bool RAD = true>
+template <int AR, int PREC, int PX>
 arc_status launch_fast(const BfArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)kStages * a.chunk * 64 + kStages * sizeof(uint64_t);
-    auto fn = gather_bf_kernel<AR, PREC, PX, RAD>;
+    auto fn = gather_bf_kernel<AR, PREC, PX>;
     if (smem > 48 * 1024) ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((a.width + kTileW - 1) / kTileW, (a.height + 16 * PX - 1) / (16 * PX));
     fn<<<grid, kThreads, smem, st>>>(a);
@@ -929,6 +920,20 @@ arc_status launch_gather_bruteforce(arc_context* ctx, const GatherLaunch& g) {
     ARC_TRY(pack_records(ctx, g, a));
     const int chosen = p.tile_config >= 0 ? p.tile_config : ctx->bf_tile_config;
     if (use_culled(p)) return run_culled(ctx, a, p, chosen, true);
+    if (p.ar_kind == ARC_AR_DISK && p.precision == ARC_PREC_KAHAN) {
+        // the radiance by the culled gather, the antiradiance by the culled disk pass
+        double *rad64 = nullptr, *ar64 = nullptr;
+        const size_t bytes = (size_t)gb.height * out.pitch * 3 * sizeof(double);
+        ARC_TRY(ctx->arena.get("bf_rad64", bytes, reinterpret_cast<void**>(&rad64)));
+        ARC_TRY(ctx->arena.get("bf_ar64", bytes, reinterpret_cast<void**>(&ar64)));
+        ArcGatherParams q = p;
+        q.ar_kind = ARC_AR_NONE;
+        a.out_res = a.out_ar = nullptr;
+        a.out_res64 = rad64;
+        ARC_TRY(run_culled(ctx, a, q, chosen, true));
+        ARC_TRY(launch_disk_antiradiance(ctx, g.avpls, &gb, &p, false, nullptr, ar64, out.pitch));
+        return launch_combine(ctx, rad64, ar64, gb.width, gb.height, &out);
+    }
     const TileShape ts = kTileShapes[chosen >= 0 ? chosen : kDefaultTileShape];
     a.chunk = ts.chunk;
     stage_begin(ctx, "bf_gather");
@@ -954,23 +959,18 @@ arc_status launch_pack_records(arc_context* ctx, const ArcAvplsGpuParam* avpls, 
 
 arc_status launch_antiradiance_only(arc_context* ctx, const GatherLaunch& g, double* ar64) {
     const ArcGatherParams& p = *g.params;
+    if (p.ar_kind == ARC_AR_DISK)
+        return launch_disk_antiradiance(ctx, g.avpls, g.gbuffer, &p, false, nullptr, ar64, g.out->pitch);
     BfArgs a = make_args(ctx, g);
     a.out_res = nullptr;
     a.out_rad = nullptr;
+    a.out_ar = nullptr;
     a.out_res64 = nullptr;
     a.out_ar64 = ar64;
-    cudaStream_t st = ctx->stream;
     ARC_TRY(pack_records(ctx, g, a));
-    if (p.ar_kind == ARC_AR_CONE) {
-        ArcGatherParams q = p;
-        q.precision = ARC_PREC_KAHAN;
-        return run_culled(ctx, a, q, -1, false);
-    }
-    a.chunk = kTileShapes[kDefaultTileShape].chunk;
-    stage_begin(ctx, "bf_antiradiance");
-    const arc_status s = launch_fast<ARC_AR_DISK, 0, 2, false>(a, st);
-    stage_end(ctx, 1);
-    return s;
+    ArcGatherParams q = p;
+    q.precision = ARC_PREC_KAHAN;
+    return run_culled(ctx, a, q, -1, false);
 }
 
 }  // namespace arc

@@ -104,3 +104,31 @@ def test_records_without_finite_radiance_are_not_dropped(ctx):
         want = _gather(ctx, pos, nrm, a, L.ARC_AR_CONE, L.ARC_PREC_NAIVE, 0.02)
         got = _gather(ctx, pos, nrm, a, L.ARC_AR_CONE, precision, 0.02)
         assert np.array_equal(np.isfinite(got[2]), np.isfinite(want[2]))
+
+
+@pytest.mark.parametrize("size", [(1, 1, 1), (16, 16, 1023), (17, 33, 1024), (40, 31, 1025), (70, 50, 5003),
+                                  (800, 800, 301)])
+def test_culled_disk_antiradiance_equals_every_pair(ctx, size):
+    """Each disk term is A or nothing, added in AVPL order with a compensated sum by both kernels: the
+    same sums, rounded once to float."""
+    for flat, radius in ((False, 0.2), (True, 0.03), (True, 0.2)):
+        pos, nrm, a = _inputs(*size, seed=sum(size) + flat, flat=flat)
+        mats = (L.ArcMaterial * 3)()
+        for i in range(3):
+            mats[i].diffuse = L.f3((0.9, 0.5 / (i + 1), 0.25))
+        ctx.upload_materials(mats)
+        dv, gb = ctx.upload_avpls(a), api.GBuffer(pos, nrm)
+        outs = []
+        for precision in (L.ARC_PREC_KAHAN_STRICT, L.ARC_PREC_KAHAN):
+            out = api.Outputs(size[0], size[1])
+            api.gather_bruteforce(ctx, dv, gb, (0.5, 0.5, -1.0),
+                                  api.gather_params(L.ARC_AR_DISK, 40.0, 0.02, radius, precision=precision), out)
+            assert ctx.synchronize() == 0
+            outs.append([t.cpu().numpy()[..., :3].astype(np.float64) for t in (out.antiradiance, out.radiance,
+                                                                                out.result, out.result64)])
+        want, got = outs
+        assert (want[0] > 0).any() or size[2] < 2
+        assert np.all(np.abs(got[0] - want[0]) <= 2.0 ** -22 * want[0])
+        # the result is the FP64 difference of the gather's own radiance and antiradiance
+        assert np.all(np.abs(got[3] - (got[1] - got[0])) <= 2.0 ** -23 * (got[1] + got[0]))
+        assert np.array_equal(got[2], got[3].astype(np.float32))
