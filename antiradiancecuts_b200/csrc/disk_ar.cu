@@ -4,15 +4,18 @@
 // A pair contributes only when the AVPL's ray p_a + s w (s > 0) passes within the disk radius of the
 // pixel, the AVPL lies in front of the pixel and the pixel behind the AVPL: a handful of AVPLs per
 // pixel.  A block owns a pixel tile and walks the AVPLs in order, kStep at a time:
-//   1. each thread tests AVPLs' rays against the tile's bounding sphere grown by the radius, and the
-//      block compacts the survivors in AVPL order;
-//   2. each warp tests survivors, one per lane, against its own pixels' sphere and their position and
-//      normal boxes, and stages the records that remain;
+//   1. each thread tests AVPLs' rays against the tile's bounding sphere grown by the radius, those that
+//      pass against each warp's sphere (a tile across a silhouette has a sphere as deep as the scene),
+//      and the block compacts the survivors in AVPL order;
+//   2. each warp tests its survivors, one per lane, against its pixels' position and normal boxes and
+//      stages the records that remain;
 //   3. every lane evaluates those for its pixels with the terms of pair_terms, in AVPL order, with one
 //      compensated sum per channel.
 // The tests drop a pair only when pair_terms is certain to give 0 (their margins exceed its rounding),
-// so the sums are those over every AVPL.  The work left is the ray tests, 20 operations per (tile,
+// so the sums are those over every AVPL.  Several blocks share a tile, each with a segment of the AVPLs
+// (tiles differ widely in work); disk_combine adds their sums in FP64.  The work left is the ray tests, 20 operations per (tile,
 // AVPL) instead of 45 per (pixel, AVPL).
+#include <algorithm>
 #include <cfloat>
 
 #include "arc_internal.h"
@@ -28,12 +31,20 @@ constexpr int kPerThread = 4;                     // rays tested per thread and 
 constexpr int kStep = kThreads * kPerThread;      // AVPLs per step
 static_assert(kPerThread * kWarps == 32, "one lane per (pass, warp) count in the block's prefix sum");
 
-// 32 x 32 tiles when they make at least this many blocks per SM, else 16 x 16
-constexpr int64_t kBigTilesPerSm = 4;
+// 32 x 32 tiles when they make at least this many blocks per SM (a quarter of the ray tests; 1280 x 720 x
+// 65,536: 0.92 against 1.34 ms), else 16 x 16 (more, smaller blocks).
+constexpr int64_t kBigTilesPerSm = 2;
+// Segments: a tile across a silhouette sees a third of all rays and takes 40 times the mean, so the
+// AVPLs are split until there are this many blocks per SM (512 x 512 x 32,768 / 1280 x 720 x 65,536: 0.49 /
+// 1.29 ms at 16 per SM, 0.42 / 0.92 ms at 64, 0.46 ms at 128, where the blocks' set-up costs more than the
+// balance gains), partial sums within kPartialBytes.
+constexpr int64_t kBlocksPerSm = 64;
+constexpr int64_t kPartialBytes = (int64_t)1 << 30;
 
 struct DiskArgs {
     const float4* records;  // 4 float4 per AVPL (launch_pack_records)
-    const float4* rays;     // 2 float4 per AVPL: {p, > 0 when it can contribute}, {w / |w|, 0}
+    // 2 float4 per AVPL: {p, 0: adds nothing, > 0: adds where its ray passes, < 0: to every pixel}, {w / |w|, 0}
+    const float4* rays;
     int n;
     const float4* gpos;
     const float4* gnrm;
@@ -47,6 +58,7 @@ struct DiskArgs {
     bool clustered;   // surface pixels as the clustered pass has them (normal.w > 0)
     float4* out_ar;
     double* out_ar64; // 3 per pixel
+    double* partial;  // several segments: [channel][segment][height][width]
     int64_t opitch;
     uint32_t* err;
 };
@@ -60,7 +72,7 @@ __global__ void disk_rays(const float4* records, int n, float4* rays) {
                  q3 = records[4 * (size_t)i + 3];
     const float la = fabsf(q3.x) + fabsf(q3.y) + fabsf(q3.z);
     const bool never = la == 0.0f || (la <= FLT_MAX && q1.z == 0.0f && q1.w == 0.0f && q2.x == 0.0f);
-    rays[2 * (size_t)i] = make_float4(q0.x, q0.y, q0.z, never ? 0.0f : 1.0f);
+    rays[2 * (size_t)i] = make_float4(q0.x, q0.y, q0.z, never ? 0.0f : la <= FLT_MAX ? 1.0f : -1.0f);
     rays[2 * (size_t)i + 1] = make_float4(q1.z * q3.w, q1.w * q3.w, q2.x * q3.w, 0.0f);
 }
 
@@ -74,12 +86,28 @@ __device__ __forceinline__ bool ray_near(float4 r0, float4 r1, float cx, float c
     return !(hx * hx + hy * hy + hz * hz > reach * reach);
 }
 
+// A pixel's antiradiance from its FP64 sums; 0 without a surface (material 0).
+__device__ __forceinline__ void write_ar(const DiskArgs& a, int x, int y, int mat, const double* S) {
+    double ar[3] = {0.0, 0.0, 0.0};
+    if (mat > 0) {
+        const float4 d = a.mats[mat].diffuse_exp;
+        const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
+        for (int c = 0; c < 3; ++c) ar[c] = (double)kd[c] * (double)a.disk_scale * S[c];
+    }
+    const int64_t o = (int64_t)y * a.opitch + x;
+    if (a.out_ar) a.out_ar[o] = make_float4((float)ar[0], (float)ar[1], (float)ar[2], 1.0f);
+    if (a.out_ar64)
+        for (int c = 0; c < 3; ++c) a.out_ar64[3 * o + c] = ar[c];
+}
+
 // PX = 1: 16 x 16 pixel tiles, 8 x 4 pixels per warp; PX = 4: 32 x 32 tiles, 16 x 8 per warp.
 template <int PX>
 __global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
-    constexpr int kSide = PX == 1 ? 16 : 32, kSub = PX == 1 ? 1 : 2;
+    constexpr int kSide = PX == 1 ? 16 : 32, kSub = PX == 1 ? 1 : 2, kIlp = 4 / PX;
     __shared__ float4 s_rec[kWarps][32 * 4];
     __shared__ int s_list[kStep];
+    __shared__ unsigned char s_who[kStep];  // the warps that an entry of the list concerns
+    __shared__ float4 s_ball[kWarps];       // each warp's bounding sphere (radius < 0: no pixels)
     __shared__ int s_cnt[32];
     __shared__ PixelBounds s_box[kWarps];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -140,18 +168,29 @@ __global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
         float tcx, tcy, tcz, wcx, wcy, wcz;
         const float trho = sphere(tb, tcx, tcy, tcz);
         const float wrho = sphere(box, wcx, wcy, wcz);
+        if (lane == 0) s_ball[w] = make_float4(wcx, wcy, wcz, warp_live ? wrho : -1.0f);
+        __syncthreads();
         float4* rec = s_rec[w];
-        for (int base = 0; base < a.n; base += kStep) {
-            unsigned m[kPerThread];
+        const int steps = (a.n + kStep - 1) / kStep;
+        const int first = (int)((int64_t)steps * blockIdx.z / gridDim.z) * kStep,
+                  last = (int)min((int64_t)a.n, (int64_t)steps * (blockIdx.z + 1) / gridDim.z * kStep);
+        for (int base = first; base < last; base += kStep) {
+            unsigned m[kPerThread], who[kPerThread];
 #pragma unroll
             for (int u = 0; u < kPerThread; ++u) {
                 const int i = base + u * kThreads + tid;
-                bool near = false;
-                if (i < a.n) {
+                who[u] = 0;
+                if (i < last) {
                     const float4 r0 = a.rays[2 * (size_t)i], r1 = a.rays[2 * (size_t)i + 1];
-                    near = r0.w != 0.0f && ray_near(r0, r1, tcx, tcy, tcz, trho);
+                    if (r0.w < 0.0f || (r0.w > 0.0f && ray_near(r0, r1, tcx, tcy, tcz, trho)))
+#pragma unroll 1
+                        for (int q = 0; q < kWarps; ++q) {
+                            const float4 ball = s_ball[q];
+                            if (ball.w >= 0.0f && (r0.w < 0.0f || ray_near(r0, r1, ball.x, ball.y, ball.z, ball.w)))
+                                who[u] |= 1u << q;
+                        }
                 }
-                m[u] = __ballot_sync(0xffffffffu, near);
+                m[u] = __ballot_sync(0xffffffffu, who[u] != 0);
                 if (lane == 0) s_cnt[u * kWarps + w] = __popc(m[u]);
             }
             __syncthreads();  // the counts; and every warp is done with the list of the step before
@@ -165,23 +204,25 @@ __global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
             const int count = __shfl_sync(0xffffffffu, incl, 31);
 #pragma unroll
             for (int u = 0; u < kPerThread; ++u) {
-                const int first = __shfl_sync(0xffffffffu, excl, u * kWarps + w);
-                if (m[u] >> lane & 1u) s_list[first + __popc(m[u] & ((1u << lane) - 1u))] = base + u * kThreads + tid;
+                const int at = __shfl_sync(0xffffffffu, excl, u * kWarps + w) + __popc(m[u] & ((1u << lane) - 1u));
+                if (who[u]) {
+                    s_list[at] = base + u * kThreads + tid;
+                    s_who[at] = (unsigned char)who[u];
+                }
             }
             __syncthreads();
             if (!warp_live) continue;
             for (int k = 0; k < count; k += 32) {
                 float4 q0, q1, q2, q3;
                 bool keep = false;
-                if (k + lane < count) {
+                if (k + lane < count && (s_who[k + lane] >> w & 1)) {
                     const int i = s_list[k + lane];
                     const float4* q = a.records + 4 * (size_t)i;
                     q0 = q[0];
                     q1 = q[1];
                     q2 = q[2];
                     q3 = q[3];
-                    keep = ray_near(q0, make_float4(q1.z * q3.w, q1.w * q3.w, q2.x * q3.w, 0.0f), wcx, wcy, wcz, wrho);
-                    if (keep) {
+                    {
                         const float p[3] = {q0.x, q0.y, q0.z}, n[3] = {q0.w, q1.x, q1.y};
                         float recv[3], back[3];
 #pragma unroll
@@ -207,18 +248,32 @@ __global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
                 }
                 __syncwarp();
                 const int kept = __popc(mk);
-                for (int i = 0; i < kept; ++i) {
-                    const float4 r0 = rec[4 * i], r1 = rec[4 * i + 1], r2 = rec[4 * i + 2], r3 = rec[4 * i + 3];
+                // kIlp records at a time: their tests are independent, the sums then take them in order
+                for (int i = 0; i < kept; i += kIlp) {
+                    float hit[kIlp][PX];
 #pragma unroll
-                    for (int j = 0; j < PX; ++j) {
-                        float g, ga;
-                        pair_terms<ARC_AR_DISK, float>(r0, r1, r2, r3, px[j], a.pc, g, ga);
-                        // (0 times a non-finite antiradiance is added too, except by the clustered pass)
-                        const float x = r3.x * ga, y = r3.y * ga, z = r3.z * ga;
-                        if (ga != 0.0f || (!a.clustered && !(x == 0.0f && y == 0.0f && z == 0.0f))) {
-                            kahan_add(sum[j][0], comp[j][0], x);
-                            kahan_add(sum[j][1], comp[j][1], y);
-                            kahan_add(sum[j][2], comp[j][2], z);
+                    for (int u = 0; u < kIlp; ++u) {
+                        const float4* r = rec + 4 * min(i + u, kept - 1);
+                        const float4 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
+#pragma unroll
+                        for (int j = 0; j < PX; ++j) {
+                            float g;
+                            pair_terms<ARC_AR_DISK, float>(r0, r1, r2, r3, px[j], a.pc, g, hit[u][j]);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < kIlp; ++u) {
+                        if (i + u >= kept) break;
+                        const float4 r3 = rec[4 * (i + u) + 3];
+#pragma unroll
+                        for (int j = 0; j < PX; ++j) {
+                            // (0 times a non-finite antiradiance is added too, except by the clustered pass)
+                            const float ga = hit[u][j], x = r3.x * ga, y = r3.y * ga, z = r3.z * ga;
+                            if (ga != 0.0f || (!a.clustered && !(x == 0.0f && y == 0.0f && z == 0.0f))) {
+                                kahan_add(sum[j][0], comp[j][0], x);
+                                kahan_add(sum[j][1], comp[j][1], y);
+                                kahan_add(sum[j][2], comp[j][2], z);
+                            }
                         }
                     }
                 }
@@ -231,18 +286,33 @@ __global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
     for (int j = 0; j < PX; ++j) {
         const int x = xb + (j % kSub) * 8, y = yb + (j / kSub) * 4;
         if (x >= a.width || y >= a.height) continue;
-        double ar[3] = {0.0, 0.0, 0.0};
-        if (mat[j] > 0) {
-            const float4 d = a.mats[mat[j]].diffuse_exp;
-            const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
-            for (int c = 0; c < 3; ++c)
-                ar[c] = (double)kd[c] * (double)a.disk_scale * ((double)sum[j][c] - (double)comp[j][c]);
+        double S[3];
+        for (int c = 0; c < 3; ++c) S[c] = (double)sum[j][c] - (double)comp[j][c];
+        if (gridDim.z > 1) {
+            double* d = a.partial + ((int64_t)blockIdx.z * a.height + y) * a.width + x;
+            const int64_t plane = (int64_t)gridDim.z * a.height * a.width;
+            if (mat[j] > 0)  // (other pixels are written by disk_combine alone)
+                for (int c = 0; c < 3; ++c) d[c * plane] = S[c];
+        } else {
+            write_ar(a, x, y, mat[j], S);
         }
-        const int64_t o = (int64_t)y * a.opitch + x;
-        if (a.out_ar) a.out_ar[o] = make_float4((float)ar[0], (float)ar[1], (float)ar[2], 1.0f);
-        if (a.out_ar64)
-            for (int c = 0; c < 3; ++c) a.out_ar64[3 * o + c] = ar[c];
     }
+}
+
+// The segments' sums of every pixel added in segment order, and the outputs.
+__global__ void __launch_bounds__(kThreads) disk_combine(DiskArgs a, int segments) {
+    const int x = blockIdx.x * 32 + threadIdx.x % 32, y = blockIdx.y * (kThreads / 32) + threadIdx.x / 32;
+    if (x >= a.width || y >= a.height) return;
+    int m = (int)a.gnrm[(int64_t)y * a.gpitch + x].w;
+    if (m < 0 || m >= a.num_mats) m = 0;
+    double S[3] = {0.0, 0.0, 0.0};
+    if (m > 0) {
+        const int64_t image = (int64_t)a.height * a.width;
+        const double* d = a.partial + (int64_t)y * a.width + x;
+        for (int s = 0; s < segments; ++s)
+            for (int c = 0; c < 3; ++c) S[c] += d[(c * segments + s) * image];
+    }
+    write_ar(a, x, y, m, S);
 }
 
 }  // namespace
@@ -278,12 +348,23 @@ arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* av
     cudaStream_t st = ctx->stream;
     stage_begin(ctx, "disk_antiradiance");
     if (a.n > 0) disk_rays<<<(a.n + 255) / 256, 256, 0, st>>>(records, a.n, rays);
-    const dim3 big((a.width + 31) / 32, (a.height + 31) / 32), small((a.width + 15) / 16, (a.height + 15) / 16);
-    if ((int64_t)big.x * big.y >= kBigTilesPerSm * ctx->sm_count)
-        disk_antiradiance<4><<<big, kThreads, 0, st>>>(a);
+    dim3 grid((a.width + 31) / 32, (a.height + 31) / 32);
+    const bool big = (int64_t)grid.x * grid.y >= kBigTilesPerSm * ctx->sm_count;
+    if (!big) grid = dim3((a.width + 15) / 16, (a.height + 15) / 16);
+    const int64_t blocks = (int64_t)grid.x * grid.y, image = (int64_t)a.width * a.height;
+    grid.z = (unsigned)std::max<int64_t>(
+        1, std::min({(kBlocksPerSm * ctx->sm_count + blocks - 1) / blocks, ((int64_t)a.n + kStep - 1) / kStep,
+                     kPartialBytes / (image * 3 * (int64_t)sizeof(double))}));
+    if (grid.z > 1)
+        ARC_TRY(ctx->arena.get("disk_partial", (size_t)(image * 3 * grid.z) * sizeof(double),
+                               reinterpret_cast<void**>(&a.partial)));
+    if (big)
+        disk_antiradiance<4><<<grid, kThreads, 0, st>>>(a);
     else
-        disk_antiradiance<1><<<small, kThreads, 0, st>>>(a);
-    stage_end(ctx, a.n > 0 ? 2 : 1);
+        disk_antiradiance<1><<<grid, kThreads, 0, st>>>(a);
+    if (grid.z > 1)
+        disk_combine<<<dim3((a.width + 31) / 32, (a.height + 7) / 8), kThreads, 0, st>>>(a, (int)grid.z);
+    stage_end(ctx, (a.n > 0 ? 2 : 1) + (grid.z > 1));
     ARC_TRY_CUDA(cudaGetLastError());
     return ARC_OK;
 }
