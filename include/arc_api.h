@@ -122,7 +122,8 @@ typedef enum arc_ar_kind {
 } arc_ar_kind;
 
 typedef enum arc_precision {
-    ARC_PREC_KAHAN = 0,        /* FP32 terms, per-chunk FP32 partials folded into Kahan sums, FP64 combine (default) */
+    ARC_PREC_KAHAN = 0,        /* FP32 terms, per-chunk FP32 partials folded into FP64 (no / cone antiradiance) or
+                                  compensated FP32 sums, FP64 combine (default) */
     ARC_PREC_KAHAN_STRICT = 1, /* FP32 terms, every term Kahan-added, FP64 combine */
     ARC_PREC_NAIVE = 2,        /* FP32 terms, plain FP32 sums, FP32 combine (the reference's arithmetic) */
     ARC_PREC_FP64 = 3          /* every operation in FP64 */
