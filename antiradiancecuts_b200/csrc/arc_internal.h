@@ -186,9 +186,10 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
                              const ArcOutputView* out);
 arc_status launch_antiradiance_only(arc_context* ctx, const GatherLaunch& g, double* ar64);
 // per-tile set-up of the tile cuts (bounds, normal cone, albedo, coarse estimate, threshold) and
-// the per-node parts of the cut bound (NodeExtra, two float4 per inner node)
+// the per-node parts of the cut bound (NodeExtra, two float4 per inner node); estimate (optional):
+// the error-bound selection's expected cut size per tile
 arc_status launch_tile_setup(arc_context* ctx, const arc_lbvh* bvh, const ArcGBufferView* gb, const ArcGatherParams* gp,
-                             const ArcCutParams* cp, float4** info_out, float4** extra_out);
+                             const ArcCutParams* cp, float4** info_out, float4** extra_out, int* estimate);
 
 }  // namespace arc
 

@@ -36,8 +36,10 @@ namespace {
 constexpr int kTile = 8;
 constexpr int kSolidStack = 64;
 constexpr int kChunkSize = 1024;  // cut entries per pool chunk
-constexpr int kSelWarps = 4;
-constexpr int kSelStack = 4096;
+constexpr int kSetupWarps = 4;
+constexpr int kSelThreads = 128;
+constexpr int kSelStack = 8192;  // nodes waiting per tile
+constexpr int kSelBlocksPerSm = 6;
 constexpr int kCoarseDepth = 5;
 
 struct MatSmem {
@@ -216,6 +218,10 @@ struct TileArgs {
     float clamp2;
     int tiles_x, tiles_y;
     float4* info;  // [tiles][4]
+    // expected cut size of the error-bound selection per tile (optional), from:
+    int* estimate;
+    const float4* extra;  // NodeExtra per inner node
+    BoundParams bp;
     uint32_t* err;
 };
 
@@ -230,14 +236,14 @@ __device__ __forceinline__ float coarse_g(float px, float py, float pz, float nx
     return rn_div(rn_mul(c1, c2), fmaxf(l2, clamp2));
 }
 
-__global__ void __launch_bounds__(32 * kSelWarps) cut_tile_setup(TileArgs a) {
-    __shared__ float sp[kSelWarps][64][7];  // p.xyz, n.xyz, valid
-    __shared__ float skd[kSelWarps][64][3];
-    __shared__ float sest[kSelWarps][64];
-    __shared__ int scoarse[kSelWarps][1 << kCoarseDepth];
-    __shared__ int sncoarse[kSelWarps];
+__global__ void __launch_bounds__(32 * kSetupWarps) cut_tile_setup(TileArgs a) {
+    __shared__ float sp[kSetupWarps][64][7];  // p.xyz, n.xyz, valid
+    __shared__ float skd[kSetupWarps][64][3];
+    __shared__ float sest[kSetupWarps][64];
+    __shared__ int scoarse[kSetupWarps][1 << kCoarseDepth];
+    __shared__ int sncoarse[kSetupWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * kSelWarps + warp;
+    const int tile = blockIdx.x * kSetupWarps + warp;
     if (tile >= a.tiles_x * a.tiles_y) return;
     const int tx0 = (tile % a.tiles_x) * kTile, ty0 = (tile / a.tiles_x) * kTile;
     float tmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, tmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
@@ -323,6 +329,7 @@ __global__ void __launch_bounds__(32 * kSelWarps) cut_tile_setup(TileArgs a) {
         sest[warp][i] = est;
     }
     __syncwarp();
+    TileInfo ti;
     if (lane == 0) {
         float sum = 0.0f;
         float4 cone = make_float4(0, 0, 0, -2.0f);  // -2: empty
@@ -365,6 +372,39 @@ __global__ void __launch_bounds__(32 * kSelWarps) cut_tile_setup(TileArgs a) {
         info[3] = make_float4(__int_as_float(nvalid), mean,
                               half_diagonal(rn_sub(tmax[0], tmin[0]), rn_sub(tmax[1], tmin[1]), rn_sub(tmax[2], tmin[2])),
                               cone_sine(cone.w));
+        ti.ncone = cone;
+        ti.tau = rn_mul(a.eps_bound, mean);
+        ti.sn = cone_sine(cone.w);
+    }
+    if (a.estimate) {
+        // A node whose bound is M contributes about M / tau nodes to the cut (its parts' bounds add up
+        // to M and each stays below tau), at most its leaves; one coarse node per lane.
+        ti.ncone.x = __shfl_sync(0xffffffffu, ti.ncone.x, 0);
+        ti.ncone.y = __shfl_sync(0xffffffffu, ti.ncone.y, 0);
+        ti.ncone.z = __shfl_sync(0xffffffffu, ti.ncone.z, 0);
+        ti.ncone.w = __shfl_sync(0xffffffffu, ti.ncone.w, 0);
+        ti.tau = __shfl_sync(0xffffffffu, ti.tau, 0);
+        ti.sn = __shfl_sync(0xffffffffu, ti.sn, 0);
+        for (int k = 0; k < 3; ++k) {
+            ti.tmin[k] = tmin[k];
+            ti.tmax[k] = tmax[k];
+        }
+        ti.kdl = kdl;
+        ti.valid = nvalid;
+        ti.rt = half_diagonal(tmax[0] - tmin[0], tmax[1] - tmin[1], tmax[2] - tmin[2]);
+        float e = 0.0f;
+        if (nvalid > 0 && lane < ncoarse) {
+            const int node = scoarse[warp][lane];
+            e = 1.0f;
+            if (node >= a.n) {
+                const int k = node - a.n;
+                const float4* b = a.bounds + 4 * (size_t)k;
+                const float m = node_bound_fast(ti, b[0], b[1], b[2], b[3], load_node_extra(a.extra, k), a.bp).m;
+                e = fminf(a.records[4 * (size_t)node + 3].w, fmaxf(1.0f, m / ti.tau));
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+        if (lane == 0) a.estimate[tile] = (int)fminf(e, 1e9f);
     }
 }
 
@@ -394,122 +434,7 @@ __device__ __forceinline__ TileInfo load_tile(const float4* info, int tile) {
     return t;
 }
 
-// ---------------------------------------------------------------------------------------
-// Error-bound cut selection: one warp per tile
-// ---------------------------------------------------------------------------------------
-struct SelArgs {
-    int n;
-    const float4* bounds;
-    const float4* records;
-    const float4* info;
-    const float4* extra;  // NodeExtra per inner node
-    BoundParams bp;
-    int tiles;
-    CutPool pool;
-    uint32_t* err;
-};
-
-__global__ void __launch_bounds__(32 * kSelWarps) cut_select_bound(SelArgs a) {
-    extern __shared__ int sstack[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * kSelWarps + warp;
-    if (tile >= a.tiles) return;
-    int* stack = sstack + warp * kSelStack;
-    const TileInfo t = load_tile(a.info, tile);
-    CutWriter cw(a.pool, tile);
-    if (t.valid == 0) {
-        if (lane == 0) a.pool.counts[tile] = 0;
-        return;
-    }
-    const unsigned lt = (1u << lane) - 1u;
-    int sp = 1;
-    if (lane == 0) stack[0] = a.n;  // root
-    __syncwarp();
-    bool overflow = false;
-    int budget = 2 * a.n;  // node visits of a valid tree
-    while (sp > 0) {
-        if (budget <= 0) {
-            if (lane == 0) set_error(a.err, ARC_DEVERR_BAD_NODE);
-            break;
-        }
-        const int m = min(32, sp);
-        budget -= m;
-        int node = -1;
-        if (lane < m) node = stack[sp - 1 - lane];
-        __syncwarp();
-        sp -= m;
-        bool accept = false, refine = false;
-        int lc = 0, rc = 0;
-        if (lane < m) {
-            if (node < a.n) {
-                accept = node >= 0;
-            } else {
-                const int k = node - a.n;
-                const float4 b0 = a.bounds[4 * (size_t)k], b1 = a.bounds[4 * (size_t)k + 1];
-                const float4 nc = a.bounds[4 * (size_t)k + 2], wc = a.bounds[4 * (size_t)k + 3];
-                const NodeExtra ne = load_node_extra(a.extra, k);
-                const NodeGeom g = node_geom(t, b0, b1, nc, wc, ne, a.bp);
-                const float M = node_bound(t, g, ne.Ls, ne.As, a.bp);
-                if (M > t.tau) {
-                    refine = true;
-                    const int l = __float_as_int(b0.w), r = __float_as_int(b1.w);
-                    lc = l >= 0 ? l : a.n - (l + 1);
-                    rc = r >= 0 ? r : a.n - (r + 1);
-                } else {
-                    accept = true;
-                }
-            }
-        }
-        unsigned rmask = __ballot_sync(0xffffffffu, refine);
-        const int nref = __popc(rmask);
-        if (sp + 2 * nref > kSelStack) {  // no room: use the nodes whole
-            if (refine) {
-                refine = false;
-                accept = true;
-            }
-            rmask = 0;
-            overflow = true;
-        }
-        const unsigned amask = __ballot_sync(0xffffffffu, accept);
-        cw.append(amask, accept, node, lane);
-        if (refine) {
-            const int q = sp + 2 * __popc(rmask & lt);
-            stack[q] = rc;
-            stack[q + 1] = lc;
-        }
-        sp += 2 * __popc(rmask);
-        __syncwarp();
-    }
-    if (lane == 0) {
-        if (cw.overflow || overflow) set_error(a.err, ARC_DEVERR_CUT_OVERFLOW);
-        a.pool.counts[tile] = cw.count;
-    }
-}
-
-// ---------------------------------------------------------------------------------------
-// Cut evaluation: one 64-thread block per tile, one pixel per thread
-// ---------------------------------------------------------------------------------------
-struct EvalArgs {
-    const float4* gpos;
-    const float4* gnrm;
-    int64_t gpitch;
-    int width, height;
-    const MaterialRecord* mats;
-    int num_mats;
-    const float4* records;
-    int tiles_x;
-    CutPool pool;
-    PairConsts pc;
-    float disk_scale;
-    float4* out_res;
-    float4* out_rad;
-    float4* out_ar;
-    double* out_res64;
-    int64_t opitch;
-    const int* order;  // block b evaluates tile order[b]
-};
-
-// Tiles in decreasing order of cut size (buckets of floor(log2(count)), empty tiles last), so that
+// Tiles in decreasing order of (expected) cut size (buckets of floor(log2(count)), empty tiles last), so that
 // the blocks with the longest cuts start first and the short ones fill the tail of the launch.
 // One block; the order within a bucket is arbitrary (each tile's result does not depend on it).
 __global__ void __launch_bounds__(1024) tile_order_kernel(const int32_t* counts, int tiles, int* order) {
@@ -535,6 +460,183 @@ __global__ void __launch_bounds__(1024) tile_order_kernel(const int32_t* counts,
         order[atomicAdd(&off[c > 0 ? 32 - __clz(c) : 0], 1)] = i;
     }
 }
+
+// ---------------------------------------------------------------------------------------
+// Error-bound cut selection: one block per tile at a time, tiles from a work counter
+// ---------------------------------------------------------------------------------------
+struct SelArgs {
+    int n;
+    const float4* bounds;
+    const float4* records;
+    const float4* info;
+    const float4* extra;  // NodeExtra per inner node
+    BoundParams bp;
+    int tiles;
+    const int* order;     // tiles, largest expected cut first
+    int* next_tile;       // tiles handed out
+    CutPool pool;
+    uint32_t* err;
+};
+
+// The rounded bound of (tile, inner node k), for the pairs that node_bound_fast leaves open.
+__device__ __noinline__ float rounded_bound(const float4* info, int tile, const float4* bounds, const float4* extra,
+                                            int k, const BoundParams& bp) {
+    const TileInfo t = load_tile(info, tile);
+    const NodeExtra ne = load_node_extra(extra, k);
+    const float4* b = bounds + 4 * (size_t)k;
+    const NodeGeom g = node_geom(t, b[0], b[1], b[2], b[3], ne, bp);
+    return node_bound(t, g, ne.Ls, ne.As, bp);
+}
+
+// A tile's walk: the block pops up to 128 nodes of a shared stack, one per thread, appends the accepted
+// ones to the tile's list in the cut pool and pushes the others' children.  Four warps share a walk
+// because the largest tiles take 10 times the mean (with one warp per tile the last of them ran
+// alone for a quarter of the launch), and tiles start in decreasing order of their expected cut.  A
+// step pops all it can, so the stack grows by at most 128 nodes per level of the tree: kSelStack holds
+// trees of 62 levels, and Morton codes of 32 bits over 2^25 leaves make 57.
+//
+// Bound by instruction issue and latency (56% issue, ALU 49%, 390 instructions per 32 nodes).  1280 x 720 x
+// 65,536 AVPLs, bound 0.01: 5.0 ms with one warp per tile and 12 warps per SM (16 KB of stack each), 3.8 ms
+// with 28, 3.5 ms with the approximate bound, 3.2 ms with the expected cuts first, 2.9 ms as it is.
+__global__ void __launch_bounds__(kSelThreads, kSelBlocksPerSm) cut_select_bound(SelArgs a) {
+    constexpr int kW = kSelThreads / 32;
+    __shared__ int stack[kSelStack];
+    __shared__ int s_acc[2][kW], s_ref[2][kW];
+    __shared__ int s_tile, s_chunk;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    for (;;) {
+        if (tid == 0) {
+            const int i = atomicAdd(a.next_tile, 1);
+            s_tile = i < a.tiles ? a.order[i] : -1;
+            stack[0] = a.n;  // root
+        }
+        __syncthreads();
+        const int tile = s_tile;
+        if (tile < 0) return;
+        const TileInfo t = load_tile(a.info, tile);
+        int32_t* table = a.pool.tables + (size_t)tile * a.pool.max_chunks;
+        int count = 0, chunk = -1;  // list length; pool chunk of its last entry
+        bool overflow = false;
+        int sp = t.valid ? 1 : 0;
+        int budget = 2 * a.n;  // node visits of a valid tree
+        for (int turn = 0; sp > 0; turn ^= 1) {
+            if (budget <= 0) {
+                if (tid == 0) set_error(a.err, ARC_DEVERR_BAD_NODE);
+                break;
+            }
+            const int m = min(kSelThreads, sp);
+            budget -= m;
+            sp -= m;
+            int node = -1, lc = 0, rc = 0;
+            bool accept = false, refine = false;
+            if (tid < m) {
+                node = stack[sp + m - 1 - tid];
+                if (node < a.n) {
+                    accept = node >= 0;
+                } else {
+                    const int k = node - a.n;
+                    const float4 b0 = a.bounds[4 * (size_t)k], b1 = a.bounds[4 * (size_t)k + 1];
+                    const float4 nc = a.bounds[4 * (size_t)k + 2], wc = a.bounds[4 * (size_t)k + 3];
+                    const NodeExtra ne = load_node_extra(a.extra, k);
+                    int over = exceeds(node_bound_fast(t, b0, b1, nc, wc, ne, a.bp), t.tau);
+                    if (over < 0) over = rounded_bound(a.info, tile, a.bounds, a.extra, k, a.bp) > t.tau;
+                    refine = over != 0;
+                    accept = over == 0;
+                    const int l = __float_as_int(b0.w), r = __float_as_int(b1.w);
+                    lc = l >= 0 ? l : a.n - (l + 1);
+                    rc = r >= 0 ? r : a.n - (r + 1);
+                }
+            }
+            unsigned am = __ballot_sync(0xffffffffu, accept);
+            const unsigned rm = __ballot_sync(0xffffffffu, refine);
+            if (lane == 0) {
+                s_acc[turn][warp] = __popc(am);
+                s_ref[turn][warp] = __popc(rm);
+            }
+            __syncthreads();  // the counts; and every popped node has been read
+            int before_a = 0, before_r = 0, na = 0, nref = 0;
+#pragma unroll
+            for (int q = 0; q < kW; ++q) {
+                const int x = s_acc[turn][q], y = s_ref[turn][q];
+                if (q < warp) {
+                    before_a += x;
+                    before_r += y;
+                }
+                na += x;
+                nref += y;
+            }
+            if (sp + 2 * nref > kSelStack) {  // no room: use the nodes whole
+                accept = accept || refine;
+                refine = false;
+                am |= rm;
+                before_a += before_r;
+                na += nref;
+                nref = 0;
+                overflow = true;
+            }
+            if (na > 0) {  // append to the list, which starts at most one new chunk (128 < kChunkSize)
+                const int first_new = (count + kChunkSize - 1) / kChunkSize, last = (count + na - 1) / kChunkSize;
+                const bool fresh = last >= first_new;
+                int id = chunk;
+                if (fresh) {
+                    if (tid == 0) {
+                        const int c = last < a.pool.max_chunks ? atomicAdd(a.pool.next, 1) : a.pool.num_chunks;
+                        if (c < a.pool.num_chunks) table[last] = c;
+                        s_chunk = c;
+                    }
+                    __syncthreads();
+                    id = s_chunk;
+                }
+                if (accept) {
+                    const int pos = count + before_a + __popc(am & lt);
+                    const int c = pos / kChunkSize == last && fresh ? id : chunk;
+                    if (c >= 0 && c < a.pool.num_chunks)
+                        a.pool.entries[(size_t)c * kChunkSize + pos % kChunkSize] = node;
+                }
+                chunk = id;
+                if (fresh && id >= a.pool.num_chunks) overflow = true;
+                // (past the pool only the entries that landed in a chunk are kept)
+                count = chunk >= a.pool.num_chunks ? min(count + na, last * kChunkSize) : count + na;
+            }
+            if (refine) {
+                const int q = sp + 2 * (before_r + __popc(rm & lt));
+                stack[q] = rc;
+                stack[q + 1] = lc;
+            }
+            sp += 2 * nref;
+            __syncthreads();  // the pushes
+        }
+        if (tid == 0) {
+            if (overflow) set_error(a.err, ARC_DEVERR_CUT_OVERFLOW);
+            a.pool.counts[tile] = count;
+        }
+        __syncthreads();  // every thread has read s_tile and left the stack
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// Cut evaluation: one 64-thread block per tile, one pixel per thread
+// ---------------------------------------------------------------------------------------
+struct EvalArgs {
+    const float4* gpos;
+    const float4* gnrm;
+    int64_t gpitch;
+    int width, height;
+    const MaterialRecord* mats;
+    int num_mats;
+    const float4* records;
+    int tiles_x;
+    CutPool pool;
+    PairConsts pc;
+    float disk_scale;
+    float4* out_res;
+    float4* out_rad;
+    float4* out_ar;
+    double* out_res64;
+    int64_t opitch;
+    const int* order;  // block b evaluates tile order[b]
+};
 
 template <int AR>
 __global__ void __launch_bounds__(64) cut_eval_kernel(EvalArgs a) {
@@ -840,7 +942,7 @@ arc_status launch_combine(arc_context* ctx, const double* rad64, const double* a
 }
 
 arc_status launch_tile_setup(arc_context* ctx, const arc_lbvh* bvh, const ArcGBufferView* gb, const ArcGatherParams* gp,
-                             const ArcCutParams* cp, float4** info_out, float4** extra_out) {
+                             const ArcCutParams* cp, float4** info_out, float4** extra_out, int* estimate) {
     const int W = gb->width, H = gb->height;
     const int tiles_x = (W + kTile - 1) / kTile, tiles_y = (H + kTile - 1) / kTile, tiles = tiles_x * tiles_y;
     float4* info = nullptr;
@@ -864,9 +966,12 @@ arc_status launch_tile_setup(arc_context* ctx, const arc_lbvh* bvh, const ArcGBu
     ta.err = ctx->d_error;
     float4* extra = nullptr;
     ARC_TRY(ctx->arena.get("node_extra", (size_t)(bvh->n - 1) * 2 * sizeof(float4), reinterpret_cast<void**>(&extra)));
+    ta.estimate = estimate;
+    ta.extra = extra;
+    ta.bp = bound_params(gp, cp);
     stage_begin(ctx, "cut_setup");
-    cut_tile_setup<<<(tiles + kSelWarps - 1) / kSelWarps, 32 * kSelWarps, 0, ctx->stream>>>(ta);
     cut_node_extra<<<(bvh->n - 1 + 255) / 256, 256, 0, ctx->stream>>>(bvh->n, ta.bounds, ta.records, extra);
+    cut_tile_setup<<<(tiles + kSetupWarps - 1) / kSetupWarps, 32 * kSetupWarps, 0, ctx->stream>>>(ta);
     stage_end(ctx, 2);
     ARC_TRY_CUDA(cudaGetLastError());
     *info_out = info;
@@ -939,38 +1044,35 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
     ARC_TRY(ctx->arena.get("cut_tables", (size_t)tiles * pool.max_chunks * sizeof(int32_t),
                            reinterpret_cast<void**>(&pool.tables)));
     ARC_TRY(ctx->arena.get("cut_counts", (size_t)tiles * sizeof(int32_t), reinterpret_cast<void**>(&pool.counts)));
-    ARC_TRY(ctx->arena.get("cut_pool_next", sizeof(int32_t), reinterpret_cast<void**>(&pool.next)));
-    ARC_TRY_CUDA(cudaMemsetAsync(pool.next, 0, sizeof(int32_t), st));
+    // the pool's allocation counter and the selection's work counter
+    ARC_TRY(ctx->arena.get("cut_pool_next", 2 * sizeof(int32_t), reinterpret_cast<void**>(&pool.next)));
+    ARC_TRY_CUDA(cudaMemsetAsync(pool.next, 0, 2 * sizeof(int32_t), st));
     float4* info = nullptr;
     float4* extra = nullptr;
-    ARC_TRY(launch_tile_setup(ctx, bvh, gb, gp, cp, &info, &extra));
-    TileArgs ta;
-    ta.gpos = reinterpret_cast<const float4*>(gb->position);
-    ta.gnrm = reinterpret_cast<const float4*>(gb->normal);
-    ta.bounds = reinterpret_cast<const float4*>(bvh->view.bounds);
-    ta.records = reinterpret_cast<const float4*>(bvh->view.records);
+    int* order = nullptr;     // tiles in the order the selection, then the evaluation takes them
+    int* estimate = nullptr;  // expected cut size per tile
+    ARC_TRY(ctx->arena.get("cut_order", (size_t)tiles * sizeof(int), reinterpret_cast<void**>(&order)));
+    if (cp->kind == ARC_CUT_ERROR_BOUND)
+        ARC_TRY(ctx->arena.get("cut_estimate", (size_t)tiles * sizeof(int), reinterpret_cast<void**>(&estimate)));
+    ARC_TRY(launch_tile_setup(ctx, bvh, gb, gp, cp, &info, &extra, estimate));
 
     if (cp->kind == ARC_CUT_ERROR_BOUND) {
         SelArgs sa;
         sa.n = bvh->n;
-        sa.bounds = ta.bounds;
-        sa.records = ta.records;
+        sa.bounds = reinterpret_cast<const float4*>(bvh->view.bounds);
+        sa.records = reinterpret_cast<const float4*>(bvh->view.records);
         sa.info = info;
         sa.extra = extra;
-        sa.bp.clamp2 = clamp2;
-        sa.bp.ar_kind = gp->ar_kind;
-        sa.bp.eps_cone = 0.001f;
-        sa.bp.cos_thr = fmaxf(cosf(gp->cone_half_angle), 0.001f);
-        sa.bp.disk_scale = gp->disk_radius > 0.0f ? 1.0f / (kPi * gp->disk_radius * gp->disk_radius) : 0.0f;
-        sa.bp.ar_uncertain = cp->ar_uncertain_factor;
+        sa.bp = bound_params(gp, cp);
+        sa.order = order;
         sa.tiles = tiles;
         sa.pool = pool;
         sa.err = ctx->d_error;
-        const size_t smem = (size_t)kSelWarps * kSelStack * sizeof(int);
-        ARC_TRY_CUDA(cudaFuncSetAttribute(cut_select_bound, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        sa.next_tile = pool.next + 1;
         stage_begin(ctx, "cut_select");
-        cut_select_bound<<<(tiles + kSelWarps - 1) / kSelWarps, 32 * kSelWarps, smem, st>>>(sa);
-        stage_end(ctx, 1);
+        tile_order_kernel<<<1, 1024, 0, st>>>(estimate, tiles, order);
+        cut_select_bound<<<std::min(tiles, ctx->sm_count * kSelBlocksPerSm), kSelThreads, 0, st>>>(sa);
+        stage_end(ctx, 2);
         ARC_TRY_CUDA(cudaGetLastError());
     } else {
         ARC_CHECK_ARG(cp->model != nullptr, "ARC_CUT_LEARNED needs a model");
@@ -978,14 +1080,14 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
     }
 
     EvalArgs ea;
-    ea.gpos = ta.gpos;
-    ea.gnrm = ta.gnrm;
+    ea.gpos = reinterpret_cast<const float4*>(gb->position);
+    ea.gnrm = reinterpret_cast<const float4*>(gb->normal);
     ea.gpitch = gb->pitch;
     ea.width = W;
     ea.height = H;
     ea.mats = ctx->d_materials;
     ea.num_mats = ctx->num_materials;
-    ea.records = ta.records;
+    ea.records = reinterpret_cast<const float4*>(bvh->view.records);
     ea.tiles_x = tiles_x;
     ea.pool = pool;
     ea.pc.cos_thr = fmaxf(cosf(gp->cone_half_angle), 0.001f);
@@ -998,8 +1100,6 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
     ea.out_ar = reinterpret_cast<float4*>(out->antiradiance);
     ea.out_res64 = out->result_fp64;
     ea.opitch = out->pitch;
-    int* order = nullptr;
-    ARC_TRY(ctx->arena.get("cut_order", (size_t)tiles * sizeof(int), reinterpret_cast<void**>(&order)));
     ea.order = order;
     stage_begin(ctx, "cut_eval");
     tile_order_kernel<<<1, 1024, 0, st>>>(pool.counts, tiles, order);

@@ -4,6 +4,8 @@
 #ifndef ARC_CUT_BOUNDS_CUH_
 #define ARC_CUT_BOUNDS_CUH_
 
+#include <cmath>
+
 #include "arc_internal.h"
 #include "device_common.cuh"
 
@@ -44,6 +46,17 @@ struct BoundParams {
     float disk_scale;
     float ar_uncertain;  // bound multiplier when the cone test may differ between the node's pairs
 };
+
+inline BoundParams bound_params(const ArcGatherParams* gp, const ArcCutParams* cp) {
+    BoundParams bp;
+    bp.clamp2 = gp->dist_clamp > 0.0f ? gp->dist_clamp * gp->dist_clamp : 0.0f;
+    bp.ar_kind = gp->ar_kind;
+    bp.eps_cone = 0.001f;
+    bp.cos_thr = fmaxf(cosf(gp->cone_half_angle), 0.001f);
+    bp.disk_scale = gp->disk_radius > 0.0f ? 1.0f / (kPi * gp->disk_radius * gp->disk_radius) : 0.0f;
+    bp.ar_uncertain = cp->ar_uncertain_factor;
+    return bp;
+}
 
 __device__ __forceinline__ float lum3(float r, float g, float b) {
     return rn_add(rn_add(rn_mul(0.2126f, r), rn_mul(0.7152f, g)), rn_mul(0.0722f, b));
@@ -169,45 +182,130 @@ __device__ __forceinline__ float node_bound(const TileInfo& t, const NodeGeom& g
     return rn_mul(t.kdl, m);
 }
 
-// Appends one warp's accepted nodes to its tile's chunked list in the cut pool.  Warp-uniform
-// state; every lane of the warp calls append() with the same `mask`.
-struct CutWriter {
-    static constexpr int kChunk = 1024;
-    CutPool pool;
-    int32_t* table;
-    int count = 0;
-    int chunk_id = -1;  // pool chunk holding entry count - 1
-    bool overflow = false;
-
-    __device__ CutWriter(const CutPool& p, int tile) : pool(p), table(p.tables + (size_t)tile * p.max_chunks) {}
-
-    __device__ __forceinline__ void append(unsigned mask, bool mine, int node, int lane) {
-        const int n = __popc(mask);
-        if (n == 0) return;
-        const int first_new = count % kChunk == 0 ? count / kChunk : count / kChunk + 1;
-        const int last = (count + n - 1) / kChunk;
-        int new_id = -1;
-        if (last >= first_new) {  // the batch starts a new chunk (at most one: n <= 32 < kChunk)
-            if (lane == 0) {
-                new_id = last < pool.max_chunks ? atomicAdd(pool.next, 1) : pool.num_chunks;
-                if (new_id < pool.num_chunks) table[last] = new_id;
-            }
-            new_id = __shfl_sync(0xffffffffu, new_id, 0);
-            if (new_id >= pool.num_chunks) overflow = true;
-        }
-        if (mine) {
-            const int pos = count + __popc(mask & ((1u << lane) - 1u));
-            const int id = pos / kChunk == last && last >= first_new ? new_id : chunk_id;
-            if (id >= 0 && id < pool.num_chunks) pool.entries[(size_t)id * kChunk + pos % kChunk] = node;
-        }
-        if (last >= first_new) chunk_id = new_id;
-        if (overflow) {
-            count = min(count + n, last * kChunk);  // keep only entries that landed in a chunk
-        } else {
-            count += n;
-        }
-    }
+// The same geometry and bound with approximate reciprocals and square roots (one instruction each,
+// 1-2 ulp, instead of the correctly rounded sequences with their branches), and a radius `err` such
+// that the rounded bound lies within m +- err whenever `sure`: a decision that m +- err leaves open, or
+// that is not sure, has to be made with node_geom / node_bound.
+//
+// Each cosine is within kCosErr = 1e-4 of its rounded value: 1 - s^2 carries at most a few 1e-7, so a
+// sine or cosine from it is within 1e-6 / its value, 5e-5 at the 0.02 below which the result is not
+// sure; the early returns of the cone functions are continuous in their arguments, and the places that
+// are not (centre distance against the radii, the cone test's thresholds) are not sure within a margin.
+struct FastBound {
+    NodeGeom g;
+    float m, err;
+    bool sure;
 };
+
+constexpr float kCosErr = 1e-4f, kSineFloor = 0.02f;
+
+__device__ __forceinline__ float sqrt_fast(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// cone_max_cos and, when asked for, cone_min_cos of two cones whose axes' cosine is cb, without
+// branches (a warp's lanes rarely agree on the early returns).
+__device__ __forceinline__ float cone_max_fast(float cb, float sb, float c1, float s1, float c2, float s2) {
+    const float cg = c1 * c2 - s1 * s2, sg = s1 * c2 + c1 * s2;
+    const bool one = c1 <= -1.0f || c2 <= -1.0f || sg < 0.0f || cb >= cg;
+    return one ? 1.0f : cb * cg + sb * sg;
+}
+
+__device__ __forceinline__ float cone_min_fast(float cb, float sb, float c1, float s1, float c2, float s2, bool& sure) {
+    const float cg = c1 * c2 - s1 * s2, sg = s1 * c2 + c1 * s2;
+    if ((sb < kSineFloor && sg > kSineFloor) || (cg < 0.0f && fabsf(sg) < kCosErr)) sure = false;
+    const bool opposite = c1 <= -1.0f || c2 <= -1.0f || sg < 0.0f || cg < -cb;
+    return opposite ? -1.0f : cb * cg - sb * sg;
+}
+
+__device__ __forceinline__ FastBound node_bound_fast(const TileInfo& t, float4 b0, float4 b1, float4 nc, float4 wc,
+                                                     const NodeExtra& ne, const BoundParams& bp) {
+    FastBound f;
+    f.sure = true;
+    NodeGeom& g = f.g;
+    const float bmin[3] = {b0.x, b0.y, b0.z}, bmax[3] = {b1.x, b1.y, b1.z};
+    float d2 = 0.0f, v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float gap = fmaxf(0.0f, fmaxf(bmin[k] - t.tmax[k], t.tmin[k] - bmax[k]));
+        d2 = fmaf(gap, gap, d2);
+        v[k] = fmaf(0.5f, t.tmin[k] + t.tmax[k], -ne.cn[k]);
+    }
+    g.d2c = fmaxf(d2, bp.clamp2);
+    const float dc2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+    float inv;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(dc2));
+    g.dc = dc2 * inv;
+    g.rn = ne.rn;
+    g.rs = ne.rn + t.rt;
+    // (also false for a centre distance of 0, where the product is not a number)
+    f.sure = fabsf(g.dc - g.rs) > 1e-5f * (g.dc + g.rs) && dc2 > 1e-30f && dc2 < 1e30f;
+    float ca = -1.0f, sa = 0.0f, ax = 0.0f, ay = 0.0f, az = 0.0f;
+    if (g.dc > g.rs) {
+        sa = g.rs * inv;
+        ca = sqrt_fast(1.0f - sa * sa);
+        ax = v[0] * inv;
+        ay = v[1] * inv;
+        az = v[2] * inv;
+        if (!(ca >= kSineFloor)) f.sure = false;
+    }
+    auto clamped = [](float x) { return fminf(fmaxf(x, -1.0f), 1.0f); };
+    auto sine = [](float c) { return sqrt_fast(fmaxf(0.0f, 1.0f - c * c)); };
+    // the sine of an angle near pi loses its digits where the other cone's is not small; near 0 the
+    // cone functions return early or multiply it by a sine as small
+    const float cbn = clamped(nc.x * ax + nc.y * ay + nc.z * az);
+    const float cbt = clamped(-(t.ncone.x * ax + t.ncone.y * ay + t.ncone.z * az));
+    const float sbn = sine(cbn), sbt = sine(cbt);
+    bool flat = (cbn < 0.0f && sbn < kSineFloor) || (cbt < 0.0f && sbt < kSineFloor);
+    g.cos2 = __saturatef(cone_max_fast(cbn, sbn, nc.w, ne.snc, ca, sa));
+    g.cos1 = __saturatef(cone_max_fast(cbt, sbt, t.ncone.w, t.sn, ca, sa));
+    g.ar_ok = 0.0f;
+    if (bp.ar_kind == ARC_AR_CONE) {
+        const float cbw = clamped(wc.x * ax + wc.y * ay + wc.z * az);
+        const float sbw = sine(cbw);
+        const float cw = cone_max_fast(cbw, sbw, wc.w, ne.swc, ca, sa);
+        flat = flat || (cbw < 0.0f && sbw < kSineFloor);
+        if (fminf(fabsf(cw - bp.cos_thr), fabsf(g.cos1 - bp.eps_cone)) < kCosErr) f.sure = false;
+        if (cw > bp.cos_thr && g.cos1 > bp.eps_cone) {
+            const float cwmin = cone_min_fast(cbw, sbw, wc.w, ne.swc, ca, sa, f.sure);
+            const float c1min = cone_min_fast(cbt, sbt, t.ncone.w, t.sn, ca, sa, f.sure);
+            if (fminf(fabsf(cwmin - bp.cos_thr), fabsf(c1min - bp.eps_cone)) < kCosErr) f.sure = false;
+            g.ar_ok = (cwmin > bp.cos_thr && c1min > bp.eps_cone) ? 1.0f : bp.ar_uncertain;
+        }
+        if (flat) f.sure = false;
+    } else {
+        if (bp.ar_kind == ARC_AR_DISK) g.ar_ok = 1.0f;
+        if (flat) f.sure = false;
+    }
+    if (!(g.d2c > 0.0f)) {
+        f.m = INFINITY;
+        f.err = 0.0f;
+        return f;
+    }
+    float id2;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(id2) : "f"(g.d2c));
+    float m = ne.Ls * (g.cos1 * g.cos2) * id2;
+    float e = ne.Ls * (g.cos1 + g.cos2 + kCosErr) * id2;
+    if (bp.ar_kind == ARC_AR_CONE) {
+        m += ne.As * (g.ar_ok * g.cos1) * id2;
+        e += ne.As * g.ar_ok * id2;
+    } else if (bp.ar_kind == ARC_AR_DISK) {
+        m += ne.As * bp.disk_scale;
+    }
+    f.m = t.kdl * m;
+    f.err = t.kdl * (kCosErr * e) + 1e-5f * f.m;
+    return f;
+}
+
+// Whether the rounded bound exceeds `limit`: 1 yes, 0 no, -1 not settled by the approximate one.
+__device__ __forceinline__ int exceeds(const FastBound& f, float limit) {
+    if (!f.sure) return -1;
+    if (f.m - f.err > limit) return 1;
+    if (f.m + f.err <= limit) return 0;
+    return -1;
+}
 
 }  // namespace arc
 

@@ -838,17 +838,6 @@ arc_status arena_get(arc_context* ctx, const char* name, size_t count, T** out) 
     return ctx->arena.get(name, sizeof(T) * (count > 0 ? count : 1), reinterpret_cast<void**>(out));
 }
 
-BoundParams bound_params(const ArcGatherParams* gp, const ArcCutParams* cp) {
-    BoundParams bp;
-    bp.clamp2 = gp->dist_clamp > 0.0f ? gp->dist_clamp * gp->dist_clamp : 0.0f;
-    bp.ar_kind = gp->ar_kind;
-    bp.eps_cone = 0.001f;
-    bp.cos_thr = fmaxf(cosf(gp->cone_half_angle), 0.001f);
-    bp.disk_scale = gp->disk_radius > 0.0f ? 1.0f / (kPi * gp->disk_radius * gp->disk_radius) : 0.0f;
-    bp.ar_uncertain = cp->ar_uncertain_factor;
-    return bp;
-}
-
 }  // namespace
 
 arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, const ArcGatherParams* gp,
@@ -994,7 +983,7 @@ extern "C" arc_status arc_cut_training_samples(arc_context* ctx, const arc_lbvh*
     const int n = bvh->n;
     float4* info = nullptr;
     float4* extra = nullptr;
-    ARC_TRY(launch_tile_setup(ctx, bvh, gb, gp, cp, &info, &extra));
+    ARC_TRY(launch_tile_setup(ctx, bvh, gb, gp, cp, &info, &extra, nullptr));
     // batch of tiles whose FP64 prefixes fit in ~8 GB
     const size_t per_tile = (size_t)(n + 1) * 64 * sizeof(double);
     const int batch = (int)std::max<size_t>(1, std::min<size_t>((size_t)tiles, ((size_t)8 << 30) / per_tile));
