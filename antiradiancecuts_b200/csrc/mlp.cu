@@ -2,7 +2,8 @@
 // the 5th-generation tensor cores.  No counterpart in the reference: it predicts, for an 8x8 pixel
 // tile and a tree node, whether the cut must refine the node.
 //
-// Two kernels.  Each 128-thread CTA walks 128-row tiles of the input (thread t owns row t):
+// Two kernels.  Each CTA walks 128-row tiles of the input (forward: thread t owns row t; training: two
+// threads per row):
 //   forward   X[128x16] -> tcgen05.mma -> TMEM -> +b, activation -> BF16 core-matrix smem -> next layer;
 //             the 64 -> 1 output layer runs on the CUDA cores from registers (mlp_tile.cuh, shared
 //             with the fused level kernel of the learned cut).
@@ -10,7 +11,7 @@
 //             dH_l = dZ_{l+1} W_{l+1}                       (M = 128 rows, B read MN-major)
 //             dW_l += dZ_l^T H_{l-1}   (accumulated in TMEM over every tile the CTA owns;
 //                                       M padded to 128 = out features, A and B read MN-major)
-//             bias / output-layer gradients are warp-reduced into shared memory.
+//             bias / output-layer gradients are column sums kept in registers.
 // Weights are kept as an FP32 master copy (Adam updates it) and rounded to BF16 into shared
 // memory by every CTA.  Every tensor-core result waits on an mbarrier with a bounded wait; the CTA
 // stops (and still frees its TMEM) if a wait gives up.
@@ -34,9 +35,8 @@ namespace mlp {
 // shared-memory carve-up (bytes); dZ is followed by 2 KB because the M-padded weight-gradient
 // MMA reads up to that far past it (the extra rows land in D rows 64..127, which are ignored)
 constexpr uint32_t sW1 = 0, sW2 = sW1 + 2048, sW3 = sW2 + 8192, sX = sW3 + 8192, sH1 = sX + 4096,
-                   sH2 = sH1 + 16384, sZ1 = sH2 + 16384, sZ2 = sZ1 + 16384, sDZ = sZ2 + 16384,
-                   sVecTrain = sDZ + 16384 + 2048;
-constexpr uint32_t kVecBytes = (4 * 64 + 4 * 64 + 4) * 4;
+                   sH2 = sH1 + 16384, sDZ = sH2 + 16384, sVecTrain = sDZ + 16384 + 2048;
+constexpr uint32_t kVecBytes = 4 * 64 * 4;
 constexpr uint32_t kSmemTrain = sVecTrain + kVecBytes;
 // inference: weights | X tile (4 KB) | hidden (16 KB) | vectors
 constexpr uint32_t sInX = kWeightBytes, sInH = sInX + 4096, sInVec = sInH + 16384,
@@ -56,36 +56,17 @@ struct Args {
     uint32_t* err;
 };
 
-// store 64 values of row t as BF16 into a K-major (K = 64) core-matrix buffer
-__device__ __forceinline__ void store_row64(unsigned char* buf, int t, const float* v) {
+// store 32 values of row r, columns c0 .. c0 + 31, as BF16 into a K-major (K = 64) core-matrix buffer
+__device__ __forceinline__ void store_row32(unsigned char* buf, int r, int c0, const float* v) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 0; c < 4; ++c) {
         uint4 q;
         q.x = pack2(v[8 * c + 0], v[8 * c + 1]);
         q.y = pack2(v[8 * c + 2], v[8 * c + 3]);
         q.z = pack2(v[8 * c + 4], v[8 * c + 5]);
         q.w = pack2(v[8 * c + 6], v[8 * c + 7]);
-        *reinterpret_cast<uint4*>(buf + tc::kmajor_offset(t, 8 * c, 64)) = q;
+        *reinterpret_cast<uint4*>(buf + tc::kmajor_offset(r, c0 + 8 * c, 64)) = q;
     }
-}
-
-__device__ __forceinline__ void load_row64(const unsigned char* buf, int t, float* v) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const uint4 q = *reinterpret_cast<const uint4*>(buf + tc::kmajor_offset(t, 8 * c, 64));
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __bfloat1622float2(p[e]);
-            v[8 * c + 2 * e] = f.x;
-            v[8 * c + 2 * e + 1] = f.y;
-        }
-    }
-}
-
-__device__ __forceinline__ void load_tmem64(uint32_t taddr, float* v) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) tc::ld16(taddr + 16 * c, v + 16 * c);
 }
 
 // one 32-lane sum, result in every lane
@@ -95,13 +76,19 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// column sums of a 128 x 64 block held one row per thread -> shared accumulator g[64]
-__device__ __forceinline__ void accumulate_columns(const float* v, float* g, int lane) {
+// Sums over a warp's 32 rows of 32 columns (one row per lane): lane c returns column c's sum.  Each step
+// sends half of what is left to the partner lane, 31 exchanges instead of 32 x 5.
+__device__ __forceinline__ float column_sums(float* v, int lane) {
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-        const float s = warp_sum(v[j]);
-        if (lane == 0) atomicAdd(&g[j], s);
+    for (int s = 16; s > 0; s >>= 1) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (int i = 0; i < s; ++i) {
+            const float send = up ? v[i] : v[i + s], keep = up ? v[i + s] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+        }
     }
+    return v[0];
 }
 
 // Forward over every row of the input: persistent CTAs, one 128-row tile at a time.
@@ -149,43 +136,54 @@ __global__ void __launch_bounds__(128) mlp_infer_kernel(Args a) {
     if (w == 0) tc::dealloc(tmem_base, 64);
 }
 
-// Forward + backward with weight-gradient accumulation in TMEM (training).
+// Forward + backward with weight-gradient accumulation in TMEM (training).  256 threads per 128-row
+// tile: thread t owns row t % 128 and columns 32 (t / 128) .. + 31 of every layer (a warp reads its
+// own quarter of the TMEM lanes, so warps w and w + 4 share a quarter).  A training batch has fewer
+// tiles than the chip has SMs, so a tile's latency is the kernel's time: two threads per row halve
+// the elementwise work between the tensor-core rounds, the column sums (bias and output-layer
+// gradients) stay in one register per lane until the end, pre-activations stay in registers, and
+// the weights arrive with independent 16-byte loads.
+constexpr int kTrainThreads = 256;
+
+// four consecutive weights of row r (K columns, 4 c ..) as BF16 into a K-major operand
+__device__ __forceinline__ void store_weights4(unsigned char* w, const float* params, int i, int K) {
+    const float4 v = *reinterpret_cast<const float4*>(params + 4 * i);
+    const int r = 4 * i / K, k = 4 * i % K;
+    *reinterpret_cast<uint2*>(w + tc::kmajor_offset(r, k, K)) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+}
+
+// adds four consecutive floats to global memory (16-byte aligned)
+__device__ __forceinline__ void red_add4(float* dst, const float* v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+                 : "memory");
+}
+
 template <int ACT>
-__global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
+__global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(Args a) {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
+    __shared__ float s_y[kRows], s_dy[kRows];
+    __shared__ float s_col[4][4][64];  // [row quarter][gw4, gb3, gb2, gb1][column]
+    __shared__ float s_b4[4];
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const int r = t & (kRows - 1), half = t >> 7, c0 = 32 * half;
     float* vec = reinterpret_cast<float*>(sm + sVecTrain);
-    float* b1 = vec;
-    float* b2 = vec + 64;
-    float* b3 = vec + 128;
-    float* w4 = vec + 192;
-    float* gb1 = vec + 256;  // training: bias / output-layer gradient accumulators
-    float* gb2 = vec + 320;
-    float* gb3 = vec + 384;
-    float* gw4 = vec + 448;
-    float* gb4 = vec + 512;
+    const float* b1 = vec + c0;
+    const float* b2 = vec + 64 + c0;
+    const float* b3 = vec + 128 + c0;
+    const float* w4 = vec + 192 + c0;
     constexpr uint32_t kCols = 256;  // D | dW3 | dW2 | dW1
 
     // weights -> BF16 core-matrix layouts, vectors -> FP32
-    for (int i = t; i < kHid * kIn; i += 128)
-        *reinterpret_cast<__nv_bfloat16*>(sm + sW1 + tc::kmajor_offset(i / kIn, i % kIn, kIn)) =
-            __float2bfloat16_rn(a.params[oW1 + i]);
-    for (int i = t; i < kHid * kHid; i += 128) {
-        *reinterpret_cast<__nv_bfloat16*>(sm + sW2 + tc::kmajor_offset(i / kHid, i % kHid, kHid)) =
-            __float2bfloat16_rn(a.params[oW2 + i]);
-        *reinterpret_cast<__nv_bfloat16*>(sm + sW3 + tc::kmajor_offset(i / kHid, i % kHid, kHid)) =
-            __float2bfloat16_rn(a.params[oW3 + i]);
+    store_weights4(sm + sW1, a.params + oW1, t, kIn);
+#pragma unroll
+    for (int i = 0; i < kHid * kHid / 4 / kTrainThreads; ++i) {
+        store_weights4(sm + sW2, a.params + oW2, i * kTrainThreads + t, kHid);
+        store_weights4(sm + sW3, a.params + oW3, i * kTrainThreads + t, kHid);
     }
-    if (t < 64) {
-        b1[t] = a.params[oB1 + t];
-        b2[t] = a.params[oB2 + t];
-        b3[t] = a.params[oB3 + t];
-        w4[t] = a.params[oW4 + t];
-    }
+    vec[t] = a.params[(t < 64 ? oB1 : t < 128 ? oB2 : t < 192 ? oB3 : oW4) + (t & 63)];
     const float b4 = a.params[oB4];
-    for (int i = t; i < 4 * 64 + 4; i += 128) gb1[i] = 0.0f;
     if (w == 0) tc::alloc(&tmem_base, kCols);
     if (t == 0) {
         mbar_init(&bar, 1);
@@ -196,11 +194,13 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const uint32_t lane_off = (uint32_t)(w * 32) << 16;
+    const uint32_t taddr = tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)c0;  // this thread's lane and columns
     const uint32_t base = smem_u32(sm);
     uint32_t phase = 0;
     bool any_tile = false;
     bool gave_up = false;  // a tensor-core wait gave up: its commit may still be in flight
+    float gw4 = 0.0f, gb3 = 0.0f, gb2 = 0.0f, gb1 = 0.0f;  // column c0 + lane over this warp's rows
+    float gb4 = 0.0f, loss = 0.0f;
 
     constexpr uint32_t idKK64 = tc::idesc_bf16(128, 64, false, false);
     constexpr uint32_t idKM64 = tc::idesc_bf16(128, 64, false, true);
@@ -233,21 +233,26 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
             tc::commit(&bar);
         }
     };
+    // this thread's half row of D
+    auto load_d = [&](float* v) { tc::ld32(taddr, v); };
+    // the pre-activation rounded to BF16, as the backward pass differentiates it
+    auto rounded = [](uint32_t z, int h) { return __uint_as_float(h ? z & 0xffff0000u : z << 16); };
 
     const int64_t ntiles = (a.rows + kRows - 1) / kRows;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t row = tile * kRows + t;
+        const int64_t row = tile * kRows + r;
         const bool valid = row < a.rows;
-        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = make_uint4(0, 0, 0, 0);
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (valid) x = reinterpret_cast<const uint4*>(a.x + row * kIn)[half];
+        *reinterpret_cast<uint4*>(sm + sX + tc::kmajor_offset(r, 8 * half, kIn)) = x;
+        float lab = 0.0f, wgt = 0.0f;
         if (valid) {
-            const uint4* xp = reinterpret_cast<const uint4*>(a.x + row * kIn);
-            x0 = xp[0];
-            x1 = xp[1];
+            lab = a.labels[row];
+            wgt = a.weights ? a.weights[row] : 1.0f;
         }
-        *reinterpret_cast<uint4*>(sm + sX + tc::kmajor_offset(t, 0, kIn)) = x0;
-        *reinterpret_cast<uint4*>(sm + sX + tc::kmajor_offset(t, 8, kIn)) = x1;
 
-        float z[64], h[64];
+        float z[32], h[32];
+        uint32_t z1[16], z2[16];  // pre-activations of the first two layers, BF16 pairs
         // ---- layer 1 (K = 16) ----
         publish_smem();
         if (t == 0) {
@@ -256,71 +261,73 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
             tc::commit(&bar);
         }
         if (!wait_mma()) break;
-        load_tmem64(tmem + lane_off, z);
+        load_d(z);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
+        for (int j = 0; j < 32; ++j) {
             z[j] += b1[j];
             h[j] = act<ACT>(z[j]);
         }
-        store_row64(sm + sH1, t, h);
-        store_row64(sm + sZ1, t, z);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) z1[j] = pack2(z[2 * j], z[2 * j + 1]);
+        store_row32(sm + sH1, r, c0, h);
         // ---- layer 2 ----
         publish_smem();
         layer64(sH1, sW2);
         if (!wait_mma()) break;
-        load_tmem64(tmem + lane_off, z);
+        load_d(z);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
+        for (int j = 0; j < 32; ++j) {
             z[j] += b2[j];
             h[j] = act<ACT>(z[j]);
         }
-        store_row64(sm + sH2, t, h);
-        store_row64(sm + sZ2, t, z);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) z2[j] = pack2(z[2 * j], z[2 * j + 1]);
+        store_row32(sm + sH2, r, c0, h);
         // ---- layer 3 (kept in registers) ----
         publish_smem();
         layer64(sH2, sW3);
         if (!wait_mma()) break;
-        load_tmem64(tmem + lane_off, z);
+        load_d(z);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
+        for (int j = 0; j < 32; ++j) {
             z[j] += b3[j];
             h[j] = act<ACT>(z[j]);
         }
-        // ---- output layer on the CUDA cores ----
-        float y = b4;
+        // ---- output layer on the CUDA cores: one sum over the row, columns 0 .. 63 in order ----
+        if (half == 0) {
+            float y = b4;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) y = fmaf(h[j], w4[j], y);
-
-        // ---- loss, output-layer gradients, dZ3 ----
-        float dy = 0.0f, l = 0.0f;
-        if (valid) {
-            const float lab = a.labels[row];
-            const float wgt = a.weights ? a.weights[row] : 1.0f;
-            if (a.loss_kind == ARC_MLP_LOSS_SQUARED) {
-                const float d = y - lab;
-                dy = wgt * 2.0f * d * a.loss_scale;
-                l = wgt * d * d * a.loss_scale;
-            } else {
-                const float p = 1.0f / (1.0f + expf(-y));
-                dy = wgt * (p - lab) * a.loss_scale;
-                l = wgt * (fmaxf(y, 0.0f) - y * lab + log1pf(expf(-fabsf(y)))) * a.loss_scale;
-            }
+            for (int j = 0; j < 32; ++j) y = fmaf(h[j], w4[j], y);
+            s_y[r] = y;
         }
-        {
-            const float ls = warp_sum(l), ds = warp_sum(dy);
-            if (lane == 0) {
-                atomicAdd(a.loss, ls);
-                atomicAdd(gb4, ds);
+        __syncthreads();
+        if (half == 1) {
+            float y = s_y[r];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) y = fmaf(h[j], w4[j], y);
+            // ---- loss and its gradient ----
+            float dy = 0.0f;
+            if (valid) {
+                if (a.loss_kind == ARC_MLP_LOSS_SQUARED) {
+                    const float d = y - lab;
+                    dy = wgt * 2.0f * d * a.loss_scale;
+                    loss += wgt * d * d * a.loss_scale;
+                } else {
+                    const float p = 1.0f / (1.0f + expf(-y));
+                    dy = wgt * (p - lab) * a.loss_scale;
+                    loss += wgt * (fmaxf(y, 0.0f) - y * lab + log1pf(expf(-fabsf(y)))) * a.loss_scale;
+                }
             }
+            gb4 += dy;
+            s_dy[r] = dy;
         }
-        float g[64];
+        __syncthreads();
+        // ---- output-layer gradients, dZ3 ----
+        const float dy = s_dy[r];
+        float g[32];
 #pragma unroll
-        for (int j = 0; j < 64; ++j) g[j] = dy * h[j];
-        accumulate_columns(g, gw4, lane);
-#pragma unroll
-        for (int j = 0; j < 64; ++j) g[j] = dy * w4[j] * act_grad<ACT>(z[j]);  // dZ3
-        accumulate_columns(g, gb3, lane);
-        store_row64(sm + sDZ, t, g);
+        for (int j = 0; j < 32; ++j) g[j] = dy * w4[j] * act_grad<ACT>(z[j]);  // dZ3
+        store_row32(sm + sDZ, r, c0, g);
         // dW3 += dZ3^T H2 ; dH2 = dZ3 W3
         publish_smem();
         if (t == 0) {
@@ -335,13 +342,16 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
                         idKM64, s > 0);
             tc::commit(&bar);
         }
-        if (!wait_mma()) break;
-        load_tmem64(tmem + lane_off, g);  // dH2
-        load_row64(sm + sZ2, t, z);
+        // (the column sums run beside the tensor cores)
+        gb3 += column_sums(g, lane);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) g[j] *= act_grad<ACT>(z[j]);  // dZ2
-        accumulate_columns(g, gb2, lane);
-        store_row64(sm + sDZ, t, g);
+        for (int j = 0; j < 32; ++j) h[j] *= dy;
+        gw4 += column_sums(h, lane);
+        if (!wait_mma()) break;
+        load_d(g);  // dH2
+#pragma unroll
+        for (int j = 0; j < 32; ++j) g[j] *= act_grad<ACT>(rounded(z2[j / 2], j & 1));  // dZ2
+        store_row32(sm + sDZ, r, c0, g);
         // dW2 += dZ2^T H1 ; dH1 = dZ2 W2
         publish_smem();
         if (t == 0) {
@@ -356,13 +366,12 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
                         idKM64, s > 0);
             tc::commit(&bar);
         }
+        gb2 += column_sums(g, lane);
         if (!wait_mma()) break;
-        load_tmem64(tmem + lane_off, g);  // dH1
-        load_row64(sm + sZ1, t, z);
+        load_d(g);  // dH1
 #pragma unroll
-        for (int j = 0; j < 64; ++j) g[j] *= act_grad<ACT>(z[j]);  // dZ1
-        accumulate_columns(g, gb1, lane);
-        store_row64(sm + sDZ, t, g);
+        for (int j = 0; j < 32; ++j) g[j] *= act_grad<ACT>(rounded(z1[j / 2], j & 1));  // dZ1
+        store_row32(sm + sDZ, r, c0, g);
         // dW1 += dZ1^T X  (N = 16)
         publish_smem();
         if (t == 0) {
@@ -373,32 +382,43 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(Args a) {
                         tc::smem_desc(base + sX + 512 * s, 256, 128), idMM16, any_tile || s > 0);
             tc::commit(&bar);
         }
+        gb1 += column_sums(g, lane);
         if (!wait_mma()) break;
         any_tile = true;
     }
 
     if (any_tile && !gave_up) {
-        // weight gradients: D rows 0..63 (= output features) live in TMEM lanes 0..63
-        if (w < 2) {
-            float v[64];
-            load_tmem64(tmem + lane_off + 64, v);
+        // weight gradients: D rows 0..63 (= output features) live in TMEM lanes 0..63, which warps
+        // 0, 1 (columns 0 .. 31) and 4, 5 (32 .. 63) read
+        if ((w & 3) < 2) {
+            float v[32];
+            tc::ld32(taddr + 64, v);
 #pragma unroll
-            for (int j = 0; j < 64; ++j) atomicAdd(&a.grads[oW3 + t * 64 + j], v[j]);
-            load_tmem64(tmem + lane_off + 128, v);
+            for (int j = 0; j < 32; j += 4) red_add4(&a.grads[oW3 + r * 64 + c0 + j], v + j);
+            tc::ld32(taddr + 128, v);
 #pragma unroll
-            for (int j = 0; j < 64; ++j) atomicAdd(&a.grads[oW2 + t * 64 + j], v[j]);
-            tc::ld16(tmem + lane_off + 192, v);
+            for (int j = 0; j < 32; j += 4) red_add4(&a.grads[oW2 + r * 64 + c0 + j], v + j);
+            if (half == 0) {
+                tc::ld16(taddr + 192, v);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) atomicAdd(&a.grads[oW1 + t * 16 + j], v[j]);
+                for (int j = 0; j < 16; j += 4) red_add4(&a.grads[oW1 + r * 16 + j], v + j);
+            }
+        }
+        float* col = &s_col[w & 3][0][c0 + lane];
+        col[0] = gw4;
+        col[64] = gb3;
+        col[128] = gb2;
+        col[192] = gb1;
+        const float ls = warp_sum(loss), ds = warp_sum(gb4);
+        if (lane == 0 && half == 1) {
+            s_b4[w & 3] = ds;
+            atomicAdd(a.loss, ls);
         }
         __syncthreads();
-        if (t < 64) {
-            atomicAdd(&a.grads[oB1 + t], gb1[t]);
-            atomicAdd(&a.grads[oB2 + t], gb2[t]);
-            atomicAdd(&a.grads[oB3 + t], gb3[t]);
-            atomicAdd(&a.grads[oW4 + t], gw4[t]);
-        }
-        if (t == 0) atomicAdd(&a.grads[oB4], gb4[0]);
+        const int k = t >> 6, c = t & 63;
+        const float v = (s_col[0][k][c] + s_col[1][k][c]) + (s_col[2][k][c] + s_col[3][k][c]);
+        atomicAdd(&a.grads[(k == 0 ? oW4 : k == 1 ? oB3 : k == 2 ? oB2 : oB1) + c], v);
+        if (t == 0) atomicAdd(&a.grads[oB4], (s_b4[0] + s_b4[1]) + (s_b4[2] + s_b4[3]));
     }
     // after a wait that gave up (the error word says so), the last commit gets a second bounded
     // wait before the TMEM and shared memory are released (the failed wait flipped the phase)
@@ -432,7 +452,8 @@ using namespace arc;
 struct arc_mlp {
     arc_context* ctx = nullptr;
     float* params = nullptr;  // device FP32 master copy
-    float* grads = nullptr;
+    float* grads = nullptr;   // kParams, then the loss of arc_mlp_gradients; zero between calls
+    float* host = nullptr;    // pinned: what arc_mlp_gradients reads back
     float* adam_m = nullptr;
     float* adam_v = nullptr;
     float* loss = nullptr;
@@ -468,7 +489,7 @@ arc_status mlp_launch(arc_mlp* m, bool train, const void* x, int64_t rows, float
         ARC_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp::kSmemTrain));
         const int grid = (int)std::min<int64_t>(tiles, ctx->sm_count);
         stage_begin(ctx, "mlp_train");
-        k<<<grid, 128, mlp::kSmemTrain, ctx->stream>>>(a);
+        k<<<grid, mlp::kTrainThreads, mlp::kSmemTrain, ctx->stream>>>(a);
         stage_end(ctx, 1);
     } else {
         auto* k = relu ? mlp::mlp_infer_kernel<mlp::kActRelu> : mlp::mlp_infer_kernel<mlp::kActGelu>;
@@ -504,7 +525,8 @@ arc_status arc_mlp_create(arc_context* ctx, uint64_t seed, arc_mlp** out) {
     m->ctx = ctx;
     const size_t bytes = sizeof(float) * mlp::kParams;
     cudaError_t e = cudaMalloc(&m->params, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&m->grads, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&m->grads, bytes + sizeof(float));
+    if (e == cudaSuccess) e = cudaMallocHost(&m->host, bytes + sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&m->adam_m, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&m->adam_v, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(float));
@@ -530,7 +552,7 @@ arc_status arc_mlp_create(arc_context* ctx, uint64_t seed, arc_mlp** out) {
     fill(mlp::oW4, 64, 64);
     fill(mlp::oB4, 1, 64);
     e = cudaMemcpy(m->params, p.data(), bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(m->grads, 0, bytes);
+    if (e == cudaSuccess) e = cudaMemset(m->grads, 0, bytes + sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(m->adam_m, 0, bytes);
     if (e == cudaSuccess) e = cudaMemset(m->adam_v, 0, bytes);
     if (e != cudaSuccess) {
@@ -550,6 +572,7 @@ arc_status arc_mlp_destroy(arc_mlp* m) {
     }
     cudaFree(m->params);
     cudaFree(m->grads);
+    cudaFreeHost(m->host);
     cudaFree(m->adam_m);
     cudaFree(m->adam_v);
     cudaFree(m->loss);
@@ -584,15 +607,20 @@ arc_status arc_mlp_gradients(arc_mlp* m, const void* features_bf16, const float*
                              int64_t rows, float weight_sum, float* host_grads, float* host_loss) {
     ARC_CHECK_ARG(m && features_bf16 && labels && rows > 0 && weight_sum > 0.0f, "bad argument");
     ARC_TRY_CUDA(cudaSetDevice(m->ctx->device));
-    ARC_TRY_CUDA(cudaMemsetAsync(m->grads, 0, sizeof(float) * mlp::kParams, m->ctx->stream));
-    ARC_TRY_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), m->ctx->stream));
-    ARC_TRY(mlp_launch(m, true, features_bf16, rows, nullptr, labels, weights, 1.0f / weight_sum));
-    if (host_grads)
-        ARC_TRY_CUDA(cudaMemcpyAsync(host_grads, m->grads, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost,
-                                     m->ctx->stream));
-    if (host_loss) ARC_TRY_CUDA(cudaMemcpyAsync(host_loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->ctx->stream));
-    ARC_TRY_CUDA(cudaStreamSynchronize(m->ctx->stream));
-    ARC_TRY_CUDA(cudaMemsetAsync(m->grads, 0, sizeof(float) * mlp::kParams, m->ctx->stream));
+    // gradients and loss in one buffer: one copy back (to pinned memory), one clear for the next call
+    const size_t bytes = sizeof(float) * (mlp::kParams + 1);
+    cudaStream_t st = m->ctx->stream;
+    float* saved = m->loss;
+    m->loss = m->grads + mlp::kParams;
+    const arc_status s = mlp_launch(m, true, features_bf16, rows, nullptr, labels, weights, 1.0f / weight_sum);
+    m->loss = saved;
+    ARC_TRY(s);
+    const cudaError_t e = cudaMemcpyAsync(m->host, m->grads, bytes, cudaMemcpyDeviceToHost, st);
+    ARC_TRY_CUDA(cudaMemsetAsync(m->grads, 0, bytes, st));
+    ARC_TRY_CUDA(e);
+    ARC_TRY_CUDA(cudaStreamSynchronize(st));
+    if (host_grads) std::memcpy(host_grads, m->host, sizeof(float) * mlp::kParams);
+    if (host_loss) *host_loss = m->host[mlp::kParams];
     return ARC_OK;
 }
 
