@@ -38,9 +38,10 @@ constexpr uint32_t sW1 = 0, sW2 = sW1 + 2048, sW3 = sW2 + 8192, sX = sW3 + 8192,
                    sH2 = sH1 + 16384, sDZ = sH2 + 16384, sVecTrain = sDZ + 16384 + 2048;
 constexpr uint32_t kVecBytes = 4 * 64 * 4;
 constexpr uint32_t kSmemTrain = sVecTrain + kVecBytes;
-// inference: weights | X tile (4 KB) | hidden (16 KB) | vectors
-constexpr uint32_t sInX = kWeightBytes, sInH = sInX + 4096, sInVec = sInH + 16384,
-                   kSmemInfer = sInVec + kVecBytesInfer;
+// inference: weights and vectors | per group the hidden rows of its tile (16 KB), whose first 4 KB hold
+// the input rows until layer 1 has read them
+constexpr int kInferGroups = 4;
+constexpr uint32_t sInH = ((kImageBytes + 127) / 128) * 128, kSmemInfer = sInH + kInferGroups * 16384;
 
 struct Args {
     const float* params;
@@ -91,49 +92,62 @@ __device__ __forceinline__ float column_sums(float* v, int lane) {
     return v[0];
 }
 
-// Forward over every row of the input: persistent CTAs, one 128-row tile at a time.
+// Forward over every row of the input: persistent CTAs of four 128-thread groups that share the
+// weights and otherwise run on their own (named barriers), one 128-row tile each; two CTAs per SM keep
+// eight tiles in flight.  A tile is a chain of three tensor-core rounds with barriers and epilogues
+// between them, so tiles in flight are what the rate follows; the next tile's rows are loaded while
+// the current one is scored.
 template <int ACT>
-__global__ void __launch_bounds__(128) mlp_infer_kernel(Args a) {
+__global__ void __launch_bounds__(128 * kInferGroups, 2) mlp_infer_kernel(Args a) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bars[kInferGroups];
     __shared__ uint32_t tmem_base;
-    const int t = threadIdx.x, w = t >> 5;
-    float* vec = reinterpret_cast<float*>(sm + sInVec);
-    load_weights<ACT>(sm, vec, a.params, t, 128);
-    if (w == 0) tc::alloc(&tmem_base, 64);
-    if (t == 0) {
-        mbar_init(&bar, 1);
+    const int t = threadIdx.x & 127, g = threadIdx.x >> 7;
+    float* vec = reinterpret_cast<float*>(sm + kWeightBytes);
+    load_weights<ACT>(sm, vec, a.params, threadIdx.x, 128 * kInferGroups);
+    if (threadIdx.x < 32) tc::alloc(&tmem_base, 64 * kInferGroups);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kInferGroups; ++i) mbar_init(&bars[i], 1);
         fence_mbar_init();
     }
     fence_proxy_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    InferCta c{smem_u32(sm), 0, sInH, sm, vec, tmem_base, &bar, 0u, a.err};
-    const int64_t ntiles = (a.rows + kRows - 1) / kRows;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint32_t h = sInH + 16384u * g;
+    InferCta c{smem_u32(sm), 0, h, sm, vec, tmem_base + 64u * g, &bars[g], 0u, a.err};
+    const GroupSync group{1 + g};
+    const int64_t ntiles = (a.rows + kRows - 1) / kRows, step = (int64_t)gridDim.x * kInferGroups;
+    uint4 x0, x1;
+    auto load_rows = [&](int64_t tile) {
         const int64_t row = tile * kRows + t;
-        const bool valid = row < a.rows;
-        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = make_uint4(0, 0, 0, 0);
-        if (valid) {
+        x0 = x1 = make_uint4(0, 0, 0, 0);
+        if (tile < ntiles && row < a.rows) {
             const uint4* xp = reinterpret_cast<const uint4*>(a.x + row * kIn);
             x0 = xp[0];
             x1 = xp[1];
         }
-        *reinterpret_cast<uint4*>(sm + sInX + tc::kmajor_offset(t, 0, kIn)) = x0;
-        *reinterpret_cast<uint4*>(sm + sInX + tc::kmajor_offset(t, 8, kIn)) = x1;
+    };
+    // consecutive tiles go to different CTAs, so that a small input spreads over the SMs
+    int64_t tile = (int64_t)g * gridDim.x + blockIdx.x;
+    load_rows(tile);
+    for (; tile < ntiles; tile += step) {
+        *reinterpret_cast<uint4*>(sm + h + tc::kmajor_offset(t, 0, kIn)) = x0;
+        *reinterpret_cast<uint4*>(sm + h + tc::kmajor_offset(t, 8, kIn)) = x1;
+        load_rows(tile + step);
         float y;
-        if (!infer_tile<ACT>(c, sInX, t, &y)) {
+        if (!infer_tiles<1, ACT, 32>(c, h, t, &y, group)) {
             // the wait gave up (the error word says so): its commit gets a second bounded wait
             // before the TMEM and shared memory are released (the failed wait flipped the phase)
-            if (t == 0) mbar_wait_bounded(&bar, c.phase ^ 1u, a.err);
+            if (t == 0) mbar_wait_bounded(c.bar, c.phase ^ 1u, a.err);
             break;
         }
-        if (valid) a.logits[row] = y;
+        const int64_t row = tile * kRows + t;
+        if (row < a.rows) a.logits[row] = y;
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (w == 0) tc::dealloc(tmem_base, 64);
+    if (threadIdx.x < 32) tc::dealloc(tmem_base, 64 * kInferGroups);
 }
 
 // Forward + backward with weight-gradient accumulation in TMEM (training).  256 threads per 128-row
@@ -159,7 +173,7 @@ __device__ __forceinline__ void red_add4(float* dst, const float* v) {
 }
 
 template <int ACT>
-__global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(Args a) {
+__global__ void __launch_bounds__(kTrainThreads, 2) mlp_train_kernel(Args a) {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
@@ -487,16 +501,19 @@ arc_status mlp_launch(arc_mlp* m, bool train, const void* x, int64_t rows, float
     if (train) {
         auto* k = relu ? mlp::mlp_train_kernel<mlp::kActRelu> : mlp::mlp_train_kernel<mlp::kActGelu>;
         ARC_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp::kSmemTrain));
-        const int grid = (int)std::min<int64_t>(tiles, ctx->sm_count);
+        // Two CTAs per SM overlap each other's tensor-core rounds once each has several tiles (500,000
+        // rows: 140 against 170 us); with few tiles a second CTA only adds weight loads and reductions.
+        const int per_sm = tiles >= 8 * (int64_t)ctx->sm_count ? 2 : 1;
+        const int grid = (int)std::min<int64_t>(tiles, (int64_t)ctx->sm_count * per_sm);
         stage_begin(ctx, "mlp_train");
         k<<<grid, mlp::kTrainThreads, mlp::kSmemTrain, ctx->stream>>>(a);
         stage_end(ctx, 1);
     } else {
         auto* k = relu ? mlp::mlp_infer_kernel<mlp::kActRelu> : mlp::mlp_infer_kernel<mlp::kActGelu>;
         ARC_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp::kSmemInfer));
-        const int grid = (int)std::min<int64_t>(tiles, (int64_t)ctx->sm_count * 4);
+        const int grid = (int)std::min<int64_t>(tiles, (int64_t)ctx->sm_count * 2);
         stage_begin(ctx, "mlp_forward");
-        k<<<grid, 128, mlp::kSmemInfer, ctx->stream>>>(a);
+        k<<<grid, 128 * mlp::kInferGroups, mlp::kSmemInfer, ctx->stream>>>(a);
         stage_end(ctx, 1);
     }
     ARC_TRY_CUDA(cudaGetLastError());

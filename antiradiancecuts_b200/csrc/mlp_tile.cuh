@@ -132,14 +132,16 @@ template <int ACT>
 __device__ __forceinline__ void load_weights(unsigned char* w, float* vec, const float* params, int t, int nthreads) {
     const float s1 = ACT == kActGelu ? kGeluS : 1.0f, sh = ACT == kActGelu ? 0.5f : 1.0f,
                 sb = ACT == kActGelu ? kGeluS : 1.0f, so = ACT == kActGelu ? kGeluOut : 1.0f;
-    for (int i = t; i < kHid * kIn; i += nthreads)
-        *reinterpret_cast<__nv_bfloat16*>(w + kW1 + tc::kmajor_offset(i / kIn, i % kIn, kIn)) =
-            __float2bfloat16_rn(s1 * params[oW1 + i]);
-    for (int i = t; i < kHid * kHid; i += nthreads) {
-        *reinterpret_cast<__nv_bfloat16*>(w + kW2 + tc::kmajor_offset(i / kHid, i % kHid, kHid)) =
-            __float2bfloat16_rn(sh * params[oW2 + i]);
-        *reinterpret_cast<__nv_bfloat16*>(w + kW3 + tc::kmajor_offset(i / kHid, i % kHid, kHid)) =
-            __float2bfloat16_rn(sh * params[oW3 + i]);
+    // four weights per 16-byte load (their offsets in the parameters are multiples of four)
+    auto put4 = [&](uint32_t at, int first, int i, int K, float scale) {
+        const float4 v = *reinterpret_cast<const float4*>(params + first + 4 * i);
+        *reinterpret_cast<uint2*>(w + at + tc::kmajor_offset(4 * i / K, 4 * i % K, K)) =
+            make_uint2(pack2(scale * v.x, scale * v.y), pack2(scale * v.z, scale * v.w));
+    };
+    for (int i = t; i < kHid * kIn / 4; i += nthreads) put4(kW1, oW1, i, kIn, s1);
+    for (int i = t; i < kHid * kHid / 4; i += nthreads) {
+        put4(kW2, oW2, i, kHid, sh);
+        put4(kW3, oW3, i, kHid, sh);
     }
     for (int i = t; i < 64; i += nthreads) {
         vec[i] = sb * params[oB1 + i];
@@ -164,19 +166,44 @@ struct InferCta {
     uint32_t* err;
 };
 
+// The threads that score together: the whole CTA, or 128 of its threads on named barrier `id` (each such
+// group has its own tile, hidden rows, TMEM columns and mbarrier, and never waits for the others).
+struct CtaSync {
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+    __device__ __forceinline__ bool all(bool ok) const { return __syncthreads_and(ok) != 0; }
+};
+struct GroupSync {
+    int id;
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+    __device__ __forceinline__ bool all(bool ok) const {
+        int r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.b32 q, %1, 0;\n\t"
+            "bar.red.and.pred p, %2, 128, q;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(r)
+            : "r"((int)ok), "r"(id)
+            : "memory");
+        return r != 0;
+    }
+};
+
 // Waits for the MMAs committed on the barrier; every thread learns whether all threads got there.
-__device__ __forceinline__ bool wait_mma(InferCta& c) {
+template <class Sync>
+__device__ __forceinline__ bool wait_mma(InferCta& c, const Sync& s) {
     const bool ok = mbar_wait_bounded(c.bar, c.phase, c.err);
     c.phase ^= 1u;
     tc::fence_after_sync();
-    return __syncthreads_and(ok) != 0;
+    return s.all(ok);
 }
 
 // Makes this thread's generic-proxy smem writes visible to the tensor cores, then barrier.
-__device__ __forceinline__ void publish_smem() {
+template <class Sync>
+__device__ __forceinline__ void publish_smem(const Sync& s) {
     fence_proxy_async_smem();
     tc::fence_before_sync();
-    __syncthreads();
+    s.sync();
 }
 
 // TMEM address of thread t's row: tile t / 128 owns accumulator columns 64 (t / 128) ..+63, and a
@@ -185,38 +212,48 @@ __device__ __forceinline__ uint32_t row_tmem(const InferCta& c, int t) {
     return c.tmem + ((uint32_t)(((t >> 5) & 3) * 32) << 16) + 64u * (uint32_t)(t >> 7);
 }
 
-// Hidden layer epilogue for this thread's row: 16 columns at a time from TMEM, + bias, the
-// activation, BF16 into the K-major hidden buffer (rows of all tiles, 64 columns).
-template <int ACT>
+// W consecutive accumulator columns of this thread's row (one wait per load)
+template <int W>
+__device__ __forceinline__ void load_columns(uint32_t taddr, float* z) {
+    if constexpr (W == 32) tc::ld32(taddr, z);
+    else tc::ld16(taddr, z);
+}
+
+// Hidden layer epilogue for this thread's row: W columns at a time from TMEM, + bias, the activation,
+// BF16 into the K-major hidden buffer (rows of all tiles, 64 columns).
+template <int ACT, int W>
 __device__ __forceinline__ void hidden_epilogue(const InferCta& c, int t, const float* bias) {
     const uint32_t taddr = row_tmem(c, t);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float z[16];
-        tc::ld16(taddr + 16 * q, z);
-        uint32_t u[8];
+    for (int q = 0; q < 64 / W; ++q) {
+        float z[W];
+        load_columns<W>(taddr + W * q, z);
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {  // biases four at a time (one broadcast 16-byte load)
-            const float4 bb = *reinterpret_cast<const float4*>(bias + 16 * q + 2 * j);
-            u[j] = hidden_pair<ACT>(f2(z[2 * j], z[2 * j + 1]), f2(bb.x, bb.y));
-            u[j + 1] = hidden_pair<ACT>(f2(z[2 * j + 2], z[2 * j + 3]), f2(bb.z, bb.w));
+        for (int i = 0; i < W / 8; ++i) {
+            uint32_t u[4];
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {  // biases four at a time (one broadcast 16-byte load)
+                const float* v = z + 8 * i + 2 * j;
+                const float4 bb = *reinterpret_cast<const float4*>(bias + W * q + 8 * i + 2 * j);
+                u[j] = hidden_pair<ACT>(f2(v[0], v[1]), f2(bb.x, bb.y));
+                u[j + 1] = hidden_pair<ACT>(f2(v[2], v[3]), f2(bb.z, bb.w));
+            }
+            *reinterpret_cast<uint4*>(c.sm + c.h + tc::kmajor_offset(t, W * q + 8 * i, 64)) =
+                make_uint4(u[0], u[1], u[2], u[3]);
         }
-        *reinterpret_cast<uint4*>(c.sm + c.h + tc::kmajor_offset(t, 16 * q, 64)) = make_uint4(u[0], u[1], u[2], u[3]);
-        *reinterpret_cast<uint4*>(c.sm + c.h + tc::kmajor_offset(t, 16 * q + 8, 64)) =
-            make_uint4(u[4], u[5], u[6], u[7]);
     }
 }
 
-// Logits of NT 128-row tiles: row t (of 128 NT, one per thread of the CTA) of the K-major input
+// Logits of NT 128-row tiles: row t (of 128 NT, one per thread of the group) of the K-major input
 // rows at smem offset x (stride between 8-row groups: 256 bytes), hidden rows at c.h (1024 bytes
-// between 8-row groups), tile u's accumulator in TMEM columns 64 u .. 64 u + 63.  Called by all
-// 128 NT threads; returns false (every thread) if a tensor-core wait gave up, after which the
-// caller frees its TMEM and stops.
-template <int NT, int ACT>
-__device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, float* logit) {
+// between 8-row groups; the input rows may lie in their first 4096 NT bytes), tile u's accumulator in
+// TMEM columns 64 u .. 64 u + 63.  Called by all 128 NT threads; returns false (every thread) if a
+// tensor-core wait gave up, after which the caller frees its TMEM and stops.
+template <int NT, int ACT, int W = 16, class Sync = CtaSync>
+__device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, float* logit, const Sync& s = Sync()) {
     constexpr uint32_t id = tc::idesc_bf16(128, 64, false, false);
     // layer 1 (K = 16)
-    publish_smem();
+    publish_smem(s);
     if (t == 0) {
         tc::fence_after_sync();
 #pragma unroll
@@ -225,25 +262,25 @@ __device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, floa
                     tc::smem_desc(c.base + c.w + kW1, 128, 256), id, false);
         tc::commit(c.bar);
     }
-    if (!wait_mma(c)) return false;
-    hidden_epilogue<ACT>(c, t, c.vec);
+    if (!wait_mma(c, s)) return false;
+    hidden_epilogue<ACT, W>(c, t, c.vec);
     // layers 2 and 3 (K = 64); layer 2 overwrites the hidden buffer it read once its MMAs are done
 #pragma unroll 1
     for (int l = 0; l < 2; ++l) {
-        publish_smem();
+        publish_smem(s);
         if (t == 0) {
             tc::fence_after_sync();
             const uint32_t wb = c.w + (l == 0 ? kW2 : kW3);
 #pragma unroll
             for (int u = 0; u < NT; ++u)
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    tc::mma(c.tmem + 64 * u, tc::smem_desc(c.base + c.h + 16384 * u + 256 * s, 128, 1024),
-                            tc::smem_desc(c.base + wb + 256 * s, 128, 1024), id, s > 0);
+                for (int k = 0; k < 4; ++k)
+                    tc::mma(c.tmem + 64 * u, tc::smem_desc(c.base + c.h + 16384 * u + 256 * k, 128, 1024),
+                            tc::smem_desc(c.base + wb + 256 * k, 128, 1024), id, k > 0);
             tc::commit(c.bar);
         }
-        if (!wait_mma(c)) return false;
-        if (l == 0) hidden_epilogue<ACT>(c, t, c.vec + 64);
+        if (!wait_mma(c, s)) return false;
+        if (l == 0) hidden_epilogue<ACT, W>(c, t, c.vec + 64);
     }
     // layer 3 epilogue and the 64 -> 1 output layer on the CUDA cores
     const uint32_t taddr = row_tmem(c, t);
@@ -251,15 +288,15 @@ __device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, floa
     const float* w4 = c.vec + 192;
     uint64_t y2 = f2(c.vec[256], 0.0f);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float z[16];
-        tc::ld16(taddr + 16 * q, z);
+    for (int q = 0; q < 64 / W; ++q) {
+        float z[W];
+        load_columns<W>(taddr + W * q, z);
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-            const float4 bb = *reinterpret_cast<const float4*>(b3 + 16 * q + 2 * j);
-            const float4 ww = *reinterpret_cast<const float4*>(w4 + 16 * q + 2 * j);
-            y2 = output_pair<ACT>(f2(z[2 * j], z[2 * j + 1]), f2(bb.x, bb.y), f2(ww.x, ww.y), y2);
-            y2 = output_pair<ACT>(f2(z[2 * j + 2], z[2 * j + 3]), f2(bb.z, bb.w), f2(ww.z, ww.w), y2);
+        for (int j = 0; j < W; j += 4) {
+            const float4 bb = *reinterpret_cast<const float4*>(b3 + W * q + j);
+            const float4 ww = *reinterpret_cast<const float4*>(w4 + W * q + j);
+            y2 = output_pair<ACT>(f2(z[j], z[j + 1]), f2(bb.x, bb.y), f2(ww.x, ww.y), y2);
+            y2 = output_pair<ACT>(f2(z[j + 2], z[j + 3]), f2(bb.z, bb.w), f2(ww.z, ww.w), y2);
         }
     }
     float y0, y1;
@@ -269,11 +306,6 @@ __device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, floa
     tc::fence_before_sync();
     *logit = y;
     return true;
-}
-
-template <int ACT>
-__device__ __forceinline__ bool infer_tile(InferCta& c, uint32_t x, int t, float* logit) {
-    return infer_tiles<1, ACT>(c, x, t, logit);
 }
 
 }  // namespace mlp
