@@ -242,9 +242,10 @@ constexpr int kLevelThreads = 256;
 // (the same node for consecutive tiles) becomes two runs that share its children.  The initial
 // frontier holds the root for every tile, so every level stays grouped by node, and a warp's
 // loads of node data mostly touch one or two nodes.  Every thread of the CTA calls it (it holds
-// barriers); se: 2 * warps + 3 shared ints, not touched by anything else.
-__device__ __forceinline__ void emit(const LevelArgs& a, int* se, int action, int tile, int node, int lc, int rc,
-                                     int depth) {
+// barriers) and learns whether all of them are `ok`; se: 2 * warps + 3 shared ints, not touched by
+// anything else.
+__device__ __forceinline__ bool emit(const LevelArgs& a, int* se, bool ok, int action, int tile, int node, int lc,
+                                     int rc, int depth) {
     constexpr int kW = kLevelThreads / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -254,21 +255,21 @@ __device__ __forceinline__ void emit(const LevelArgs& a, int* se, int action, in
         se[w] = __popc(am);
         se[kW + w] = __popc(pm);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int sa = 0, sp = 0;
+    const bool all_ok = __syncthreads_and(ok) != 0;
+    if (lane == 0 && w < 2) {  // warp 0 reserves the accepts, warp 1 the pushes
+        int* cnt = se + kW * w;
+        int sum = 0;
         for (int i = 0; i < kW; ++i) {
-            const int x = se[i], y = se[kW + i];
-            se[i] = sa;
-            se[kW + i] = sp;
-            sa += x;
-            sp += y;
+            const int x = cnt[i];
+            cnt[i] = sum;
+            sum += x;
         }
-        const int ba = sa ? atomicAdd(a.acc_count, sa) : 0;
-        const int bp = sp ? atomicAdd(a.out_count, 2 * sp) : 0;
-        se[2 * kW] = ba;
-        se[2 * kW + 1] = bp;
-        se[2 * kW + 2] = sp;
+        if (w == 0) {
+            se[2 * kW] = sum ? atomicAdd(a.acc_count, sum) : 0;
+        } else {
+            se[2 * kW + 1] = sum ? atomicAdd(a.out_count, 2 * sum) : 0;
+            se[2 * kW + 2] = sum;
+        }
     }
     __syncthreads();
     if (action == kAccept) {
@@ -292,6 +293,7 @@ __device__ __forceinline__ void emit(const LevelArgs& a, int* se, int action, in
         if (okr) a.out[pr] = entry(tile, rc, depth + 1);
         if (!okl || !okr) set_error(a.err, ARC_DEVERR_CUT_OVERFLOW);
     }
+    return all_ok;
 }
 
 // learned_level: 256 threads, one pair per thread per chunk, rows scored two 128-row tiles at a
@@ -306,7 +308,8 @@ constexpr uint32_t kLevelTmemCols = 64 * kLevelTiles;
 // BF16 core-matrix weights + FP32 vectors, once per selection
 template <int ACT>
 __global__ void weight_image(const float* params, unsigned char* img) {
-    mlp::load_weights<ACT>(img, reinterpret_cast<float*>(img + mlp::kWeightBytes), params, threadIdx.x, blockDim.x);
+    mlp::load_weights<ACT>(img, reinterpret_cast<float*>(img + mlp::kWeightBytes), params,
+                           blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 template <int ACT>
@@ -337,7 +340,6 @@ __global__ void __launch_bounds__(kLevelThreads) learned_level(LevelArgs a) {
     __syncthreads();
     tc::fence_after_sync();
     bool ok = __syncthreads_and(mbar_wait_bounded(&wbar, 0, a.err)) != 0;
-    bool mma_gave_up = false;  // a tensor-core wait gave up: its commit may still be in flight
     mlp::InferCta c{smem_u32(sm), fW, fH, sm, vec, tmem_base, &bar, 0u, a.err};
     unsigned long long scored = 0;
     // The next chunk's index and entries are fetched one chunk ahead, so that neither the work
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(kLevelThreads) learned_level(LevelArgs a) {
         }
         if (t == 0 && !done) s_chunk = next;
         // emit's barriers also order every staging of this chunk before s_staged is read
-        emit(a, s_emit, action, tile, node, lc, rc, depth);
+        emit(a, s_emit, true, action, tile, node, lc, rc, depth);
         if (!done) {
             chunk = s_chunk;
             const int64_t en = (int64_t)chunk * kLevelThreads + t;
@@ -429,17 +431,16 @@ __global__ void __launch_bounds__(kLevelThreads) learned_level(LevelArgs a) {
                 }
             }
             float y = 0.0f;
-            if (!mlp::infer_tiles<kLevelTiles, ACT>(c, fX, t, &y)) {
-                ok = false;
-                mma_gave_up = true;
-                break;
-            }
+            const bool scored_ok = mlp::infer_tiles<kLevelTiles, ACT, true>(c, fX, t, &y, mlp::CtaSync());
             scored += n_rows;
             const int act = t < n_rows ? (y >= a.thr_logit ? kRefine : kAccept) : kNone;
             const int mnode = m.y & ((1 << kDepthShift) - 1), mdepth = m.y >> kDepthShift;
             const int mlc = child_index(cl, a.n), mrc = child_index(cr, a.n);
             // after emit's barriers every thread has read its pair: the rows can be moved
-            emit(a, s_emit, act, m.x, mnode, mlc, mrc, mdepth);
+            if (!emit(a, s_emit, scored_ok, act, m.x, mnode, mlc, mrc, mdepth)) {
+                ok = false;  // (the error word says so; the pairs emitted meanwhile are valid ones)
+                break;
+            }
             const int rest = staged - n_rows;
             if (t < rest) {
                 const int r = kLevelThreads + t;
@@ -459,9 +460,9 @@ __global__ void __launch_bounds__(kLevelThreads) learned_level(LevelArgs a) {
     if (!ok && t == 0) {
         // a bounded wait gave up (the error word says so): before this CTA's shared memory and
         // TMEM are released, give its weight copy and its last tensor-core commit a second
-        // bounded wait (the failed wait has already flipped the phase)
+        // bounded wait
         mbar_wait_bounded(&wbar, 0, a.err);
-        if (mma_gave_up) mbar_wait_bounded(&bar, c.phase ^ 1u, a.err);
+        if (!c.ok) mlp::drain_mma(c);
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -858,8 +859,12 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     ARC_TRY(arena_get(ctx, "lc_front_b", cap, &fb));
     ARC_TRY(arena_get(ctx, "lc_accepted", acc_cap, &accepted));
     // counters: [3] accepted, [4] total chunks, then per level l at 8 + 4 l: [0] entries, [2] work
-    constexpr int kMaxLevels = 96;
+    constexpr int kMaxLevels = 64;
     constexpr int kSlots = 8 + 4 * (kMaxLevels + 1);
+    // Each level of the radix tree adds at least one bit to the common prefix of (Morton code, leaf
+    // index): at most 32 + ceil(log2 n) levels of inner nodes, and one of leaves.
+    int levels = 33;
+    while (levels < kMaxLevels && ((int64_t)1 << (levels - 33)) < n) ++levels;
     ARC_TRY(arena_get(ctx, "lc_counters", kSlots, &counters));
     ARC_TRY(arena_get(ctx, "lc_tile_counts", tiles, &tile_counts));
     ARC_TRY(arena_get(ctx, "lc_chunk_base", tiles, &chunk_base));
@@ -913,18 +918,18 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     int kernels = 0;
     const int grid = ctx->sm_count * 8;
     if (relu)
-        weight_image<mlp::kActRelu><<<1, 256, 0, st>>>(mlp_params(cp->model), img);
+        weight_image<mlp::kActRelu><<<16, 256, 0, st>>>(mlp_params(cp->model), img);
     else
-        weight_image<mlp::kActGelu><<<1, 256, 0, st>>>(mlp_params(cp->model), img);
+        weight_image<mlp::kActGelu><<<16, 256, 0, st>>>(mlp_params(cp->model), img);
     init_frontier<<<(tiles + 255) / 256, 256, 0, st>>>(fa, counters + 8, info, tiles, n);
     tile_info_transpose<<<(tiles + 255) / 256, 256, 0, st>>>(info, info_t, tiles);
     kernels += 3;
     int2 *cur = fa, *nxt = fb;
-    // Every level up to kMaxLevels is launched without reading anything back: a launch past the
-    // tree's last level finds an empty frontier and returns at once, so the selection holds no
-    // host synchronisation and can be recorded into a CUDA graph.  Pairs still in the frontier
-    // after the last launch (a tree deeper than kMaxLevels) are accepted.
-    for (int level = 0; level < kMaxLevels; ++level) {
+    // Every possible level is launched without reading anything back: a launch past the tree's last
+    // level finds an empty frontier and returns at once (about 2 us), so the selection holds no host
+    // synchronisation and can be recorded into a CUDA graph.  (Pairs still in the frontier after the
+    // last launch, which a valid tree never leaves, are accepted.)
+    for (int level = 0; level < levels; ++level) {
         la.in = cur;
         la.in_count = counters + 8 + 4 * level;
         la.work = counters + 8 + 4 * level + 2;
@@ -935,7 +940,7 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
         std::swap(cur, nxt);
     }
     la.in = cur;
-    la.in_count = counters + 8 + 4 * kMaxLevels;
+    la.in_count = counters + 8 + 4 * levels;
     accept_frontier<<<grid, 256, 0, st>>>(la);
     ++kernels;
     stage_end(ctx, kernels);

@@ -136,10 +136,8 @@ __global__ void __launch_bounds__(128 * kInferGroups, 2) mlp_infer_kernel(Args a
         *reinterpret_cast<uint4*>(sm + h + tc::kmajor_offset(t, 8, kIn)) = x1;
         load_rows(tile + step);
         float y;
-        if (!infer_tiles<1, ACT, 32>(c, h, t, &y, group)) {
-            // the wait gave up (the error word says so): its commit gets a second bounded wait
-            // before the TMEM and shared memory are released (the failed wait flipped the phase)
-            if (t == 0) mbar_wait_bounded(c.bar, c.phase ^ 1u, a.err);
+        if (!group.all(infer_tiles<1, ACT, false>(c, h, t, &y, group))) {  // (the error word says so)
+            if (t == 0) drain_mma(c);
             break;
         }
         const int64_t row = tile * kRows + t;

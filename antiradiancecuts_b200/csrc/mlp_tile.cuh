@@ -164,6 +164,8 @@ struct InferCta {
     uint64_t* bar;
     uint32_t phase;  // parity of the next barrier completion
     uint32_t* err;
+    bool ok = true;         // this thread's waits have all succeeded
+    uint32_t committed = 0; // issuing thread: parity of its last commit
 };
 
 // The threads that score together: the whole CTA, or 128 of its threads on named barrier `id` (each such
@@ -189,14 +191,19 @@ struct GroupSync {
     }
 };
 
-// Waits for the MMAs committed on the barrier; every thread learns whether all threads got there.
-template <class Sync>
-__device__ __forceinline__ bool wait_mma(InferCta& c, const Sync& s) {
-    const bool ok = mbar_wait_bounded(c.bar, c.phase, c.err);
+// Waits for the MMAs committed on the barrier.  A wait that gives up is remembered in c.ok, without a
+// barrier to tell the other threads (three per tile cost 5% of the learned selection): the issuing
+// thread issues nothing more, so every thread's next wait gives up too at the latest, and the caller
+// learns of it at its own next barrier.
+__device__ __forceinline__ void wait_mma(InferCta& c) {
+    if (!mbar_wait_bounded(c.bar, c.phase, c.err)) c.ok = false;
     c.phase ^= 1u;
     tc::fence_after_sync();
-    return s.all(ok);
 }
+
+// A CTA that stops after a wait gave up: the issuing thread gives its last commit a second bounded wait
+// before the TMEM and the shared memory are released.
+__device__ __forceinline__ void drain_mma(const InferCta& c) { mbar_wait_bounded(c.bar, c.committed, c.err); }
 
 // Makes this thread's generic-proxy smem writes visible to the tensor cores, then barrier.
 template <class Sync>
@@ -206,55 +213,126 @@ __device__ __forceinline__ void publish_smem(const Sync& s) {
     s.sync();
 }
 
-// TMEM address of thread t's row: tile t / 128 owns accumulator columns 64 (t / 128) ..+63, and a
-// warp may only read its lane quarter, 32 ((t / 32) % 4) .. +31.
-__device__ __forceinline__ uint32_t row_tmem(const InferCta& c, int t) {
-    return c.tmem + ((uint32_t)(((t >> 5) & 3) * 32) << 16) + 64u * (uint32_t)(t >> 7);
+// The epilogues read the accumulators as MMA fragments: a thread then holds few columns of several rows
+// (2 of every 8 columns, 4 of the warp's 32 rows), so it needs 16 of a layer's 64 biases instead of all
+// of them, and a warp stores whole 8 x 8 core matrices with stmatrix.  (With one row per thread the
+// broadcast loads of biases and output weights took most of the shared-memory bandwidth that the tensor
+// cores' operands also need: L1 at 90%.)
+
+// TMEM address of rows 16 h .. 16 h + 15 of thread t's warp: tile t / 128 owns accumulator columns
+// 64 (t / 128) ..+63, and a warp may only read its lane quarter, 32 ((t / 32) % 4) .. +31.
+__device__ __forceinline__ uint32_t rows_tmem(const InferCta& c, int t, int h) {
+    return c.tmem + ((uint32_t)(((t >> 5) & 3) * 32 + 16 * h) << 16) + 64u * (uint32_t)(t >> 7);
 }
 
-// W consecutive accumulator columns of this thread's row (one wait per load)
-template <int W>
-__device__ __forceinline__ void load_columns(uint32_t taddr, float* z) {
-    if constexpr (W == 32) tc::ld32(taddr, z);
-    else tc::ld16(taddr, z);
+// this thread's pairs of a 64-vector: columns 2 (lane % 4), + 1 of each 8-column block of 32
+__device__ __forceinline__ void load_pairs(const float* v, int lane, uint64_t* p) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const uint64_t*>(v + 8 * i + 2 * (lane & 3));
 }
 
-// Hidden layer epilogue for this thread's row: W columns at a time from TMEM, + bias, the activation,
-// BF16 into the K-major hidden buffer (rows of all tiles, 64 columns).
-template <int ACT, int W>
+// Hidden layer epilogue for the warp's 32 rows: 32 columns of 16 rows at a time from TMEM, + bias, the
+// activation, BF16 into the K-major hidden buffer (rows of all tiles, 64 columns).
+template <int ACT>
 __device__ __forceinline__ void hidden_epilogue(const InferCta& c, int t, const float* bias) {
-    const uint32_t taddr = row_tmem(c, t);
+    const int lane = t & 31, row0 = t & ~31;
+    // address of the core-matrix row this lane stores: 8-row group (lane / 8) % 2, 8-column block lane / 16
+    const uint32_t dst = c.base + c.h + tc::kmajor_offset(row0 + (lane & 15), 8 * (lane >> 4), 64);
 #pragma unroll
-    for (int q = 0; q < 64 / W; ++q) {
-        float z[W];
-        load_columns<W>(taddr + W * q, z);
+    for (int q = 0; q < 2; ++q) {
+        uint64_t b[4];
+        load_pairs(bias + 32 * q, lane, b);
 #pragma unroll
-        for (int i = 0; i < W / 8; ++i) {
-            uint32_t u[4];
+        for (int h = 0; h < 2; ++h) {
+            float z[16];
+            tc::ld_frag32(rows_tmem(c, t, h) + 32 * q, z);
 #pragma unroll
-            for (int j = 0; j < 4; j += 2) {  // biases four at a time (one broadcast 16-byte load)
-                const float* v = z + 8 * i + 2 * j;
-                const float4 bb = *reinterpret_cast<const float4*>(bias + W * q + 8 * i + 2 * j);
-                u[j] = hidden_pair<ACT>(f2(v[0], v[1]), f2(bb.x, bb.y));
-                u[j + 1] = hidden_pair<ACT>(f2(v[2], v[3]), f2(bb.z, bb.w));
-            }
-            *reinterpret_cast<uint4*>(c.sm + c.h + tc::kmajor_offset(t, W * q + 8 * i, 64)) =
-                make_uint4(u[0], u[1], u[2], u[3]);
+            for (int i = 0; i < 4; i += 2)
+                tc::stmatrix4(dst + 2048 * h + (32 * q / 8 + i) * 128,
+                              hidden_pair<ACT>(f2(z[4 * i], z[4 * i + 1]), b[i]),
+                              hidden_pair<ACT>(f2(z[4 * i + 2], z[4 * i + 3]), b[i]),
+                              hidden_pair<ACT>(f2(z[4 * i + 4], z[4 * i + 5]), b[i + 1]),
+                              hidden_pair<ACT>(f2(z[4 * i + 6], z[4 * i + 7]), b[i + 1]));
         }
     }
+}
+
+// Layer 3 epilogue and the 64 -> 1 output layer: the logit of row t.
+template <int ACT>
+__device__ __forceinline__ float output_epilogue(const InferCta& c, int t) {
+    const int lane = t & 31;
+    uint64_t y2[2][2] = {};  // [row half][row T / 4 or T / 4 + 8], even and odd columns
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        uint64_t b[4], wt[4];
+        load_pairs(c.vec + 128 + 32 * q, lane, b);
+        load_pairs(c.vec + 192 + 32 * q, lane, wt);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float z[16];
+            tc::ld_frag32(rows_tmem(c, t, h) + 32 * q, z);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                y2[h][0] = output_pair<ACT>(f2(z[4 * i], z[4 * i + 1]), b[i], wt[i], y2[h][0]);
+                y2[h][1] = output_pair<ACT>(f2(z[4 * i + 2], z[4 * i + 3]), b[i], wt[i], y2[h][1]);
+            }
+        }
+    }
+    // sums over the four lanes that share a row, then row t's to thread t
+    float y = 0.0f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float lo, hi;
+            f2_split(y2[h][e], lo, hi);
+            float v = lo + hi;
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v = __shfl_sync(0xffffffffu, v, 4 * (lane & 7));
+            if ((lane >> 3) == 2 * h + e) y = v;
+        }
+    return y + c.vec[256];
+}
+
+// The same with one row per thread and its columns in order: the sum that the learned selection
+// compares with its threshold (another order of the sum, 1e-7 away, decides a few pairs per frame the
+// other way, which moves single pixels of the antiradiance by 1e-3).
+template <int ACT>
+__device__ __forceinline__ float output_in_order(const InferCta& c, int t) {
+    const uint32_t taddr = rows_tmem(c, t, 0);
+    const float* b3 = c.vec + 128;
+    const float* w4 = c.vec + 192;
+    uint64_t y2 = f2(c.vec[256], 0.0f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float z[16];
+        tc::ld16(taddr + 16 * q, z);
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+            const float4 bb = *reinterpret_cast<const float4*>(b3 + 16 * q + j);
+            const float4 ww = *reinterpret_cast<const float4*>(w4 + 16 * q + j);
+            y2 = output_pair<ACT>(f2(z[j], z[j + 1]), f2(bb.x, bb.y), f2(ww.x, ww.y), y2);
+            y2 = output_pair<ACT>(f2(z[j + 2], z[j + 3]), f2(bb.z, bb.w), f2(ww.z, ww.w), y2);
+        }
+    }
+    float y0, y1;
+    f2_split(y2, y0, y1);
+    return y0 + y1;
 }
 
 // Logits of NT 128-row tiles: row t (of 128 NT, one per thread of the group) of the K-major input
 // rows at smem offset x (stride between 8-row groups: 256 bytes), hidden rows at c.h (1024 bytes
 // between 8-row groups; the input rows may lie in their first 4096 NT bytes), tile u's accumulator in
-// TMEM columns 64 u .. 64 u + 63.  Called by all 128 NT threads; returns false (every thread) if a
-// tensor-core wait gave up, after which the caller frees its TMEM and stops.
-template <int NT, int ACT, int W = 16, class Sync = CtaSync>
-__device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, float* logit, const Sync& s = Sync()) {
+// TMEM columns 64 u .. 64 u + 63.  Called by all 128 NT threads; returns c.ok: false for a thread whose
+// tensor-core wait gave up, after which the CTA calls drain_mma, frees its TMEM and stops.
+template <int NT, int ACT, bool IN_ORDER, class Sync>
+__device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, float* logit, const Sync& s) {
     constexpr uint32_t id = tc::idesc_bf16(128, 64, false, false);
     // layer 1 (K = 16)
     publish_smem(s);
-    if (t == 0) {
+    if (t == 0 && c.ok) {
+        c.committed = c.phase;
         tc::fence_after_sync();
 #pragma unroll
         for (int u = 0; u < NT; ++u)
@@ -262,13 +340,14 @@ __device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, floa
                     tc::smem_desc(c.base + c.w + kW1, 128, 256), id, false);
         tc::commit(c.bar);
     }
-    if (!wait_mma(c, s)) return false;
-    hidden_epilogue<ACT, W>(c, t, c.vec);
+    wait_mma(c);
+    hidden_epilogue<ACT>(c, t, c.vec);
     // layers 2 and 3 (K = 64); layer 2 overwrites the hidden buffer it read once its MMAs are done
 #pragma unroll 1
     for (int l = 0; l < 2; ++l) {
         publish_smem(s);
-        if (t == 0) {
+        if (t == 0 && c.ok) {
+            c.committed = c.phase;
             tc::fence_after_sync();
             const uint32_t wb = c.w + (l == 0 ? kW2 : kW3);
 #pragma unroll
@@ -279,33 +358,14 @@ __device__ __forceinline__ bool infer_tiles(InferCta& c, uint32_t x, int t, floa
                             tc::smem_desc(c.base + wb + 256 * k, 128, 1024), id, k > 0);
             tc::commit(c.bar);
         }
-        if (!wait_mma(c, s)) return false;
-        if (l == 0) hidden_epilogue<ACT, W>(c, t, c.vec + 64);
+        wait_mma(c);
+        if (l == 0) hidden_epilogue<ACT>(c, t, c.vec + 64);
     }
-    // layer 3 epilogue and the 64 -> 1 output layer on the CUDA cores
-    const uint32_t taddr = row_tmem(c, t);
-    const float* b3 = c.vec + 128;
-    const float* w4 = c.vec + 192;
-    uint64_t y2 = f2(c.vec[256], 0.0f);
-#pragma unroll
-    for (int q = 0; q < 64 / W; ++q) {
-        float z[W];
-        load_columns<W>(taddr + W * q, z);
-#pragma unroll
-        for (int j = 0; j < W; j += 4) {
-            const float4 bb = *reinterpret_cast<const float4*>(b3 + W * q + j);
-            const float4 ww = *reinterpret_cast<const float4*>(w4 + W * q + j);
-            y2 = output_pair<ACT>(f2(z[j], z[j + 1]), f2(bb.x, bb.y), f2(ww.x, ww.y), y2);
-            y2 = output_pair<ACT>(f2(z[j + 2], z[j + 3]), f2(bb.z, bb.w), f2(ww.z, ww.w), y2);
-        }
-    }
-    float y0, y1;
-    f2_split(y2, y0, y1);
-    const float y = y0 + y1;
+    const float y = IN_ORDER ? output_in_order<ACT>(c, t) : output_epilogue<ACT>(c, t);
     // every thread's TMEM reads are done before the next round's MMAs overwrite the accumulators
     tc::fence_before_sync();
     *logit = y;
-    return true;
+    return c.ok;
 }
 
 }  // namespace mlp

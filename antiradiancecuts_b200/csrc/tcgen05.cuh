@@ -101,6 +101,30 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float* v) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 16 TMEM lanes x 32 columns as MMA fragments: thread T of the warp gets, for each 8-column block i,
+// columns 2 (T % 4) and + 1 of row T / 4 in v[4 i], v[4 i + 1] and of row T / 4 + 8 in v[4 i + 2],
+// v[4 i + 3].  taddr: lane 0 or 16 of the warp's quarter.
+__device__ __forceinline__ void ld_frag32(uint32_t taddr, float* v) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Four 8 x 8 BF16 matrices in fragment layout to shared memory; lane 8 j + i gives the address of row
+// i of matrix j (16 bytes).
+__device__ __forceinline__ void stmatrix4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b),
+                 "r"(c), "r"(d)
+                 : "memory");
+}
+
 // Byte offset of element (row, k) in a K-major core-matrix layout with K bf16 columns.
 __host__ __device__ constexpr uint32_t kmajor_offset(int row, int k, int K) {
     return (uint32_t)((row >> 3) * (K >> 3) * 128 + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
