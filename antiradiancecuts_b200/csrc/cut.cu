@@ -355,8 +355,8 @@ __global__ void __launch_bounds__(32 * kSetupWarps) cut_tile_setup(TileArgs a) {
                 for (int q = 0; q < 2; ++q) {
                     float d = rn_dot(ax, ay, az, cc[q].x, cc[q].y, cc[q].z);
                     d = fminf(fmaxf(d, -1.0f), 1.0f);
-                    const float sd = rn_sqrt(fmaxf(0.0f, rn_sub(1.0f, rn_mul(d, d))));
-                    const float si = rn_sqrt(fmaxf(0.0f, rn_sub(1.0f, rn_mul(cc[q].w, cc[q].w))));
+                    const float sd = rn_sqrt_z(fmaxf(0.0f, rn_sub(1.0f, rn_mul(d, d))));
+                    const float si = rn_sqrt_z(fmaxf(0.0f, rn_sub(1.0f, rn_mul(cc[q].w, cc[q].w))));
                     const float v = cc[q].w < -d ? -1.0f : rn_sub(rn_mul(d, cc[q].w), rn_mul(sd, si));
                     res = fminf(res, v);
                 }

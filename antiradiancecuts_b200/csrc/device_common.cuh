@@ -21,6 +21,18 @@ __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, 
 __device__ __forceinline__ float rn_mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float rn_div(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ float rn_sqrt(float a) { return __fsqrt_rn(a); }
+// The same results where zeros are common: the rounded square root and division leave their fast path
+// for a call at a zero operand, so it gets a one in its place and the zero is put back.
+__device__ __forceinline__ float rn_sqrt_z(float a) {
+    const float r = __fsqrt_rn(a == 0.0f ? 1.0f : a);
+    return a == 0.0f ? a : r;
+}
+// a / b for a >= 0, b >= 0 (0 / 0 is not a number)
+__device__ __forceinline__ float rn_div_z(float a, float b) {
+    const bool zero = a == 0.0f || b == 0.0f;
+    const float r = __fdiv_rn(zero ? 1.0f : a, zero ? 1.0f : b);
+    return !zero ? r : b != 0.0f ? a : a != 0.0f ? __int_as_float(0x7f800000) : __int_as_float(0x7fffffff);
+}
 __device__ __forceinline__ float rn_dot(float ax, float ay, float az, float bx, float by, float bz) {
     return rn_add(rn_add(rn_mul(ax, bx), rn_mul(ay, by)), rn_mul(az, bz));
 }

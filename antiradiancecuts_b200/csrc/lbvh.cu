@@ -7,14 +7,17 @@
 //                       four sort passes
 //   3. radix sort       4 x 8-bit stable LSD passes, one kernel each: tiles ranked with warp
 //                       match/ballot, tile offsets by decoupled look-back with bounded waits
-//   4. lbvh_karras      Karras inner node i (bvh.cu:189-266) fused with the gather of sorted
-//                       leaf i (the reference's zip-iterator payload sort, bvh.cu:793-808)
-//   5. lbvh_bottom_up   second-arriving thread merges the two children (kernel_innerNodes +
-//                       cluster, bvh.cu:280-316, 726-744) with release/acquire ordering that
-//                       the reference lacks (no fence before its atomic)
+//   4. lbvh_topology    Karras inner node i (bvh.cu:189-266)
+//   5. lbvh_blocks      per 128 sorted leaves: the gather of the leaves (the reference's zip-iterator
+//                       payload sort, bvh.cu:793-808) and every inner node over them (kernel_innerNodes
+//                       + cluster, bvh.cu:280-316, 726-744), merged height by height in shared memory
+//   6. lbvh_climb       the other inner nodes: from each block's roots, the second-arriving thread merges
+//                       the two children, with release/acquire ordering that the reference lacks (no
+//                       fence before its atomic); lbvh_top_nodes writes their data
 //
 // Every floating-point result is computed with explicitly rounded operations in a fixed order,
 // so codes, topology, bounds, sums, representatives and cones equal the CPU build bit for bit.
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 
@@ -27,8 +30,6 @@ namespace arc {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortKPT = 8;  // keys per thread
-constexpr int kSortTile = kSortThreads * kSortKPT;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
@@ -205,6 +206,7 @@ struct SortPassArgs {
     uint32_t* err;
 };
 
+template <int kSortKPT>
 __global__ void __launch_bounds__(kSortThreads) lbvh_sort_pass(SortPassArgs s) {
     __shared__ uint32_t warp_cnt[kSortWarps][256];
     __shared__ uint32_t tile_off[256];
@@ -219,31 +221,39 @@ __global__ void __launch_bounds__(kSortThreads) lbvh_sort_pass(SortPassArgs s) {
     for (int i = tid; i < kSortWarps * 256; i += kSortThreads) (&warp_cnt[0][0])[i] = 0;
     __syncthreads();
     const int tile = tile_sh;
-    const int64_t base = (int64_t)tile * kSortTile + (int64_t)warp * 32 * kSortKPT;
+    const int64_t base = (int64_t)tile * kSortThreads * kSortKPT + (int64_t)warp * 32 * kSortKPT;
 
     uint32_t key[kSortKPT], digit[kSortKPT], rank[kSortKPT];
+    unsigned peers[kSortKPT];
     int32_t val[kSortKPT];
     const unsigned lt = (1u << lane) - 1u;
+    // (all loads before the first shared-memory update, which the compiler would not move them across)
 #pragma unroll
     for (int j = 0; j < kSortKPT; ++j) {
         const int64_t idx = base + j * 32 + lane;
-        const bool in = idx < s.n;
-        key[j] = in ? s.keys_in[idx] : 0xffffffffu;
-        val[j] = in ? s.vals_in[idx] : 0;
+        key[j] = idx < s.n ? s.keys_in[idx] : 0xffffffffu;
+        val[j] = idx < s.n ? s.vals_in[idx] : 0;
+    }
+    // lanes with the same digit, by a ballot per bit (match.any takes a step per distinct digit)
+#pragma unroll
+    for (int j = 0; j < kSortKPT; ++j) {
+        const bool in = base + j * 32 + lane < s.n;
         digit[j] = in ? ((key[j] >> s.shift) & 0xffu) : 256u;
         const unsigned active = __ballot_sync(0xffffffffu, in);
-        rank[j] = 0;
-        if (in) {
-            const unsigned peers = __match_any_sync(active, digit[j]);
-            const int leader = __ffs(peers) - 1;
-            uint32_t before = 0;
-            if (lane == leader) {
-                before = warp_cnt[warp][digit[j]];
-                warp_cnt[warp][digit[j]] = before + __popc(peers);
-            }
-            before = __shfl_sync(peers, before, leader);
-            rank[j] = before + __popc(peers & lt);
+        peers[j] = in ? active : ~active;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const unsigned m = __ballot_sync(0xffffffffu, (digit[j] >> b) & 1u);
+            peers[j] &= (digit[j] >> b) & 1u ? m : ~m;
         }
+    }
+#pragma unroll
+    for (int j = 0; j < kSortKPT; ++j) {
+        const bool in = digit[j] < 256u;
+        const uint32_t before = in ? warp_cnt[warp][digit[j]] : 0u;
+        rank[j] = before + __popc(peers[j] & lt);
+        __syncwarp();
+        if (in && lane == __ffs(peers[j]) - 1) warp_cnt[warp][digit[j]] = before + __popc(peers[j]);
         __syncwarp();
     }
     __syncthreads();
@@ -264,23 +274,34 @@ __global__ void __launch_bounds__(kSortThreads) lbvh_sort_pass(SortPassArgs s) {
             st[d] = kFlagPrefix | total;
         } else {
             st[(size_t)tile * 256 + d] = kFlagAgg | total;
+            // kWindow tiles' words are loaded at once: the walk back to the nearest known prefix is a
+            // chain of loads, and its length times their latency was most of a pass
+            constexpr int kWindow = 16;
             int t = tile - 1;
             uint32_t spins = 0;
-            while (t >= 0) {
-                const uint32_t v = st[(size_t)t * 256 + d];
-                if ((v & ~kValueMask) == 0) {
-                    if (++spins > s.spin_limit) {
-                        // publish what was summed: later tiles' offsets stay within the digit's
-                        // range, and the passes after this one do not run
-                        set_error(s.err, ARC_DEVERR_TIMEOUT);
-                        atomicMax(s.abort, (uint32_t)s.pass + 1u);
-                        break;
+            bool walking = true;
+            while (walking) {
+                uint32_t v[kWindow];
+#pragma unroll
+                for (int q = 0; q < kWindow; ++q)
+                    v[q] = t - q >= 0 ? (uint32_t)st[(size_t)(t - q) * 256 + d] : (uint32_t)kFlagPrefix;  // before the first tile: 0
+                int used = 0;
+#pragma unroll
+                for (int q = 0; q < kWindow; ++q) {
+                    if (walking && used == q && (v[q] & ~kValueMask) != 0) {
+                        excl += v[q] & kValueMask;
+                        used = q + 1;
+                        if (v[q] & kFlagPrefix) walking = false;
                     }
-                    continue;
                 }
-                excl += v & kValueMask;
-                if (v & kFlagPrefix) break;
-                --t;
+                t -= used;
+                if (walking && used < kWindow && ++spins > s.spin_limit) {
+                    // publish what was summed: later tiles' offsets stay within the digit's
+                    // range, and the passes after this one do not run
+                    set_error(s.err, ARC_DEVERR_TIMEOUT);
+                    atomicMax(s.abort, (uint32_t)s.pass + 1u);
+                    break;
+                }
             }
             __threadfence();
             st[(size_t)tile * 256 + d] = kFlagPrefix | (excl + total);
@@ -306,115 +327,48 @@ __device__ __forceinline__ int kdelta(const uint32_t* __restrict__ m, int num_no
     return d;
 }
 
-struct KarrasArgs {
+struct TopologyArgs {
     const uint32_t* morton;
-    const int32_t* sorted_index;
-    ArcAvplsGpuParam a;
-    const MaterialRecord* mats;
-    int32_t num_mats;
     int32_t n;
-    uint32_t seed;
     int32_t* left;
     int32_t* right;
     int32_t* parents;
     int32_t* range;
-    float4* records;   // [2N-1][4]
-    float4* cones;     // [2N-1][2] {normal axis, cos}, {direction axis, cos}
-    float4* dirstat;   // [2N-1] {S.xyz, a}: a = sum of antiradiance luminances, S = sum of a_i w_i / |w_i|
-    float4* bbox;      // [2N-1][2] scratch: {min, 0}, {max, 0} of leaf boxes then inner boxes
-    ArcAvplBvhNodeDataParam nd;
-    ArcFloat3* sorted_pos;
-    ArcFloat3* sorted_nrm;
     const uint32_t* abort;  // set when the sort gave up: its order is not a permutation
-    uint32_t* err;
 };
 
-__global__ void __launch_bounds__(256) lbvh_karras(KarrasArgs k) {
+__global__ void __launch_bounds__(256) lbvh_topology(TopologyArgs k) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = k.n, num_nodes = n - 1;
-    if (i >= n || *k.abort != 0u) return;
-    // ---- inner node i ----
-    if (i < num_nodes) {
-        const uint32_t* m = k.morton;
-        const int d = (kdelta(m, num_nodes, i, i + 1) - kdelta(m, num_nodes, i, i - 1)) < 0 ? -1 : 1;
-        const int delta_min = kdelta(m, num_nodes, i, i - d);
-        int64_t l_max = 128;
-        while (kdelta(m, num_nodes, i, i + l_max * d) > delta_min) l_max *= 4;
-        int64_t l = 0;
-        for (int64_t t = l_max / 2; t > 0; t /= 2)
-            if (kdelta(m, num_nodes, i, i + (l + t) * d) > delta_min) l += t;
-        const int64_t j = i + l * d;
-        const int delta_node = kdelta(m, num_nodes, i, j);
-        int64_t s = 0, kk = 2, t = (l + kk - 1) / kk;
-        while (true) {
-            if (kdelta(m, num_nodes, i, i + (s + t) * d) > delta_node) s += t;
-            if (t <= 1) break;
-            kk *= 2;
-            t = (l + kk - 1) / kk;
-        }
-        const int split = (int)(i + s * d + min(d, 0));
-        const int lo = (int)min((int64_t)i, j), hi = (int)max((int64_t)i, j);
-        const int lc = lo == split ? split : -(split + 1);
-        const int rc = hi == split + 1 ? split + 1 : -(split + 2);
-        k.left[i] = lc;
-        k.right[i] = rc;
-        k.range[2 * i] = lo;
-        k.range[2 * i + 1] = hi;
-        k.parents[lc >= 0 ? lc : n - (lc + 1)] = i;
-        k.parents[rc >= 0 ? rc : n - (rc + 1)] = i;
-        if (i == 0) k.parents[n] = -1;
+    if (i >= num_nodes || *k.abort != 0u) return;
+    const uint32_t* m = k.morton;
+    const int d = (kdelta(m, num_nodes, i, i + 1) - kdelta(m, num_nodes, i, i - 1)) < 0 ? -1 : 1;
+    const int delta_min = kdelta(m, num_nodes, i, i - d);
+    int64_t l_max = 128;
+    while (kdelta(m, num_nodes, i, i + l_max * d) > delta_min) l_max *= 4;
+    int64_t l = 0;
+    for (int64_t t = l_max / 2; t > 0; t /= 2)
+        if (kdelta(m, num_nodes, i, i + (l + t) * d) > delta_min) l += t;
+    const int64_t j = i + l * d;
+    const int delta_node = kdelta(m, num_nodes, i, j);
+    int64_t s = 0, kk = 2, t = (l + kk - 1) / kk;
+    while (true) {
+        if (kdelta(m, num_nodes, i, i + (s + t) * d) > delta_node) s += t;
+        if (t <= 1) break;
+        kk *= 2;
+        t = (l + kk - 1) / kk;
     }
-    // ---- sorted leaf i ----
-    const int src = k.sorted_index[i];
-    const float3 p = ld3(k.a.position, src), nr = ld3(k.a.normal, src), w = ld3(k.a.incDirection, src);
-    const float3 L = ld3(k.a.incRadiance, src), A = ld3(k.a.antiradiance, src);
-    int mat = k.a.materialIndex[src];
-    if (mat < 0 || mat >= k.num_mats) {
-        set_error(k.err, ARC_DEVERR_BAD_MATERIAL);
-        mat = 0;
-    }
-    const float4 dif = k.mats[mat].diffuse_exp;
-    const bool light = (w.x == 0.0f && w.y == 0.0f && w.z == 0.0f);
-    float4* r = k.records + 4 * (size_t)i;
-    r[0] = make_float4(p.x, p.y, p.z, nr.x);
-    r[1] = make_float4(nr.y, nr.z, w.x, w.y);
-    r[2] = make_float4(w.z, light ? L.x : rn_mul(L.x, rn_mul(kOneOverPi, dif.x)),
-                       light ? L.y : rn_mul(L.y, rn_mul(kOneOverPi, dif.y)),
-                       light ? L.z : rn_mul(L.z, rn_mul(kOneOverPi, dif.z)));
-    r[3] = make_float4(A.x, A.y, A.z, 1.0f);
-    // leaf cones: (n, 1) and (w/|w|, 1), or the whole sphere when w = 0
-    float4* c = k.cones + 2 * (size_t)i;
-    c[0] = make_float4(nr.x, nr.y, nr.z, 1.0f);
-    const float ww = rn_dot(w.x, w.y, w.z, w.x, w.y, w.z);
-    const float a_lum = rn_add(rn_add(rn_mul(0.2126f, A.x), rn_mul(0.7152f, A.y)), rn_mul(0.0722f, A.z));
-    if (ww > 0.0f) {
-        const float inv = rn_div(1.0f, rn_sqrt(ww));
-        c[1] = make_float4(rn_mul(w.x, inv), rn_mul(w.y, inv), rn_mul(w.z, inv), 1.0f);
-        k.dirstat[i] = make_float4(rn_mul(a_lum, c[1].x), rn_mul(a_lum, c[1].y), rn_mul(a_lum, c[1].z), a_lum);
-    } else {
-        c[1] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-        k.dirstat[i] = make_float4(0.0f, 0.0f, 0.0f, a_lum);
-    }
-    k.bbox[2 * (size_t)i] = make_float4(p.x, p.y, p.z, 0.0f);
-    k.bbox[2 * (size_t)i + 1] = make_float4(p.x, p.y, p.z, 0.0f);
-    // reference node-data layout (AvplBvhNodeData, bvh.cu:673-724, sorted as bvh.cu:793-808)
-    k.nd.size[i] = 1;
-    k.nd.materialIndex[i] = mat;
-    k.nd.randomNumbers[i] = arc_node_random(k.seed, (uint32_t)i);
-    reinterpret_cast<float*>(k.nd.position)[3 * i + 0] = p.x;
-    reinterpret_cast<float*>(k.nd.position)[3 * i + 1] = p.y;
-    reinterpret_cast<float*>(k.nd.position)[3 * i + 2] = p.z;
-    reinterpret_cast<float*>(k.nd.normal)[3 * i + 0] = nr.x;
-    reinterpret_cast<float*>(k.nd.normal)[3 * i + 1] = nr.y;
-    reinterpret_cast<float*>(k.nd.normal)[3 * i + 2] = nr.z;
-    reinterpret_cast<float*>(k.nd.incRadiance)[3 * i + 0] = L.x;
-    reinterpret_cast<float*>(k.nd.incRadiance)[3 * i + 1] = L.y;
-    reinterpret_cast<float*>(k.nd.incRadiance)[3 * i + 2] = L.z;
-    reinterpret_cast<float*>(k.nd.incDirection)[3 * i + 0] = w.x;
-    reinterpret_cast<float*>(k.nd.incDirection)[3 * i + 1] = w.y;
-    reinterpret_cast<float*>(k.nd.incDirection)[3 * i + 2] = w.z;
-    k.sorted_pos[i] = ArcFloat3{p.x, p.y, p.z};
-    k.sorted_nrm[i] = ArcFloat3{nr.x, nr.y, nr.z};
+    const int split = (int)(i + s * d + min(d, 0));
+    const int lo = (int)min((int64_t)i, j), hi = (int)max((int64_t)i, j);
+    const int lc = lo == split ? split : -(split + 1);
+    const int rc = hi == split + 1 ? split + 1 : -(split + 2);
+    k.left[i] = lc;
+    k.right[i] = rc;
+    k.range[2 * i] = lo;
+    k.range[2 * i + 1] = hi;
+    k.parents[lc >= 0 ? lc : n - (lc + 1)] = i;
+    k.parents[rc >= 0 ? rc : n - (rc + 1)] = i;
+    if (i == 0) k.parents[n] = -1;
 }
 
 // union of two cones; same operation order as the CPU build's cone_union
@@ -431,153 +385,495 @@ __device__ __forceinline__ float4 cone_union(float4 c1, float4 c2) {
     for (int q = 0; q < 2; ++q) {
         float d = rn_dot(ax, ay, az, ci[q].x, ci[q].y, ci[q].z);
         d = fminf(fmaxf(d, -1.0f), 1.0f);
-        const float sd = rn_sqrt(fmaxf(0.0f, rn_sub(1.0f, rn_mul(d, d))));
-        const float si = rn_sqrt(fmaxf(0.0f, rn_sub(1.0f, rn_mul(ci[q].w, ci[q].w))));
+        const float sd = rn_sqrt_z(fmaxf(0.0f, rn_sub(1.0f, rn_mul(d, d))));
+        const float si = rn_sqrt_z(fmaxf(0.0f, rn_sub(1.0f, rn_mul(ci[q].w, ci[q].w))));
         const float v = ci[q].w < -d ? -1.0f : rn_sub(rn_mul(d, ci[q].w), rn_mul(sd, si));
         res = fminf(res, v);
     }
     return make_float4(ax, ay, az, res);
 }
 
-struct BottomUpArgs {
-    const uint32_t* abort;  // set when the sort gave up
+// What a merge needs of a node, and what the node's outputs are made of.  Representatives are kept as
+// leaves, so that a merge moves two indices instead of their positions, normals and directions.
+struct NodeState {
+    float bb[6];          // box
+    float L[3];           // summed radiance
+    float Lp[3], A[3];    // the packed record's sums
+    float4 dir;           // direction statistics {S, a}
+    float4 cn, cw;        // normal and direction cones
+    int size, rep, arep;  // leaves below; radiance and antiradiance representative (sorted leaf)
+};
+constexpr int kStateWords = 30;
+
+// Merges two children into inner node t (record index); same operations and order as the CPU build's
+// bottom-up pass.  In three independent parts, which lbvh_blocks gives to three threads: everything but
+// the cones, and the two cones.
+__device__ __forceinline__ void merge_sums(NodeState& o, const NodeState& l, const NodeState& r, uint32_t seed, int t,
+                                           float* rnd_out) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        o.bb[q] = fminf(l.bb[q], r.bb[q]);
+        o.bb[3 + q] = fmaxf(l.bb[3 + q], r.bb[3 + q]);
+        o.L[q] = rn_add(l.L[q], r.L[q]);
+        o.Lp[q] = rn_add(l.Lp[q], r.Lp[q]);
+        o.A[q] = rn_add(l.A[q], r.A[q]);
+    }
+    // representative (cluster, bvh.cu:726-744)
+    const float i1 = rn_sqrt_z(rn_dot(l.L[0], l.L[1], l.L[2], l.L[0], l.L[1], l.L[2]));
+    const float i2 = rn_sqrt_z(rn_dot(r.L[0], r.L[1], r.L[2], r.L[0], r.L[1], r.L[2]));
+    const float rnd = arc_node_random(seed, (uint32_t)t);
+    const bool right = rnd > rn_div_z(i1, rn_add(i1, i2));
+    o.rep = right ? r.rep : l.rep;
+    o.size = l.size + r.size;
+    // direction statistics, and the antiradiance representative: drawn in proportion to
+    // antiradiance luminance with the same random number; its direction is the record's w
+    o.dir = make_float4(rn_add(l.dir.x, r.dir.x), rn_add(l.dir.y, r.dir.y), rn_add(l.dir.z, r.dir.z),
+                        rn_add(l.dir.w, r.dir.w));
+    const bool aright = o.dir.w > 0.0f ? rnd > rn_div_z(l.dir.w, o.dir.w) : right;
+    o.arep = aright ? r.arep : l.arep;
+    *rnd_out = rnd;
+}
+
+struct BlockArgs {
+    const uint32_t* abort;  // set when the sort gave up: its order is not a permutation
     uint32_t* err;
+    const int32_t* sorted_index;
+    ArcAvplsGpuParam a;
+    const MaterialRecord* mats;
+    int32_t num_mats;
     int32_t n;
     uint32_t seed;
     const int32_t* left;
     const int32_t* right;
     const int32_t* parents;
     const int32_t* range;  // [N-1][2]: first and last leaf of each inner node
-    int32_t* visit;
-    float4* records;
-    float4* cones;
-    float4* dirstat;
-    float4* bbox;
-    float4* bounds;  // [N-1][4]
+    float4* records;       // [2N-1][4]
+    float4* dirstat;       // [2N-1] {S.xyz, a}: a = sum of antiradiance luminances, S = sum of a_i w_i / |w_i|
+    float4* bounds;        // [N-1][4]
     ArcAvplBvhNodeDataParam nd;
+    ArcFloat3* sorted_pos;
+    ArcFloat3* sorted_nrm;
+    // the nodes that reach over a block's leaves, and the nodes below them
+    float4* state;         // [2N-1][8]: NodeState of a block's roots and of the nodes above them
+    int32_t* visit;        // [N-1] arrivals
+    int32_t* roots;        // record indices of every block's roots
+    int32_t* top;          // inner nodes above them
+    int32_t* counts;       // roots, top nodes
 };
 
-// Loads of a child's data in the merge.  A child merged by a thread of the same block (LOCAL) was
-// published with a block-scope release, so the load goes through the SM's L1; a child merged in
-// another block was published with a device-scope release and is read from L2.
-template <bool LOCAL, typename T>
-__device__ __forceinline__ T ld_child(const T* p) {
-    if (LOCAL) return *p;
-    return __ldcg(p);
+__device__ __forceinline__ void store3(ArcFloat3* p, int64_t i, float x, float y, float z) {
+    float* f = reinterpret_cast<float*>(p) + 3 * i;
+    f[0] = x;
+    f[1] = y;
+    f[2] = z;
 }
 
-// Merges the two children of inner node k (the second thread to arrive does it); same operations
-// and order as the CPU build's bottom-up pass.
-template <bool LOCAL>
-__device__ __forceinline__ void merge_node(const BottomUpArgs& b, int k, int lc, int rc) {
-    const int n = b.n;
-    const int t = n + k;
-    const int l = lc >= 0 ? lc : n - (lc + 1);
-    const int r = rc >= 0 ? rc : n - (rc + 1);
-    // bounding box
-    const float4 lmin = ld_child<LOCAL>(b.bbox + 2 * (size_t)l), lmax = ld_child<LOCAL>(b.bbox + 2 * (size_t)l + 1);
-    const float4 rmin = ld_child<LOCAL>(b.bbox + 2 * (size_t)r), rmax = ld_child<LOCAL>(b.bbox + 2 * (size_t)r + 1);
-    const float bt[6] = {fminf(lmin.x, rmin.x), fminf(lmin.y, rmin.y), fminf(lmin.z, rmin.z),
-                         fmaxf(lmax.x, rmax.x), fmaxf(lmax.y, rmax.y), fmaxf(lmax.z, rmax.z)};
-    b.bbox[2 * (size_t)t] = make_float4(bt[0], bt[1], bt[2], 0.0f);
-    b.bbox[2 * (size_t)t + 1] = make_float4(bt[3], bt[4], bt[5], 0.0f);
-    // representative (cluster, bvh.cu:726-744)
-    const float* Lf = reinterpret_cast<const float*>(b.nd.incRadiance);
-    const float Ll[3] = {ld_child<LOCAL>(Lf + 3 * l), ld_child<LOCAL>(Lf + 3 * l + 1), ld_child<LOCAL>(Lf + 3 * l + 2)};
-    const float Lr[3] = {ld_child<LOCAL>(Lf + 3 * r), ld_child<LOCAL>(Lf + 3 * r + 1), ld_child<LOCAL>(Lf + 3 * r + 2)};
-    const float i1 = rn_sqrt(rn_dot(Ll[0], Ll[1], Ll[2], Ll[0], Ll[1], Ll[2]));
-    const float i2 = rn_sqrt(rn_dot(Lr[0], Lr[1], Lr[2], Lr[0], Lr[1], Lr[2]));
-    const float rnd = arc_node_random(b.seed, (uint32_t)t);
-    const int repr = rnd > rn_div(i1, rn_add(i1, i2)) ? r : l;
-    const int sl = ld_child<LOCAL>(b.nd.size + l), sr = ld_child<LOCAL>(b.nd.size + r);
+__device__ __forceinline__ void store_state(float4* state, int node, const NodeState& s) {
+    float4* d = state + 8 * (size_t)node;
+    d[0] = make_float4(s.bb[0], s.bb[1], s.bb[2], s.bb[3]);
+    d[1] = make_float4(s.bb[4], s.bb[5], s.L[0], s.L[1]);
+    d[2] = make_float4(s.L[2], s.Lp[0], s.Lp[1], s.Lp[2]);
+    d[3] = make_float4(s.A[0], s.A[1], s.A[2], __int_as_float(s.size));
+    d[4] = s.dir;
+    d[5] = s.cn;
+    d[6] = s.cw;
+    d[7] = make_float4(__int_as_float(s.rep), __int_as_float(s.arep), 0.0f, 0.0f);
+}
+
+// (states are written and read by different blocks of one launch: through L2)
+__device__ __forceinline__ NodeState load_state(const float4* state, int node) {
+    const float4* p = state + 8 * (size_t)node;
+    const float4 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(p + 2), d = __ldcg(p + 3), h = __ldcg(p + 7);
+    NodeState s;
+    s.bb[0] = a.x; s.bb[1] = a.y; s.bb[2] = a.z; s.bb[3] = a.w;
+    s.bb[4] = b.x; s.bb[5] = b.y;
+    s.L[0] = b.z; s.L[1] = b.w; s.L[2] = c.x;
+    s.Lp[0] = c.y; s.Lp[1] = c.z; s.Lp[2] = c.w;
+    s.A[0] = d.x; s.A[1] = d.y; s.A[2] = d.z;
+    s.size = __float_as_int(d.w);
+    s.dir = __ldcg(p + 4);
+    s.cn = __ldcg(p + 5);
+    s.cw = __ldcg(p + 6);
+    s.rep = __float_as_int(h.x);
+    s.arep = __float_as_int(h.y);
+    return s;
+}
+
+// Inner node k's outputs: record (representative p / n, antiradiance representative's w, summed L' and A,
+// count), direction statistics, bounds and the reference's node data.
+__device__ __forceinline__ void write_node(const BlockArgs& b, int k, int lc, int rc, const NodeState& s, float rnd,
+                                           float3 p, float3 nr, float3 w, float3 aw, int mat) {
+    const int64_t t = (int64_t)b.n + k;
+    float4* rec = b.records + 4 * t;
+    rec[0] = make_float4(p.x, p.y, p.z, nr.x);
+    rec[1] = make_float4(nr.y, nr.z, aw.x, aw.y);
+    rec[2] = make_float4(aw.z, s.Lp[0], s.Lp[1], s.Lp[2]);
+    rec[3] = make_float4(s.A[0], s.A[1], s.A[2], (float)s.size);
+    b.dirstat[t] = s.dir;
+    float4* bd = b.bounds + 4 * (size_t)k;
+    bd[0] = make_float4(s.bb[0], s.bb[1], s.bb[2], __int_as_float(lc));
+    bd[1] = make_float4(s.bb[3], s.bb[4], s.bb[5], __int_as_float(rc));
+    bd[2] = s.cn;
+    bd[3] = s.cw;
     b.nd.randomNumbers[t] = rnd;
-    b.nd.size[t] = sl + sr;
-    b.nd.materialIndex[t] = ld_child<LOCAL>(b.nd.materialIndex + repr);
-    float* Lt = reinterpret_cast<float*>(b.nd.incRadiance);
-    float* P = reinterpret_cast<float*>(b.nd.position);
-    float* N = reinterpret_cast<float*>(b.nd.normal);
-    float* W = reinterpret_cast<float*>(b.nd.incDirection);
+    b.nd.size[t] = s.size;
+    b.nd.materialIndex[t] = mat;
+    store3(b.nd.incRadiance, t, s.L[0], s.L[1], s.L[2]);
+    store3(b.nd.position, t, p.x, p.y, p.z);
+    store3(b.nd.normal, t, nr.x, nr.y, nr.z);
+    store3(b.nd.incDirection, t, w.x, w.y, w.z);
+}
+
+constexpr int kBlockLeaves = 128;
+constexpr int kMaxHeight = 63;  // a radix tree of 32-bit codes over 2^29 leaves has at most 61 levels
+constexpr int kWRow = kStateWords;  // three more rows (leaves only): w as given
+constexpr int kBlockSmem = (kStateWords * 2 + 3) * kBlockLeaves * 4;
+
+// Bound by the latency of its phases and by the L1 / L2 accesses of 41 sectors per leaf (54% of L1, 604 MB of
+// DRAM traffic): 1,000,003 leaves take 262 us, where one thread per leaf climbing through global memory took
+// 600 us.  128 leaves per block leave five blocks per SM to overlap (256 leaves, three blocks: 396 us).
+// One block per 128 sorted leaves; thread j owns leaf base + j and inner node base + j.  An inner node is
+// one end of its own leaf range, so the nodes whose range lies inside the block are among those 128.
+// They are merged by height (the longest path down), all nodes of a height in consecutive threads:
+// climbing from the leaves instead keeps one or two lanes of every warp busy for the whole height.
+__global__ void __launch_bounds__(kBlockLeaves) lbvh_blocks(BlockArgs b) {
+    extern __shared__ float st[];  // [word][local node]: leaf j at j, inner node base + j at 128 + j
+    __shared__ int s_mat[kBlockLeaves], s_src[kBlockLeaves];
+    __shared__ int s_up[2 * kBlockLeaves];  // local parent (0 .. 127) or -1
+    __shared__ short2 s_child[kBlockLeaves], s_rep[kBlockLeaves];
+    __shared__ int2 s_link[kBlockLeaves];
+    __shared__ int s_arrived[kBlockLeaves], s_height[kBlockLeaves];
+    __shared__ int s_first[kMaxHeight + 2], s_list[kBlockLeaves];
+    __shared__ float s_rnd[kBlockLeaves];
+    __shared__ int s_count[2], s_base[2];
+    if (*b.abort != 0u) return;  // uniform over the CTA: before any barrier
+    const int j = threadIdx.x, base = blockIdx.x * kBlockLeaves, i = base + j, n = b.n;
+    constexpr int kN = 2 * kBlockLeaves;
+    auto put_sums = [&](int id, const NodeState& s) {
+        float* d = st + id;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) d[q * kN] = s.bb[q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            d[(6 + q) * kN] = s.L[q];
+            d[(9 + q) * kN] = s.Lp[q];
+            d[(12 + q) * kN] = s.A[q];
+        }
+        d[15 * kN] = s.dir.x; d[16 * kN] = s.dir.y; d[17 * kN] = s.dir.z; d[18 * kN] = s.dir.w;
+        d[27 * kN] = __int_as_float(s.size);
+        d[28 * kN] = __int_as_float(s.rep);
+        d[29 * kN] = __int_as_float(s.arep);
+    };
+    auto get_sums = [&](int id, NodeState& s) {
+        const float* d = st + id;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) s.bb[q] = d[q * kN];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            s.L[q] = d[(6 + q) * kN];
+            s.Lp[q] = d[(9 + q) * kN];
+            s.A[q] = d[(12 + q) * kN];
+        }
+        s.dir = make_float4(d[15 * kN], d[16 * kN], d[17 * kN], d[18 * kN]);
+        s.size = __float_as_int(d[27 * kN]);
+        s.rep = __float_as_int(d[28 * kN]);
+        s.arep = __float_as_int(d[29 * kN]);
+    };
+    // which: 0 the normal cone, 1 the direction cone
+    auto put_cone = [&](int id, int which, float4 c) {
+        float* d = st + (19 + 4 * which) * kN + id;
+        d[0] = c.x; d[kN] = c.y; d[2 * kN] = c.z; d[3 * kN] = c.w;
+    };
+    auto get_cone = [&](int id, int which) {
+        const float* d = st + (19 + 4 * which) * kN + id;
+        return make_float4(d[0], d[kN], d[2 * kN], d[3 * kN]);
+    };
+    auto get = [&](int id) {
+        NodeState s;
+        get_sums(id, s);
+        s.cn = get_cone(id, 0);
+        s.cw = get_cone(id, 1);
+        return s;
+    };
+    // ---- topology of the block ----
+    int lc = 0, rc = 0;
+    bool local = false;
+    if (i < n - 1) {
+        const int2 rg = *reinterpret_cast<const int2*>(b.range + 2 * (size_t)i);
+        lc = b.left[i];
+        rc = b.right[i];
+        local = rg.x >= base && rg.y < base + kBlockLeaves;
+    }
+    s_up[j] = s_up[kBlockLeaves + j] = -1;
+    s_arrived[j] = s_height[j] = 0;
+    static_assert(kBlockLeaves >= kMaxHeight + 2, "one thread per entry of s_first");
+    if (j < kMaxHeight + 2) s_first[j] = 0;
+    if (j < 2) s_count[j] = 0;
+    __syncthreads();
+    auto local_id = [&](int c) { return c >= 0 ? c - base : kBlockLeaves - (c + 1) - base; };
+    if (local) {
+        s_up[local_id(lc)] = j;
+        s_up[local_id(rc)] = j;
+        s_child[j] = make_short2((short)local_id(lc), (short)local_id(rc));
+    }
+    // ---- sorted leaf i ----
+    // The three components of a vector are loaded by neighbouring lanes, so that each random access costs
+    // the sectors it touches once, not once per component.
+    s_src[j] = i < n ? b.sorted_index[i] : -1;
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        Lt[3 * t + q] = rn_add(Ll[q], Lr[q]);
-        P[3 * t + q] = ld_child<LOCAL>(P + 3 * repr + q);
-        N[3 * t + q] = ld_child<LOCAL>(N + 3 * repr + q);
-        W[3 * t + q] = ld_child<LOCAL>(W + 3 * repr + q);
+        const int e = j + q * kBlockLeaves, m = e / 3, c = e - 3 * m, src = s_src[m];
+        if (src >= 0) {
+            auto f = [&](const ArcFloat3* v) { return reinterpret_cast<const float*>(v)[3 * (int64_t)src + c]; };
+            const float p = f(b.a.position), nr = f(b.a.normal), w = f(b.a.incDirection), L = f(b.a.incRadiance),
+                        A = f(b.a.antiradiance);
+            st[c * kN + m] = p;
+            st[(3 + c) * kN + m] = p;
+            st[(19 + c) * kN + m] = nr;
+            st[kWRow * kN + c * kBlockLeaves + m] = w;
+            st[(6 + c) * kN + m] = L;
+            st[(12 + c) * kN + m] = A;
+        }
     }
-    // direction statistics, and the antiradiance representative: drawn in proportion to
-    // antiradiance luminance with the same random number; its direction is the record's w
-    const float4 dl = ld_child<LOCAL>(b.dirstat + l), dr = ld_child<LOCAL>(b.dirstat + r);
-    const float4 dt = make_float4(rn_add(dl.x, dr.x), rn_add(dl.y, dr.y), rn_add(dl.z, dr.z), rn_add(dl.w, dr.w));
-    b.dirstat[t] = dt;
-    const int arep = dt.w > 0.0f ? (rnd > rn_div(dl.w, dt.w) ? r : l) : repr;
-    // packed record: representative p/n, antiradiance representative's w, summed L' and A, count
-    const float* R = reinterpret_cast<const float*>(b.records);
-    float rt[16];
+    __syncthreads();
+    if (i < n) {
+        int mat = b.a.materialIndex[s_src[j]];
+        if (mat < 0 || mat >= b.num_mats) {
+            set_error(b.err, ARC_DEVERR_BAD_MATERIAL);
+            mat = 0;
+        }
+        auto vec = [&](int r) { return f3(st[r * kN + j], st[(r + 1) * kN + j], st[(r + 2) * kN + j]); };
+        const float3 p = vec(0), nr = vec(19), L = vec(6), A = vec(12);
+        const float3 w = f3(st[kWRow * kN + j], st[kWRow * kN + kBlockLeaves + j], st[kWRow * kN + 2 * kBlockLeaves + j]);
+        const float4 dif = b.mats[mat].diffuse_exp;
+        const bool light = (w.x == 0.0f && w.y == 0.0f && w.z == 0.0f);
+        NodeState s;
+        s.bb[0] = s.bb[3] = p.x;
+        s.bb[1] = s.bb[4] = p.y;
+        s.bb[2] = s.bb[5] = p.z;
+        s.L[0] = L.x; s.L[1] = L.y; s.L[2] = L.z;
+        s.Lp[0] = light ? L.x : rn_mul(L.x, rn_mul(kOneOverPi, dif.x));
+        s.Lp[1] = light ? L.y : rn_mul(L.y, rn_mul(kOneOverPi, dif.y));
+        s.Lp[2] = light ? L.z : rn_mul(L.z, rn_mul(kOneOverPi, dif.z));
+        s.A[0] = A.x; s.A[1] = A.y; s.A[2] = A.z;
+        // leaf cones: (n, 1) and (w/|w|, 1), or the whole sphere when w = 0
+        s.cn = make_float4(nr.x, nr.y, nr.z, 1.0f);
+        const float ww = rn_dot(w.x, w.y, w.z, w.x, w.y, w.z);
+        const float a_lum = rn_add(rn_add(rn_mul(0.2126f, A.x), rn_mul(0.7152f, A.y)), rn_mul(0.0722f, A.z));
+        if (ww > 0.0f) {
+            const float inv = rn_div(1.0f, rn_sqrt(ww));
+            s.cw = make_float4(rn_mul(w.x, inv), rn_mul(w.y, inv), rn_mul(w.z, inv), 1.0f);
+            s.dir = make_float4(rn_mul(a_lum, s.cw.x), rn_mul(a_lum, s.cw.y), rn_mul(a_lum, s.cw.z), a_lum);
+        } else {
+            s.cw = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+            s.dir = make_float4(0.0f, 0.0f, 0.0f, a_lum);
+        }
+        s.size = 1;
+        s.rep = s.arep = i;
+        put_sums(j, s);
+        put_cone(j, 0, s.cn);
+        put_cone(j, 1, s.cw);
+        s_mat[j] = mat;
+        b.dirstat[i] = s.dir;
+        b.nd.size[i] = 1;
+        b.nd.materialIndex[i] = mat;
+        b.nd.randomNumbers[i] = arc_node_random(b.seed, (uint32_t)i);
+    }
+    __syncthreads();
+    // ---- heights: the second arrival at a node carries its height up ----
+    if (i < n) {
+        int h = 0;
+        for (int u = s_up[j]; u >= 0; u = s_up[kBlockLeaves + u]) {
+            atomicMax(&s_height[u], h + 1);
+            __threadfence_block();
+            if (atomicAdd(&s_arrived[u], 1) == 0) break;
+            __threadfence_block();
+            h = *reinterpret_cast<volatile int*>(&s_height[u]);
+        }
+    }
+    __syncthreads();
+    const int height = local ? min(s_height[j], kMaxHeight) : 0;
+    int rank = 0;
+    if (local) rank = atomicAdd(&s_first[height + 1], 1);
+    __syncthreads();
+    if (j < 32) {  // s_first[h]: nodes of height < h, h = 1 .. 64 (two per lane)
+        static_assert(kMaxHeight + 1 == 64, "two entries per lane");
+        const int x = s_first[1 + 2 * j], y = s_first[2 + 2 * j];
+        int incl = x + y;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) rt[q] = ld_child<LOCAL>(R + 16 * (size_t)repr + q);
-#pragma unroll
-    for (int q = 6; q < 9; ++q) rt[q] = ld_child<LOCAL>(R + 16 * (size_t)arep + q);
-#pragma unroll
-    for (int q = 9; q < 15; ++q)
-        rt[q] = rn_add(ld_child<LOCAL>(R + 16 * (size_t)l + q), ld_child<LOCAL>(R + 16 * (size_t)r + q));
-    rt[15] = (float)(sl + sr);
-    float4* rec = b.records + 4 * (size_t)t;
-    rec[0] = make_float4(rt[0], rt[1], rt[2], rt[3]);
-    rec[1] = make_float4(rt[4], rt[5], rt[6], rt[7]);
-    rec[2] = make_float4(rt[8], rt[9], rt[10], rt[11]);
-    rec[3] = make_float4(rt[12], rt[13], rt[14], rt[15]);
-    // cones
-    const float4 cnl = ld_child<LOCAL>(b.cones + 2 * (size_t)l), cnr = ld_child<LOCAL>(b.cones + 2 * (size_t)r);
-    const float4 cwl = ld_child<LOCAL>(b.cones + 2 * (size_t)l + 1), cwr = ld_child<LOCAL>(b.cones + 2 * (size_t)r + 1);
-    const float4 cn = cone_union(cnl, cnr), cw = cone_union(cwl, cwr);
-    b.cones[2 * (size_t)t] = cn;
-    b.cones[2 * (size_t)t + 1] = cw;
-    float4* bd = b.bounds + 4 * (size_t)k;
-    bd[0] = make_float4(bt[0], bt[1], bt[2], __int_as_float(lc));
-    bd[1] = make_float4(bt[3], bt[4], bt[5], __int_as_float(rc));
-    bd[2] = cn;
-    bd[3] = cw;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (j >= o) incl += v;
+        }
+        s_first[1 + 2 * j] = incl - y;
+        s_first[2 + 2 * j] = incl;
+    }
+    __syncthreads();
+    if (local) s_list[s_first[height] + rank] = j;
+    __syncthreads();
+    const int total = s_first[kMaxHeight + 1];
+    // ---- merges, height by height ----
+    for (int h = 1; s_first[h] < total; ++h) {
+        const int first = s_first[h], count = s_first[h + 1] - first;
+        // three threads per node: the sums, the normal cone, the direction cone
+        for (int q = j; q < 3 * count; q += kBlockLeaves) {
+            const int part = q >= 2 * count ? 2 : q >= count ? 1 : 0;
+            const int k = s_list[first + q - part * count];
+            const short2 c = s_child[k];
+            if (part == 0) {
+                NodeState l, r, o;
+                get_sums(c.x, l);
+                get_sums(c.y, r);
+                merge_sums(o, l, r, b.seed, n + base + k, &s_rnd[k]);
+                put_sums(kBlockLeaves + k, o);
+            } else {
+                put_cone(kBlockLeaves + k, part - 1, cone_union(get_cone(c.x, part - 1), get_cone(c.y, part - 1)));
+            }
+        }
+        __syncthreads();
+    }
+    // ---- outputs, consecutive threads to consecutive words ----
+    // (32-byte sectors half written by each store of a thread's own record cost 50 sector accesses per
+    // leaf instead of 20.)  The slots of inner nodes that reach over the block are written too, with
+    // values that lbvh_top_nodes replaces.
+    const int leaves = min(kBlockLeaves, n - base), nodes = min(kBlockLeaves, n - 1 - base);
+    const bool has_node = i < n - 1;
+    NodeState s;
+    if (local) s = get(kBlockLeaves + j);
+    const int rl = local ? s.rep - base : 0, al = local ? s.arep - base : 0;  // both lie in the node's range
+    s_rep[j] = make_short2((short)rl, (short)al);
+    if (has_node) {
+        const int64_t t = (int64_t)n + i;
+        b.dirstat[t] = local ? s.dir : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        b.nd.size[t] = local ? s.size : 0;
+        b.nd.randomNumbers[t] = local ? s_rnd[j] : 0.0f;
+        b.nd.materialIndex[t] = s_mat[rl];
+    }
+    s_link[j] = make_int2(lc, rc);
+    __syncthreads();
+    {
+        // 16-byte quarter of a record or bounds entry that this thread writes (the same for each pass)
+        const int quarter = j & 3;
+        auto w_at = [&](int c, int leaf) { return st[kWRow * kN + c * kBlockLeaves + leaf]; };
+        auto row = [&](int r, int id) { return st[r * kN + id]; };
+        for (int e = j; e < 4 * kBlockLeaves; e += kBlockLeaves) {
+            const int m = e >> 2, own = kBlockLeaves + m;
+            const int r = s_rep[m].x, ar = s_rep[m].y;
+            float4 lf, nf, bf;
+            if (quarter == 0) {
+                lf = make_float4(row(0, m), row(1, m), row(2, m), row(19, m));
+                nf = make_float4(row(0, r), row(1, r), row(2, r), row(19, r));
+                bf = make_float4(row(0, own), row(1, own), row(2, own), __int_as_float(s_link[m].x));
+            } else if (quarter == 1) {
+                lf = make_float4(row(20, m), row(21, m), w_at(0, m), w_at(1, m));
+                nf = make_float4(row(20, r), row(21, r), w_at(0, ar), w_at(1, ar));
+                bf = make_float4(row(3, own), row(4, own), row(5, own), __int_as_float(s_link[m].y));
+            } else if (quarter == 2) {
+                lf = make_float4(w_at(2, m), row(9, m), row(10, m), row(11, m));
+                nf = make_float4(w_at(2, ar), row(9, own), row(10, own), row(11, own));
+                bf = make_float4(row(19, own), row(20, own), row(21, own), row(22, own));
+            } else {
+                lf = make_float4(row(12, m), row(13, m), row(14, m), 1.0f);
+                nf = make_float4(row(12, own), row(13, own), row(14, own), (float)__float_as_int(row(27, own)));
+                bf = make_float4(row(23, own), row(24, own), row(25, own), row(26, own));
+            }
+            if (m < leaves) b.records[4 * (size_t)base + e] = lf;
+            if (m < nodes) {
+                b.records[4 * ((size_t)n + base) + e] = nf;
+                b.bounds[4 * (size_t)base + e] = bf;
+            }
+        }
+        // reference node-data layout (AvplBvhNodeData, bvh.cu:673-724, sorted as bvh.cu:793-808)
+        for (int e = j; e < 3 * kBlockLeaves; e += kBlockLeaves) {
+            const int m = e / 3, c = e - 3 * m, own = kBlockLeaves + m, r = s_rep[m].x;
+            const int64_t lo = 3 * (int64_t)base + e, no = 3 * ((int64_t)n + base) + e;
+            auto f = [](ArcFloat3* p) { return reinterpret_cast<float*>(p); };
+            if (m < leaves) {
+                const float p = row(c, m), nr = row(19 + c, m);
+                f(b.nd.position)[lo] = p;
+                f(b.nd.normal)[lo] = nr;
+                f(b.nd.incRadiance)[lo] = row(6 + c, m);
+                f(b.nd.incDirection)[lo] = w_at(c, m);
+                f(b.sorted_pos)[lo] = p;
+                f(b.sorted_nrm)[lo] = nr;
+            }
+            if (m < nodes) {
+                f(b.nd.position)[no] = row(c, r);
+                f(b.nd.normal)[no] = row(19 + c, r);
+                f(b.nd.incRadiance)[no] = row(6 + c, own);
+                f(b.nd.incDirection)[no] = w_at(c, r);
+            }
+        }
+    }
+    // ---- what is left to lbvh_climb: roots of the block (nodes whose parent reaches over it) ----
+    const bool leaf_root = i < n && s_up[j] < 0, node_root = local && s_up[kBlockLeaves + j] < 0;
+    const bool above = has_node && !local;
+    int slot[3] = {0, 0, 0};
+    if (leaf_root) slot[0] = atomicAdd(&s_count[0], 1);
+    if (node_root) slot[1] = atomicAdd(&s_count[0], 1);
+    if (above) slot[2] = atomicAdd(&s_count[1], 1);
+    __syncthreads();
+    if (j < 2) s_base[j] = atomicAdd(&b.counts[j], s_count[j]);
+    __syncthreads();
+    if (leaf_root) {
+        b.roots[s_base[0] + slot[0]] = i;
+        store_state(b.state, i, get(j));
+    }
+    if (node_root) {
+        b.roots[s_base[0] + slot[1]] = n + i;
+        store_state(b.state, n + i, s);
+    }
+    if (above) {
+        b.top[s_base[1] + slot[2]] = i;
+        b.visit[i] = 0;
+    }
 }
 
-// One thread per leaf climbs towards the root; at each inner node the first thread to arrive
-// stops and the second merges the two children.  Nodes whose leaf range lies inside the block's
-// kBottomUpThreads leaves are settled in shared memory with block-scope ordering (both arrivals
-// come from this block); the others through the global visit counters with device-scope fences.
-constexpr int kBottomUpThreads = 256;
+// From every block root towards the tree's root: at each inner node above the blocks the first thread to
+// arrive stops and the second merges the two children's states.
+__global__ void __launch_bounds__(128) lbvh_climb(BlockArgs b) {
+    if (*b.abort != 0u) return;
+    const int n = b.n, roots = b.counts[0];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < roots; q += gridDim.x * blockDim.x) {
+        int parent = b.parents[b.roots[q]];
+        // a valid tree reaches the root within n - 1 steps; the bound guards against a corrupt one
+        for (int steps = 0; parent >= 0; ++steps) {
+            if (steps >= n || parent >= n - 1) {
+                set_error(b.err, ARC_DEVERR_BAD_NODE);
+                break;
+            }
+            const int k = parent;
+            const int lc = b.left[k], rc = b.right[k];
+            parent = b.parents[n + k];
+            __threadfence();  // release this thread's state of the child
+            if (atomicAdd(&b.visit[k], 1) == 0) break;
+            __threadfence();  // acquire the sibling's
+            const NodeState l = load_state(b.state, lc >= 0 ? lc : n - (lc + 1)),
+                            r = load_state(b.state, rc >= 0 ? rc : n - (rc + 1));
+            float rnd;
+            NodeState o;
+            merge_sums(o, l, r, b.seed, n + k, &rnd);
+            o.cn = cone_union(l.cn, r.cn);
+            o.cw = cone_union(l.cw, r.cw);
+            store_state(b.state, n + k, o);
+        }
+    }
+}
 
-__global__ void __launch_bounds__(kBottomUpThreads) lbvh_bottom_up(BottomUpArgs b) {
-    __shared__ int arrivals[kBottomUpThreads];
-    arrivals[threadIdx.x] = 0;
-    __syncthreads();
-    const int base = blockIdx.x * kBottomUpThreads;
-    const int i = base + threadIdx.x;
-    const int n = b.n;
-    if (*b.abort != 0u) return;  // uniform over the CTA: before any barrier below
-    if (i >= n) return;
-    int parent = b.parents[i];
-    // a valid tree reaches the root within n - 1 steps; the bound guards against a corrupt one
-    for (int steps = 0; parent >= 0; ++steps) {
-        if (steps >= n || parent >= n - 1) {
-            set_error(b.err, ARC_DEVERR_BAD_NODE);
-            return;
-        }
-        const int k = parent;
-        const int2 rg = *reinterpret_cast<const int2*>(b.range + 2 * (size_t)k);
-        const int lc = b.left[k], rc = b.right[k];
-        // node k is one end of its own range, so a local node's slot k - base is in [0, 256)
-        const bool local = rg.x >= base && rg.y < base + kBottomUpThreads && k >= base && k < base + kBottomUpThreads;
-        if (local) {
-            __threadfence_block();  // release this thread's writes (the child it just finished)
-            if (atomicAdd(&arrivals[k - base], 1) == 0) return;
-            __threadfence_block();  // acquire the sibling's writes
-            merge_node<true>(b, k, lc, rc);
-        } else {
-            __threadfence();
-            if (atomicAdd(&b.visit[k], 1) == 0) return;
-            __threadfence();
-            merge_node<false>(b, k, lc, rc);
-        }
-        parent = b.parents[n + k];
+// Outputs of the nodes above the blocks, one thread each.
+__global__ void __launch_bounds__(128) lbvh_top_nodes(BlockArgs b) {
+    if (*b.abort != 0u) return;
+    const int n = b.n, count = b.counts[1];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        const int k = b.top[q];
+        const NodeState s = load_state(b.state, n + k);
+        const float4* r = b.records + 4 * (size_t)s.rep;
+        const float4* ra = b.records + 4 * (size_t)s.arep;
+        const float4 q0 = r[0], q1 = r[1], a1 = ra[1];
+        write_node(b, k, b.left[k], b.right[k], s, arc_node_random(b.seed, (uint32_t)(n + k)), f3(q0.x, q0.y, q0.z),
+                   f3(q0.w, q1.x, q1.y), f3(q1.z, q1.w, r[2].x), f3(a1.z, a1.w, ra[2].x),
+                   b.nd.materialIndex[s.rep]);
     }
 }
 
@@ -613,29 +909,35 @@ arc_status launch_lbvh_build(arc_lbvh* bvh, const ArcAvplsGpuParam* avpls, const
     ARC_CHECK_ARG(p->bbox_mode == ARC_BBOX_SCENE || p->bbox_mode == ARC_BBOX_AVPL_REFERENCE, "bad bbox_mode");
     cudaStream_t st = ctx->stream;
     const int total = 2 * n - 1;
-    const int tiles = (n + kSortTile - 1) / kSortTile;
+    // Keys per thread of a sort pass: few for small inputs, whose passes are one tile's latency (four
+    // passes over 16,384 keys: 36 / 37 / 50 us with 4 / 8 / 16), many for large ones, whose tiles wait on
+    // each other in a row (262,144: 66 / 52 / 59 us; 1,000,003: 273 / 153 / 109 us).
+    const int kpt = n <= (1 << 16) ? 4 : n <= (1 << 19) ? 8 : 16;
+    const int tiles = (n + kSortThreads * kpt - 1) / (kSortThreads * kpt);
 
     uint32_t *keys0, *keys1, *hist, *status, *bb;
-    int32_t *vals0, *vals1, *left, *right, *parents, *range, *visit;
-    float4 *records, *cones, *bounds, *dirstat;
-    float4* bbox;
+    int32_t *vals0, *vals1, *left, *right, *parents, *range;
+    float4 *records, *bounds, *dirstat;
+    BlockArgs bu;
     ARC_TRY(get(bvh, "keys0", n, &keys0));
     ARC_TRY(get(bvh, "keys1", n, &keys1));
     ARC_TRY(get(bvh, "vals0", n, &vals0));
     ARC_TRY(get(bvh, "vals1", n, &vals1));
-    // hist[4*256] | tile counters[4] | bbox[12] | abort word share one zeroed block
-    ARC_TRY(get(bvh, "hist", 1024 + 4 + 12 + 1, &hist));
+    // hist[4*256] | tile counters[4] | root and top node counts[2] | abort word | bbox[12] share one block,
+    // zeroed but for the box
+    ARC_TRY(get(bvh, "hist", 1024 + 4 + 2 + 1 + 12, &hist));
     ARC_TRY(get(bvh, "status", (size_t)4 * tiles * 256, &status));
     ARC_TRY(get(bvh, "left", n - 1, &left));
     ARC_TRY(get(bvh, "right", n - 1, &right));
     ARC_TRY(get(bvh, "parents", total, &parents));
     ARC_TRY(get(bvh, "range", 2 * (n - 1), &range));
-    ARC_TRY(get(bvh, "visit", n - 1, &visit));
+    ARC_TRY(get(bvh, "visit", n - 1, &bu.visit));
+    ARC_TRY(get(bvh, "roots", total, &bu.roots));
+    ARC_TRY(get(bvh, "top", n - 1, &bu.top));
     ARC_TRY(get(bvh, "records", (size_t)4 * total, &records));
-    ARC_TRY(get(bvh, "cones", (size_t)2 * total, &cones));
     ARC_TRY(get(bvh, "dirstat", total, &dirstat));
     ARC_TRY(get(bvh, "bounds", (size_t)4 * (n - 1), &bounds));
-    ARC_TRY(get(bvh, "bbox", (size_t)2 * total, &bbox));
+    ARC_TRY(get(bvh, "state", (size_t)8 * total, &bu.state));
     ArcAvplBvhNodeDataParam nd;
     ARC_TRY(get(bvh, "nd_size", total, &nd.size));
     ARC_TRY(get(bvh, "nd_mat", total, &nd.materialIndex));
@@ -646,14 +948,13 @@ arc_status launch_lbvh_build(arc_lbvh* bvh, const ArcAvplsGpuParam* avpls, const
     ARC_TRY(get(bvh, "nd_w", total, &nd.incDirection));
     ARC_TRY(get(bvh, "sorted_pos", n, &bvh->sorted_positions));
     ARC_TRY(get(bvh, "sorted_nrm", n, &bvh->sorted_normals));
-    bb = hist + 1024 + 4;
     uint32_t* tile_counters = hist + 1024;
-    uint32_t* abort = hist + 1024 + 4 + 12;
+    bu.counts = reinterpret_cast<int32_t*>(hist + 1024 + 4);
+    uint32_t* abort = hist + 1024 + 4 + 2;
+    bb = abort + 1;
 
-    ARC_TRY_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * 1028, st));
-    ARC_TRY_CUDA(cudaMemsetAsync(abort, 0, sizeof(uint32_t), st));
+    ARC_TRY_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * (1024 + 4 + 2 + 1), st));
     ARC_TRY_CUDA(cudaMemsetAsync(status, 0, sizeof(uint32_t) * 4 * (size_t)tiles * 256, st));
-    ARC_TRY_CUDA(cudaMemsetAsync(visit, 0, sizeof(int32_t) * (size_t)(n - 1), st));
 
     const int grid_stride_blocks = ctx->sm_count * 4;
     stage_begin(ctx, "lbvh_morton");
@@ -698,7 +999,8 @@ arc_status launch_lbvh_build(arc_lbvh* bvh, const ArcAvplsGpuParam* avpls, const
         s.spin_limit = p->wait_limit ? p->wait_limit : (1u << 26);
         s.abort = abort;
         s.err = ctx->d_error;
-        lbvh_sort_pass<<<tiles, kSortThreads, 0, st>>>(s);
+        auto* pass_kernel = kpt == 4 ? lbvh_sort_pass<4> : kpt == 8 ? lbvh_sort_pass<8> : lbvh_sort_pass<16>;
+        pass_kernel<<<tiles, kSortThreads, 0, st>>>(s);
         ARC_TRY_CUDA(cudaGetLastError());
         std::swap(kin, kout);
         std::swap(vin, vout);
@@ -707,50 +1009,45 @@ arc_status launch_lbvh_build(arc_lbvh* bvh, const ArcAvplsGpuParam* avpls, const
     stage_end(ctx, 4);
     stage_begin(ctx, "lbvh_karras");
 
-    KarrasArgs k;
+    TopologyArgs k;
     k.morton = kin;
-    k.sorted_index = vin;
-    k.a = *avpls;
-    k.mats = ctx->d_materials;
-    k.num_mats = ctx->num_materials;
     k.n = n;
-    k.seed = p->repr_seed;
     k.left = left;
     k.right = right;
     k.parents = parents;
     k.range = range;
-    k.records = records;
-    k.cones = cones;
-    k.dirstat = dirstat;
-    k.bbox = bbox;
-    k.nd = nd;
-    k.sorted_pos = bvh->sorted_positions;
-    k.sorted_nrm = bvh->sorted_normals;
     k.abort = abort;
-    k.err = ctx->d_error;
-    lbvh_karras<<<(n + 255) / 256, 256, 0, st>>>(k);
+    lbvh_topology<<<(n - 1 + 255) / 256, 256, 0, st>>>(k);
     stage_end(ctx, 1);
     ARC_TRY_CUDA(cudaGetLastError());
 
-    BottomUpArgs bu;
+    bu.abort = abort;
+    bu.err = ctx->d_error;
+    bu.sorted_index = vin;
+    bu.a = *avpls;
+    bu.mats = ctx->d_materials;
+    bu.num_mats = ctx->num_materials;
     bu.n = n;
     bu.seed = p->repr_seed;
     bu.left = left;
     bu.right = right;
     bu.parents = parents;
     bu.range = range;
-    bu.visit = visit;
     bu.records = records;
-    bu.cones = cones;
     bu.dirstat = dirstat;
-    bu.bbox = bbox;
     bu.bounds = bounds;
     bu.nd = nd;
-    bu.abort = abort;
-    bu.err = ctx->d_error;
+    bu.sorted_pos = bvh->sorted_positions;
+    bu.sorted_nrm = bvh->sorted_normals;
     stage_begin(ctx, "lbvh_bottom_up");
-    lbvh_bottom_up<<<(n + kBottomUpThreads - 1) / kBottomUpThreads, kBottomUpThreads, 0, st>>>(bu);
-    stage_end(ctx, 1);
+    const int blocks = (n + kBlockLeaves - 1) / kBlockLeaves;
+    ARC_TRY_CUDA(cudaFuncSetAttribute(lbvh_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockSmem));
+    lbvh_blocks<<<blocks, kBlockLeaves, kBlockSmem, st>>>(bu);
+    // (a block has about ten roots)
+    const int top_blocks = std::min(blocks, ctx->sm_count * 8);
+    lbvh_climb<<<top_blocks, 128, 0, st>>>(bu);
+    lbvh_top_nodes<<<top_blocks, 128, 0, st>>>(bu);
+    stage_end(ctx, 3);
     ARC_TRY_CUDA(cudaGetLastError());
 
     bvh->n = n;
