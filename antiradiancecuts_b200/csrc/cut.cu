@@ -35,6 +35,7 @@ namespace {
 
 constexpr int kTile = 8;
 constexpr int kSolidStack = 64;
+constexpr int kSolidThreads = 64;
 constexpr int kChunkSize = 1024;  // cut entries per pool chunk
 constexpr int kSetupWarps = 4;
 constexpr int kSelThreads = 128;
@@ -59,8 +60,10 @@ struct SolidArgs {
     float3 cam;
     int n;
     const float4* bounds;
+    const float4* records;
     ArcAvplBvhNodeDataParam nd;
     float thresh;
+    float cos2, cos2_margin;  // (1 - thresh / 2 pi)^2; distance from it at which the approximate test holds
     float clamp2;
     double* rad64;
     float4* out_rad;
@@ -105,92 +108,151 @@ __device__ __forceinline__ float3 node_radiance(const SolidArgs& a, const MatSme
     return f3(L.x * fl.x * fr.x * g, L.y * fl.y * fr.y * g, L.z * fl.z * fr.z * g);
 }
 
-__global__ void __launch_bounds__(256) cut_solid_angle_kernel(SolidArgs a) {
+__device__ __forceinline__ float rcp_approx(float x) {  // 1 ulp
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The same without specular materials, leaving out the receiver's diffuse / pi (a constant of the pixel):
+// L f_l max(n.d, 0) max(-n_a.d, 0) / (d^2 max(d^2, clamp^2)), d = p_a - p.  The 1/|d| factors of the two
+// cosines are one reciprocal of d^2.
+__device__ __forceinline__ float3 node_radiance_diffuse(const SolidArgs& a, const MatSmem& sm, float3 p, float3 n,
+                                                        int idx) {
+    const float4 q0 = a.records[4 * (size_t)idx], q1 = a.records[4 * (size_t)idx + 1];  // p_a, n_a
+    const float3 wa = ld3(a.nd.incDirection, idx), L = ld3(a.nd.incRadiance, idx);
+    int ma = a.nd.materialIndex[idx];
+    if (ma < 0 || ma >= a.num_mats) ma = 0;
+    const float3 v = f3(q0.x, q0.y, q0.z) - p, na = f3(q0.w, q1.x, q1.y);
+    const float l2 = dot(v, v);
+    if (!(l2 > 0.0f)) return f3(0, 0, 0);
+    float3 f = L;
+    if (dot(wa, wa) != 0.0f) {
+        const float4 d = sm.m[ma].diffuse_exp;
+        f = f3(L.x * (kOneOverPi * d.x), L.y * (kOneOverPi * d.y), L.z * (kOneOverPi * d.z));
+    }
+    const float c1 = fmaxf(dot(n, v) * rcp_approx(l2), 0.0f);
+    const float c2 = fmaxf(-dot(na, v) * rsqrtf(dot(na, na)) * rcp_approx(fmaxf(l2, a.clamp2)), 0.0f);
+    return (c1 * c2) * f;
+}
+
+// One warp per 8 x 4 pixels walks the tree once for all of them: an entry of its stack is a node and the
+// mask of the pixels that visit it.  Each pixel visits the nodes of its own walk in its own order (the
+// sums are the same), but a node's data are loaded once per warp from one address instead of by 32 lanes
+// from as many, and neighbouring pixels' walks coincide almost everywhere.
+template <bool SPECULAR>
+__global__ void __launch_bounds__(kSolidThreads) cut_solid_angle_kernel(SolidArgs a) {
     __shared__ MatSmem sm;
+    __shared__ int s_node[kSolidThreads / 32][kSolidStack];
+    __shared__ unsigned s_mask[kSolidThreads / 32][kSolidStack];
     for (int i = threadIdx.x; i < a.num_mats; i += blockDim.x) sm.m[i] = a.mats[i];
     __syncthreads();
-    const int x = blockIdx.x * 16 + threadIdx.x % 16;
-    const int y = blockIdx.y * 16 + threadIdx.x / 16;
-    if (x >= a.width || y >= a.height) return;
-    const float4 gp = a.gpos[(int64_t)y * a.gpitch + x];
-    const float4 gn = a.gnrm[(int64_t)y * a.gpitch + x];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // a block's two warps: 8 x 8 pixels (small blocks, because neighbouring tiles' walks differ in length)
+    const int x = blockIdx.x * 8 + (lane & 7);
+    const int y = blockIdx.y * 8 + w * 4 + (lane >> 3);
+    const bool inside = x < a.width && y < a.height;
+    float4 gp = make_float4(0, 0, 0, 0), gn = make_float4(0, 0, 0, 0);
+    if (inside) {
+        gp = a.gpos[(int64_t)y * a.gpitch + x];
+        gn = a.gnrm[(int64_t)y * a.gpitch + x];
+    }
     const int mat = (int)gn.w;
-    const int64_t o = (int64_t)y * a.opitch + x;
     float s[3] = {0, 0, 0}, c[3] = {0, 0, 0};
-    bool error = false;
-    if (mat != 0 && !(mat > 0 && mat < a.num_mats)) set_error(a.err, ARC_DEVERR_BAD_MATERIAL);
-    if (mat > 0 && mat < a.num_mats) {
-        const float3 p = f3(gp.x, gp.y, gp.z);
-        const float3 nraw = f3(gn.x, gn.y, gn.z);
-        const float3 n = norm3(nraw);
-        const float3 w_o = norm3(a.cam - p);
-        const bool dbg = a.used && x == a.dbg_x && y == a.dbg_y;
-        int stack[kSolidStack];
-        stack[0] = -1;
-        int sp = 1;
-        const float two_pi = rn_mul(2.0f, kPi);
-        // every node is visited at most once in a valid tree: 2n - 1 pops bound the walk
-        int budget = 2 * a.n;
-        while (sp > 0) {
-            if (--budget < 0) {
-                error = true;
-                set_error(a.err, ARC_DEVERR_BAD_NODE);
-                break;
+    const bool surface = mat > 0 && mat < a.num_mats;
+    if (mat != 0 && !surface) set_error(a.err, ARC_DEVERR_BAD_MATERIAL);
+    const float3 p = f3(gp.x, gp.y, gp.z);
+    const float3 nraw = f3(gn.x, gn.y, gn.z);
+    const float3 n = norm3(nraw);
+    const float3 w_o = norm3(a.cam - p);
+    const bool dbg = a.used && x == a.dbg_x && y == a.dbg_y;
+    const float two_pi = rn_mul(2.0f, kPi);
+    int* nodes = s_node[w];
+    unsigned* masks = s_mask[w];
+    const unsigned start = __ballot_sync(0xffffffffu, surface);
+    unsigned failed = 0;  // pixels whose walk was given up
+    int sp = 0;
+    if (start) {
+        if (lane == 0) {
+            nodes[0] = -1;
+            masks[0] = start;
+        }
+        sp = 1;
+    }
+    __syncwarp();
+    // every node is visited at most once in a valid tree: 2n - 1 pops bound the walk
+    int budget = 2 * a.n;
+    while (sp > 0) {
+        --sp;
+        const int node = nodes[sp];
+        const unsigned mask = masks[sp] & ~failed;
+        __syncwarp();  // read by every lane before the children overwrite the entry
+        if (--budget < 0 || node >= a.n || node < -(a.n - 1)) {
+            failed |= mask;
+            if (lane == 0) set_error(a.err, ARC_DEVERR_BAD_NODE);
+            if (budget < 0) break;
+            continue;
+        }
+        bool use = mask >> lane & 1u;
+        int idx = node;
+        if (node < 0) {
+            const int k = -(node + 1);
+            idx = a.n + k;
+            const float4 b0 = a.bounds[4 * (size_t)k], b1 = a.bounds[4 * (size_t)k + 1];
+            const float4 q0 = a.records[4 * (size_t)idx];  // the representative's position
+            // visibility of the box corners (cudaGather.cu:405-408); the sign of
+            // n.normalize(v) is the sign of n.v
+            use = use &&
+                  (rn_dot(nraw.x, nraw.y, nraw.z, rn_sub(b1.x, p.x), rn_sub(b1.y, p.y), rn_sub(b1.z, p.z)) > 0.0f ||
+                   rn_dot(nraw.x, nraw.y, nraw.z, rn_sub(b0.x, p.x), rn_sub(b0.y, p.y), rn_sub(b0.z, p.z)) > 0.0f);
+            const float ex = rn_sub(b1.x, b0.x), ey = rn_sub(b1.y, b0.y), ez = rn_sub(b1.z, b0.z);
+            const float vx = rn_sub(q0.x, p.x), vy = rn_sub(q0.y, p.y), vz = rn_sub(q0.z, p.z);
+            const float d2 = rn_dot(vx, vy, vz, vx, vy, vz), e2 = rn_dot(ex, ey, ez, ex, ey, ez);
+            // solid angle < threshold <=> d^2 / (d^2 + r^2) > cos^2, without the square roots and the
+            // division unless the two sides are closer than the rounding of the test as written
+            const float h2 = fmaf(0.25f, e2, d2), gap = fmaf(-a.cos2, h2, d2);
+            bool below = gap > 0.0f;
+            if (use && !(fabsf(gap) > a.cos2_margin * h2)) {
+                const float radius = rn_mul(0.5f, rn_sqrt(e2)), dist = rn_sqrt(d2);
+                below = rn_mul(two_pi, rn_sub(1.0f, rn_div(dist, rn_sqrt(rn_add(rn_mul(radius, radius),
+                                                                                rn_mul(dist, dist)))))) < a.thresh;
             }
-            const int node = stack[--sp];
-            if (node >= a.n) {
-                error = true;
-                set_error(a.err, ARC_DEVERR_BAD_NODE);
-                break;
-            }
-            int idx;
-            if (node >= 0) {
-                idx = node;
-            } else {
-                const int k = -(node + 1);
-                if (k >= a.n - 1) {
-                    error = true;
-                    set_error(a.err, ARC_DEVERR_BAD_NODE);
-                    break;
-                }
-                const float4 b0 = a.bounds[4 * (size_t)k], b1 = a.bounds[4 * (size_t)k + 1];
-                // visibility of the box corners (cudaGather.cu:405-408); the sign of
-                // n.normalize(v) is the sign of n.v
-                const bool vis = rn_dot(nraw.x, nraw.y, nraw.z, rn_sub(b1.x, p.x), rn_sub(b1.y, p.y), rn_sub(b1.z, p.z)) >
-                                     0.0f ||
-                                 rn_dot(nraw.x, nraw.y, nraw.z, rn_sub(b0.x, p.x), rn_sub(b0.y, p.y), rn_sub(b0.z, p.z)) >
-                                     0.0f;
-                if (!vis) continue;
-                idx = a.n + k;
-                const float3 pr = ld3(a.nd.position, idx);
-                const float ex = rn_sub(b1.x, b0.x), ey = rn_sub(b1.y, b0.y), ez = rn_sub(b1.z, b0.z);
-                const float radius = rn_mul(0.5f, rn_sqrt(rn_dot(ex, ey, ez, ex, ey, ez)));
-                const float vx = rn_sub(pr.x, p.x), vy = rn_sub(pr.y, p.y), vz = rn_sub(pr.z, p.z);
-                const float dist = rn_sqrt(rn_dot(vx, vy, vz, vx, vy, vz));
-                const float solid = rn_mul(
-                    two_pi,
-                    rn_sub(1.0f, rn_div(dist, rn_sqrt(rn_add(rn_mul(radius, radius), rn_mul(dist, dist))))));
-                if (!(solid < a.thresh)) {
-                    if (sp + 2 > kSolidStack) {
-                        error = true;
-                        set_error(a.err, ARC_DEVERR_STACK_OVERFLOW);
-                        break;
+            const bool refine = use && !below;
+            use = use && !refine;
+            const unsigned down = __ballot_sync(0xffffffffu, refine);
+            if (down) {
+                if (sp + 2 > kSolidStack) {
+                    failed |= down;
+                    if (lane == 0) set_error(a.err, ARC_DEVERR_STACK_OVERFLOW);
+                } else {
+                    if (lane < 2) {
+                        nodes[sp + lane] = __float_as_int(lane == 0 ? b0.w : b1.w);
+                        masks[sp + lane] = down;
                     }
-                    stack[sp++] = __float_as_int(b0.w);
-                    stack[sp++] = __float_as_int(b1.w);
-                    continue;
+                    sp += 2;
                 }
             }
-            const float3 t = node_radiance(a, sm, p, n, mat, w_o, idx);
+        }
+        if (use) {
+            const float3 t = SPECULAR ? node_radiance(a, sm, p, n, mat, w_o, idx)
+                                      : node_radiance_diffuse(a, sm, p, n, idx);
             kahan_add(s[0], c[0], t.x);
             kahan_add(s[1], c[1], t.y);
             kahan_add(s[2], c[2], t.z);
             if (dbg) a.used[idx] = 1;
         }
+        __syncwarp();  // the pushes
     }
+    if (!inside) return;
+    const int64_t o = (int64_t)y * a.opitch + x;
     double r[3];
     for (int q = 0; q < 3; ++q) r[q] = (double)s[q] - (double)c[q];
-    if (error) {
+    if (!SPECULAR) {
+        const float4 d = sm.m[surface ? mat : 0].diffuse_exp;
+        const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
+        for (int q = 0; q < 3; ++q) r[q] = surface ? r[q] * (double)kd[q] : 0.0;
+    }
+    if (failed >> lane & 1u) {
         r[0] = 100000.0;
         r[1] = 0.0;
         r[2] = 100000.0;
@@ -1008,8 +1070,13 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
         a.cam = cam;
         a.n = bvh->n;
         a.bounds = reinterpret_cast<const float4*>(bvh->view.bounds);
+        a.records = reinterpret_cast<const float4*>(bvh->view.records);
         a.nd = bvh->view.node_data;
         a.thresh = cp->solid_angle_threshold;
+        const double cosine = 1.0 - (double)a.thresh / (2.0 * 3.14159265358979);
+        a.cos2 = (float)(cosine * cosine);
+        // the test as written is within 5e-7 of the cosine (a dozen roundings of values <= 1)
+        a.cos2_margin = cosine >= 0.0 && cosine <= 1.0 ? 4e-6f : INFINITY;
         a.clamp2 = clamp2;
         a.rad64 = rad64;
         a.out_rad = reinterpret_cast<float4*>(out->radiance);
@@ -1018,9 +1085,12 @@ arc_status launch_gather_cut(arc_context* ctx, const arc_lbvh* bvh, const ArcAvp
         a.dbg_y = cp->debug_pixel_y;
         a.used = cp->used_nodes;
         a.err = ctx->d_error;
-        dim3 grid((W + 15) / 16, (H + 15) / 16);
+        dim3 grid((W + 7) / 8, (H + 7) / 8);
         stage_begin(ctx, "cut_solid_angle");
-        cut_solid_angle_kernel<<<grid, 256, 0, st>>>(a);
+        if (ctx->any_specular)
+            cut_solid_angle_kernel<true><<<grid, kSolidThreads, 0, st>>>(a);
+        else
+            cut_solid_angle_kernel<false><<<grid, kSolidThreads, 0, st>>>(a);
         stage_end(ctx, 1);
         ARC_TRY_CUDA(cudaGetLastError());
         if (gp->ar_kind != ARC_AR_NONE) {
