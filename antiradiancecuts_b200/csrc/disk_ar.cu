@@ -4,16 +4,19 @@
 // A pair contributes only when the AVPL's ray p_a + s w (s > 0) passes within the disk radius of the
 // pixel, the AVPL lies in front of the pixel and the pixel behind the AVPL: a handful of AVPLs per
 // pixel.  A block owns a pixel tile and walks the AVPLs in order, kStep at a time:
-//   1. each thread tests AVPLs' rays against the tile's bounding sphere grown by the radius, those that
-//      pass against each warp's sphere (a tile across a silhouette has a sphere as deep as the scene),
-//      and the block compacts the survivors in AVPL order;
-//   2. each warp tests its survivors, one per lane, against its pixels' position and normal boxes and
-//      stages the records that remain;
+//   1. each thread tests AVPLs' rays against the tile's bounding spheres grown by the radius (two, the
+//      halves of a split along the longest axis: a tile across a silhouette has one as deep as the
+//      scene), and the block compacts the survivors of several steps in AVPL order;
+//   2. each warp tests the survivors, one per lane, against its own pixels' two spheres and their position
+//      and normal boxes, and stages the records that remain;
 //   3. every lane evaluates those for its pixels with the terms of pair_terms, in AVPL order, with one
 //      compensated sum per channel.
 // The tests drop a pair only when pair_terms is certain to give 0 (their margins exceed its rounding),
 // so the sums are those over every AVPL.  Several blocks share a tile, each with a segment of the AVPLs
-// (tiles differ widely in work); disk_combine adds their sums in FP64.  The work left is the ray tests, 20 operations per (tile,
+// (tiles differ in work); disk_combine adds their sums in FP64.
+//
+// Bound by latency (a step's loads, ballots and barrier; the lists hold a few per cent of the rays).
+// 512 x 512 x 32,768: 0.28 ms, 21.5 ms for the kernel that evaluated every pair.  The work left is the ray tests, 20 operations per (tile,
 // AVPL) instead of 45 per (pixel, AVPL).
 #include <algorithm>
 #include <cfloat>
@@ -27,24 +30,27 @@ namespace arc {
 namespace {
 
 constexpr int kThreads = 256, kWarps = kThreads / 32;
-constexpr int kPerThread = 4;                     // rays tested per thread and step
+constexpr int kPerThread = 2;                     // rays tested per thread and step
 constexpr int kStep = kThreads * kPerThread;      // AVPLs per step
-static_assert(kPerThread * kWarps == 32, "one lane per (pass, warp) count in the block's prefix sum");
+constexpr int kList = 1024;                       // survivors collected before the warps go over them
+constexpr int kCounts = kPerThread * kWarps;      // survivor counts of a step, one per (pass, warp)
+static_assert(kCounts <= 32, "one lane per count in the block's prefix sum");
 
 // 32 x 32 tiles when they make at least this many blocks per SM (a quarter of the ray tests; 1280 x 720 x
-// 65,536: 0.92 against 1.34 ms), else 16 x 16 (more, smaller blocks).
+// 65,536: 0.55 against 0.99 ms), else 16 x 16 (more, smaller blocks).
 constexpr int64_t kBigTilesPerSm = 2;
-// Segments: a tile across a silhouette sees a third of all rays and takes 40 times the mean, so the
-// AVPLs are split until there are this many blocks per SM (512 x 512 x 32,768 / 1280 x 720 x 65,536: 0.49 /
-// 1.29 ms at 16 per SM, 0.42 / 0.92 ms at 64, 0.46 ms at 128, where the blocks' set-up costs more than the
-// balance gains), partial sums within kPartialBytes.
-constexpr int64_t kBlocksPerSm = 64;
+// Segments: blocks per SM at which the AVPLs are no longer split (512 x 512 x 32,768 / 1280 x 720 x 65,536:
+// 0.28 / 0.64 ms at 8 per SM, 0.28 / 0.55 ms at 16, 0.29 / 0.51 ms at 32: the blocks' set-up against their
+// balance), partial sums within kPartialBytes.
+constexpr int64_t kBlocksPerSm = 24;
 constexpr int64_t kPartialBytes = (int64_t)1 << 30;
 
 struct DiskArgs {
     const float4* records;  // 4 float4 per AVPL (launch_pack_records)
-    // 2 float4 per AVPL: {p, 0: adds nothing, > 0: adds where its ray passes, < 0: to every pixel}, {w / |w|, 0}
+    // 2 float4 per AVPL that can add something: {p, > 0: where its ray passes, < 0: to every pixel},
+    // {w / |w|, index}; counts[s] of them from kStep s on
     const float4* rays;
+    const int* counts;
     int n;
     const float4* gpos;
     const float4* gnrm;
@@ -63,17 +69,41 @@ struct DiskArgs {
     uint32_t* err;
 };
 
-// The rays of the packed records.  An AVPL without antiradiance or without a direction adds 0 to
-// every pixel; one with a non-finite antiradiance is kept.
-__global__ void disk_rays(const float4* records, int n, float4* rays) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 q0 = records[4 * (size_t)i], q1 = records[4 * (size_t)i + 1], q2 = records[4 * (size_t)i + 2],
-                 q3 = records[4 * (size_t)i + 3];
-    const float la = fabsf(q3.x) + fabsf(q3.y) + fabsf(q3.z);
-    const bool never = la == 0.0f || (la <= FLT_MAX && q1.z == 0.0f && q1.w == 0.0f && q2.x == 0.0f);
-    rays[2 * (size_t)i] = make_float4(q0.x, q0.y, q0.z, never ? 0.0f : la <= FLT_MAX ? 1.0f : -1.0f);
-    rays[2 * (size_t)i + 1] = make_float4(q1.z * q3.w, q1.w * q3.w, q2.x * q3.w, 0.0f);
+// The rays of the packed records, compacted within each step of kStep AVPLs (in AVPL order; counts[s] of
+// step s are left).  An AVPL without antiradiance or without a direction adds 0 to every pixel and is
+// dropped (half of them); one with a non-finite antiradiance is kept.
+__global__ void __launch_bounds__(kStep) disk_rays(const float4* records, int n, float4* rays, int* counts) {
+    __shared__ int s_cnt[kStep / 32];
+    const int i = blockIdx.x * kStep + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float4 q0, q1, q2, q3;
+    bool keep = false, finite = true;
+    if (i < n) {
+        q0 = records[4 * (size_t)i];
+        q1 = records[4 * (size_t)i + 1];
+        q2 = records[4 * (size_t)i + 2];
+        q3 = records[4 * (size_t)i + 3];
+        const float la = fabsf(q3.x) + fabsf(q3.y) + fabsf(q3.z);
+        finite = la <= FLT_MAX;
+        keep = !(la == 0.0f || (finite && q1.z == 0.0f && q1.w == 0.0f && q2.x == 0.0f));
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) s_cnt[w] = __popc(m);
+    __syncthreads();
+    static_assert(kStep / 32 <= 32, "one lane per warp's count");
+    const int mine = lane < kStep / 32 ? s_cnt[lane] : 0;
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int first = __shfl_sync(0xffffffffu, incl - mine, w);
+    if (threadIdx.x == 31) counts[blockIdx.x] = incl;
+    if (keep) {
+        const size_t d = (size_t)blockIdx.x * kStep + first + __popc(m & ((1u << lane) - 1u));
+        rays[2 * d] = make_float4(q0.x, q0.y, q0.z, finite ? 1.0f : -1.0f);
+        rays[2 * d + 1] = make_float4(q1.z * q3.w, q1.w * q3.w, q2.x * q3.w, __int_as_float(i));
+    }
 }
 
 // Whether the ray from r0 along the unit vector r1 can pass within `radius` of a point of the sphere
@@ -102,13 +132,12 @@ __device__ __forceinline__ void write_ar(const DiskArgs& a, int x, int y, int ma
 
 // PX = 1: 16 x 16 pixel tiles, 8 x 4 pixels per warp; PX = 4: 32 x 32 tiles, 16 x 8 per warp.
 template <int PX>
-__global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
+__global__ void __launch_bounds__(kThreads, PX == 1 ? 3 : 2) disk_antiradiance(DiskArgs a) {
     constexpr int kSide = PX == 1 ? 16 : 32, kSub = PX == 1 ? 1 : 2, kIlp = 4 / PX;
     __shared__ float4 s_rec[kWarps][32 * 4];
-    __shared__ int s_list[kStep];
-    __shared__ unsigned char s_who[kStep];  // the warps that an entry of the list concerns
-    __shared__ float4 s_ball[kWarps];       // each warp's bounding sphere (radius < 0: no pixels)
-    __shared__ int s_cnt[32];
+    __shared__ int s_list[kList];
+    __shared__ PixelBounds s_half[2][kWarps];  // (positions only)
+    __shared__ int s_cnt[2][kCounts];
     __shared__ PixelBounds s_box[kWarps];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int xb = blockIdx.x * kSide + (w & 1) * 8 * kSub + (lane & 7);
@@ -157,67 +186,116 @@ __global__ void __launch_bounds__(kThreads) disk_antiradiance(DiskArgs a) {
         __syncthreads();
         PixelBounds tb = s_box[0];
         for (int q = 1; q < kWarps; ++q) tb.merge(s_box[q]);
-        // bounding spheres of the tile and of the warp, grown by the disk radius
-        auto sphere = [&](const PixelBounds& b, float& cx, float& cy, float& cz) {
-            cx = 0.5f * (b.pmin[0] + b.pmax[0]);
-            cy = 0.5f * (b.pmin[1] + b.pmax[1]);
-            cz = 0.5f * (b.pmin[2] + b.pmax[2]);
+        // bounding sphere of a box, grown by the disk radius (radius -1: empty)
+        auto sphere = [&](const PixelBounds& b) {
             const float ex = b.pmax[0] - b.pmin[0], ey = b.pmax[1] - b.pmin[1], ez = b.pmax[2] - b.pmin[2];
-            return 0.5001f * sqrtf(ex * ex + ey * ey + ez * ez) + a.radius;
+            return make_float4(0.5f * (b.pmin[0] + b.pmax[0]), 0.5f * (b.pmin[1] + b.pmax[1]),
+                               0.5f * (b.pmin[2] + b.pmax[2]),
+                               b.pmin[0] <= b.pmax[0] ? 0.5001f * sqrtf(ex * ex + ey * ey + ez * ez) + a.radius : -1.0f);
         };
-        float tcx, tcy, tcz, wcx, wcy, wcz;
-        const float trho = sphere(tb, tcx, tcy, tcz);
-        const float wrho = sphere(box, wcx, wcy, wcz);
-        if (lane == 0) s_ball[w] = make_float4(wcx, wcy, wcz, warp_live ? wrho : -1.0f);
+        // the warp's pixels on one side of the middle of a box's longest axis
+        auto half = [&](const PixelBounds& whole, int side) {
+            const float e[3] = {whole.pmax[0] - whole.pmin[0], whole.pmax[1] - whole.pmin[1],
+                                whole.pmax[2] - whole.pmin[2]};
+            const int axis = e[0] >= e[1] && e[0] >= e[2] ? 0 : e[1] >= e[2] ? 1 : 2;
+            const float mid = 0.5f * (axis == 0   ? whole.pmin[0] + whole.pmax[0]
+                                      : axis == 1 ? whole.pmin[1] + whole.pmax[1]
+                                                  : whole.pmin[2] + whole.pmax[2]);
+            PixelBounds b;
+            b.clear();
+#pragma unroll
+            for (int j = 0; j < PX; ++j) {
+                const float v = axis == 0 ? px[j].px : axis == 1 ? px[j].py : px[j].pz;
+                if (mat[j] && !(v > mid) == (side == 0))  // (a position that is not a number: side 0)
+                    b.add(px[j].px, px[j].py, px[j].pz, 0, 0, 0, 0, 0, 0);
+            }
+            b.reduce_warp_positions();
+            return b;
+        };
+        const float4 mine0 = sphere(half(box, 0)), mine1 = sphere(half(box, 1));
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const PixelBounds h = half(tb, side);
+            if (lane == 0) s_half[side][w] = h;
+        }
         __syncthreads();
+        float4 tile0, tile1;
+        {
+            PixelBounds h0 = s_half[0][0], h1 = s_half[1][0];
+            for (int q = 1; q < kWarps; ++q) {
+                h0.merge(s_half[0][q]);
+                h1.merge(s_half[1][q]);
+            }
+            tile0 = sphere(h0);
+            tile1 = sphere(h1);
+        }
+        auto near_any = [&](float4 ray0, float4 ray1, float4 b0, float4 b1) {
+            return ray0.w < 0.0f || (b0.w >= 0.0f && ray_near(ray0, ray1, b0.x, b0.y, b0.z, b0.w)) ||
+                   (b1.w >= 0.0f && ray_near(ray0, ray1, b1.x, b1.y, b1.z, b1.w));
+        };
         float4* rec = s_rec[w];
         const int steps = (a.n + kStep - 1) / kStep;
-        const int first = (int)((int64_t)steps * blockIdx.z / gridDim.z) * kStep,
-                  last = (int)min((int64_t)a.n, (int64_t)steps * (blockIdx.z + 1) / gridDim.z * kStep);
-        for (int base = first; base < last; base += kStep) {
-            unsigned m[kPerThread], who[kPerThread];
+        const int first = (int)((int64_t)steps * blockIdx.z / gridDim.z),
+                  last = (int)((int64_t)steps * (blockIdx.z + 1) / gridDim.z);
+        // rays of one step ahead
+        float4 r0[kPerThread], r1[kPerThread];
+        int rays = 0;
+        auto load_step = [&](int step) {
+            rays = step < last ? a.counts[step] : 0;
 #pragma unroll
             for (int u = 0; u < kPerThread; ++u) {
-                const int i = base + u * kThreads + tid;
-                who[u] = 0;
-                if (i < last) {
-                    const float4 r0 = a.rays[2 * (size_t)i], r1 = a.rays[2 * (size_t)i + 1];
-                    if (r0.w < 0.0f || (r0.w > 0.0f && ray_near(r0, r1, tcx, tcy, tcz, trho)))
-#pragma unroll 1
-                        for (int q = 0; q < kWarps; ++q) {
-                            const float4 ball = s_ball[q];
-                            if (ball.w >= 0.0f && (r0.w < 0.0f || ray_near(r0, r1, ball.x, ball.y, ball.z, ball.w)))
-                                who[u] |= 1u << q;
-                        }
+                const int i = u * kThreads + tid;
+                if (i < rays) {
+                    const float4* r = a.rays + 2 * ((size_t)step * kStep + i);
+                    r0[u] = r[0];
+                    r1[u] = r[1];
                 }
-                m[u] = __ballot_sync(0xffffffffu, who[u] != 0);
-                if (lane == 0) s_cnt[u * kWarps + w] = __popc(m[u]);
             }
-            __syncthreads();  // the counts; and every warp is done with the list of the step before
-            int incl = s_cnt[lane];
+        };
+        load_step(first);
+        int count = 0;  // survivors in the list
+        for (int step = first; step < last; ++step) {
+            unsigned m[kPerThread];
+            int* cnt = s_cnt[step & 1];
+#pragma unroll
+            for (int u = 0; u < kPerThread; ++u) {
+                m[u] = __ballot_sync(0xffffffffu,
+                                     u * kThreads + tid < rays && near_any(r0[u], r1[u], tile0, tile1));
+                if (lane == 0) cnt[u * kWarps + w] = __popc(m[u]);
+            }
+            load_step(step + 1);
+            __syncthreads();  // the counts; and the list's readers are done
+            const int mine = lane < kCounts ? cnt[lane] : 0;
+            int incl = mine;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int v = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += v;
             }
-            const int excl = incl - s_cnt[lane];
-            const int count = __shfl_sync(0xffffffffu, incl, 31);
+            const int excl = count + incl - mine;
+            count += __shfl_sync(0xffffffffu, incl, 31);
 #pragma unroll
             for (int u = 0; u < kPerThread; ++u) {
                 const int at = __shfl_sync(0xffffffffu, excl, u * kWarps + w) + __popc(m[u] & ((1u << lane) - 1u));
-                if (who[u]) {
-                    s_list[at] = base + u * kThreads + tid;
-                    s_who[at] = (unsigned char)who[u];
-                }
+                if (m[u] >> lane & 1u) s_list[at] = step * kStep + u * kThreads + tid;
             }
+            if (count + kStep <= kList && step + 1 < last) continue;  // room for another step
             __syncthreads();
+            const int listed = count;
+            count = 0;
             if (!warp_live) continue;
-            for (int k = 0; k < count; k += 32) {
+            for (int k = 0; k < listed; k += 32) {
                 float4 q0, q1, q2, q3;
                 bool keep = false;
-                if (k + lane < count && (s_who[k + lane] >> w & 1)) {
-                    const int i = s_list[k + lane];
-                    const float4* q = a.records + 4 * (size_t)i;
+                float4 ray0, ray1;
+                if (k + lane < listed) {
+                    const float4* r = a.rays + 2 * (size_t)s_list[k + lane];
+                    ray0 = r[0];
+                    ray1 = r[1];
+                    keep = near_any(ray0, ray1, mine0, mine1);
+                }
+                if (keep) {
+                    const float4* q = a.records + 4 * (size_t)__float_as_int(ray1.w);
                     q0 = q[0];
                     q1 = q[1];
                     q2 = q[2];
@@ -326,8 +404,13 @@ arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* av
     a.records = records;
     a.n = avpls->numAvpls;
     float4* rays = nullptr;
-    ARC_TRY(ctx->arena.get("disk_rays", (size_t)(a.n + 1) * 2 * sizeof(float4), reinterpret_cast<void**>(&rays)));
+    const int steps = (a.n + kStep - 1) / kStep;
+    int* counts = nullptr;
+    ARC_TRY(ctx->arena.get("disk_rays", ((size_t)steps * kStep + 1) * 2 * sizeof(float4),
+                           reinterpret_cast<void**>(&rays)));
+    ARC_TRY(ctx->arena.get("disk_ray_counts", (size_t)(steps + 1) * sizeof(int), reinterpret_cast<void**>(&counts)));
     a.rays = rays;
+    a.counts = counts;
     a.gpos = reinterpret_cast<const float4*>(gb->position);
     a.gnrm = reinterpret_cast<const float4*>(gb->normal);
     a.gpitch = gb->pitch;
@@ -347,13 +430,13 @@ arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* av
     a.err = ctx->d_error;
     cudaStream_t st = ctx->stream;
     stage_begin(ctx, "disk_antiradiance");
-    if (a.n > 0) disk_rays<<<(a.n + 255) / 256, 256, 0, st>>>(records, a.n, rays);
+    if (a.n > 0) disk_rays<<<steps, kStep, 0, st>>>(records, a.n, rays, counts);
     dim3 grid((a.width + 31) / 32, (a.height + 31) / 32);
     const bool big = (int64_t)grid.x * grid.y >= kBigTilesPerSm * ctx->sm_count;
     if (!big) grid = dim3((a.width + 15) / 16, (a.height + 15) / 16);
     const int64_t blocks = (int64_t)grid.x * grid.y, image = (int64_t)a.width * a.height;
     grid.z = (unsigned)std::max<int64_t>(
-        1, std::min({(kBlocksPerSm * ctx->sm_count + blocks - 1) / blocks, ((int64_t)a.n + kStep - 1) / kStep,
+        1, std::min({(kBlocksPerSm * ctx->sm_count + blocks - 1) / blocks, (int64_t)steps,
                      kPartialBytes / (image * 3 * (int64_t)sizeof(double))}));
     if (grid.z > 1)
         ARC_TRY(ctx->arena.get("disk_partial", (size_t)(image * 3 * grid.z) * sizeof(double),

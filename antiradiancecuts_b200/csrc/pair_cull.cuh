@@ -59,6 +59,15 @@ struct PixelBounds {
                 nmax[k] = fmaxf(nmax[k], __shfl_xor_sync(0xffffffffu, nmax[k], o));
             }
     }
+    __device__ __forceinline__ void reduce_warp_positions() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                pmin[k] = fminf(pmin[k], __shfl_xor_sync(0xffffffffu, pmin[k], o));
+                pmax[k] = fmaxf(pmax[k], __shfl_xor_sync(0xffffffffu, pmax[k], o));
+            }
+    }
     __device__ __forceinline__ void merge(const PixelBounds& b) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
