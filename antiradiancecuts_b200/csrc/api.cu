@@ -77,9 +77,9 @@ using namespace arc;
 namespace {
 
 arc_status check_device_errors(arc_context* ctx) {
-    uint32_t word = 0;
-    ARC_TRY_CUDA(cudaMemcpyAsync(&word, ctx->d_error, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    ARC_TRY_CUDA(cudaMemcpyAsync(ctx->h_error, ctx->d_error, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     ARC_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+    const uint32_t word = *ctx->h_error;
     if (word) {
         ARC_TRY_CUDA(cudaMemsetAsync(ctx->d_error, 0, sizeof(uint32_t), ctx->stream));
         char buf[128];
@@ -191,6 +191,7 @@ arc_status arc_context_create(int32_t device, void* cuda_stream, arc_context** o
     }
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_error, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_error, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_error, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_materials, sizeof(MaterialRecord) * ARC_MAX_MATERIALS);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_learned_rows, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_learned_rows, 0, sizeof(unsigned long long));
@@ -212,6 +213,7 @@ arc_status arc_context_destroy(arc_context* ctx) {
     for (auto e : ctx->timer.begin) cudaEventDestroy(e);
     for (auto e : ctx->timer.end) cudaEventDestroy(e);
     if (ctx->d_error) cudaFree(ctx->d_error);
+    if (ctx->h_error) cudaFreeHost(ctx->h_error);
     if (ctx->d_materials) cudaFree(ctx->d_materials);
     if (ctx->d_learned_rows) cudaFree(ctx->d_learned_rows);
     for (int i = 0; i < 2; ++i) {
@@ -226,9 +228,9 @@ arc_status arc_context_destroy(arc_context* ctx) {
 arc_status arc_context_synchronize(arc_context* ctx, uint32_t* device_error_word) {
     ARC_CHECK_ARG(ctx != nullptr, "ctx is NULL");
     ARC_TRY_CUDA(cudaSetDevice(ctx->device));
-    uint32_t word = 0;
-    ARC_TRY_CUDA(cudaMemcpyAsync(&word, ctx->d_error, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    ARC_TRY_CUDA(cudaMemcpyAsync(ctx->h_error, ctx->d_error, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     ARC_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+    const uint32_t word = *ctx->h_error;
     if (word) ARC_TRY_CUDA(cudaMemsetAsync(ctx->d_error, 0, sizeof(uint32_t), ctx->stream));
     if (device_error_word) *device_error_word = word;
     return ARC_OK;
@@ -362,7 +364,9 @@ arc_status arc_avpls_upload(arc_context* ctx, const ArcAvplHost* avpls, int32_t 
     ArcFloat3* hA = hL + n;
     int32_t* hm = reinterpret_cast<int32_t*>(hA + n);
     int32_t* hb = hm + n;
-#pragma omp parallel for schedule(static) if (n >= 65536)
+    // (serial, 32,768 AVPLs took 210 us, as long as the rest of a small frame; the whole team or one
+    // thread, because a smaller team makes the runtime drop the others and start them again later)
+#pragma omp parallel for schedule(static) if (n >= 8192)
     for (size_t i = 0; i < n; ++i) {
         hp[i] = avpls[i].position;
         hn[i] = avpls[i].normal;

@@ -113,6 +113,7 @@ struct arc_context {
     bool owns_stream = false;
     arc::Arena arena;
     uint32_t* d_error = nullptr;  // device error word (ARC_DEVERR_*)
+    uint32_t* h_error = nullptr;  // pinned: where it is read back
     // materials
     arc::MaterialRecord* d_materials = nullptr;
     int32_t num_materials = 0;
