@@ -212,7 +212,6 @@ struct LevelArgs {
     int2* accepted;         // {tile, node}
     int* acc_count;
     int acc_capacity;
-    int* tile_counts;
     float band;             // M > band * tau: refine without the network
     float clamp2, cos_thr;
     uint32_t* err;
@@ -280,9 +279,6 @@ __device__ __forceinline__ bool emit(const LevelArgs& a, int* se, bool ok, int a
             a.accepted[pos] = make_int2(tile, node);
         else
             set_error(a.err, ARC_DEVERR_CUT_OVERFLOW);
-        // one per-tile count update per group of lanes with the same tile
-        const unsigned grp = __match_any_sync(am, ok ? tile : -1 - lane);
-        if (ok && lane == __ffs(grp) - 1) atomicAdd(&a.tile_counts[tile], __popc(grp));
     } else if (action == kRefine) {
         // every reserved slot below the capacity is written; the rest do not exist (the next level
         // reads min(count, capacity) entries)
@@ -479,12 +475,10 @@ __global__ void accept_frontier(LevelArgs a) {
             continue;
         }
         const int pos = atomicAdd(a.acc_count, 1);
-        if ((unsigned)pos < (unsigned)a.acc_capacity) {
+        if ((unsigned)pos < (unsigned)a.acc_capacity)
             a.accepted[pos] = make_int2(en.x, en.y & ((1 << kDepthShift) - 1));
-            atomicAdd(&a.tile_counts[en.x], 1);
-        } else {
+        else
             set_error(a.err, ARC_DEVERR_CUT_OVERFLOW);
-        }
     }
 }
 
@@ -541,19 +535,21 @@ __global__ void tile_chunk_scan(const int* counts, int tiles, int* base, int* to
     if (threadIdx.x == 0) *total = carry;
 }
 
-struct ScatterArgs {
+struct ListArgs {
     const int2* accepted;
     const int* acc_count;
     int acc_capacity;
-    const int* tile_counts;
+    int tiles;
+    int slabs, groups, group_tiles;
+    int* slab_counts;  // slabs rows of one count per tile; after list_bases, the slab's first slot
+    int* tile_counts;
     const int* chunk_base;
-    int* fill;
     CutPool pool;
     const int* total_chunks;
     uint32_t* err;
 };
 
-__global__ void scatter_tables(ScatterArgs s, int tiles) {
+__global__ void scatter_tables(ListArgs s, int tiles) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= tiles) return;
     const int total = *s.total_chunks;
@@ -571,44 +567,93 @@ __global__ void scatter_tables(ScatterArgs s, int tiles) {
     s.pool.counts[t] = cnt;
 }
 
-// Each thread takes kScatterIlp pairs per trip (a warp reads 32 consecutive pairs for each), and
-// all their loads, then all their slot reservations, are issued before any result is used, so
-// that several global atomics per thread are in flight.  (blockDim a multiple of 32: every lane
-// of a warp takes the same loop trips.)
-constexpr int kScatterIlp = 4;
+// The accepted pairs, grouped by tile: the pairs are cut into slabs, one CTA counts a slab's pairs
+// per tile in shared memory (list_pass<false>), list_bases turns the counts of all slabs into the
+// first slot of every slab in every tile's list, and the second pass (list_pass<true>) hands the
+// slots out with shared atomics.  Tiles that do not fit one CTA's shared memory are split into
+// groups, and each group's CTA reads the whole slab.
+//
+// Bound by the scattered 4-byte stores (a sector each; a tile's consecutive entries come from
+// consecutive nodes), not by the slots: the first form (one global counter per tile, incremented by
+// learned_level and again by the scatter) took 14.4 ms here and 6 ms more in learned_level for the
+// 640M pairs of 1920x1080 x 1,048,576, and 230 us for 1,024 tiles, whose counters are 32 lines.
+// Now 10.3 ms (the counting pass 0.76 ms, 5 GB) and 200 us.  What matters is how many sectors are open
+// at once: one CTA per SM with 8 pairs per thread and trip 10.3 ms, two CTAs with 4 pairs 12.2 to
+// 14.9 ms; two slabs per SM 10.3 ms, a quarter as many 13.6 ms, eight times as many 10.9 ms.  Up to
+// kListGroups groups of about kListTiles tiles: 1 group 13.6 ms, 2: 10.7, 4: 10.3, 8: 12.2 (every
+// group reads all pairs); larger frames only take more groups where shared memory asks for it.
+constexpr int kListIlp = 8;
+constexpr int kListThreads = 1024;
+constexpr int kListTiles = 8192;
+constexpr int kListGroups = 4;
+constexpr int kListMaxTiles = 50176;  // 196 KB of shared memory
+constexpr int kListSlabsPerSm = 2;
 
-__global__ void scatter_nodes(ScatterArgs s) {
+template <bool SCATTER>
+__global__ void __launch_bounds__(kListThreads, 1) list_pass(ListArgs s) {
+    extern __shared__ int s_slot[];
+    const int t = threadIdx.x;
+    const int slab = blockIdx.x / s.groups, lo = (blockIdx.x % s.groups) * s.group_tiles;
+    const int width = min(s.group_tiles, s.tiles - lo);
+    int* row = s.slab_counts + (size_t)slab * s.tiles + lo;
+    for (int j = t; j < width; j += kListThreads) s_slot[j] = SCATTER ? row[j] : 0;
+    __syncthreads();
     // every reserved slot below the capacity was written; the counter may have wrapped past 2^31
-    const int count = (int)min((unsigned)*s.acc_count, (unsigned)s.acc_capacity);
-    const int lane = threadIdx.x & 31;
-    const int64_t trip = (int64_t)blockDim.x * kScatterIlp;
-    for (int64_t b = (int64_t)blockIdx.x * trip; b < count; b += (int64_t)gridDim.x * trip) {
-        int2 p[kScatterIlp];
-        bool valid[kScatterIlp];
+    const int64_t count = min((unsigned)*s.acc_count, (unsigned)s.acc_capacity);
+    const int64_t per = (count + s.slabs - 1) / s.slabs;
+    const int64_t last = min(count, (slab + 1) * per);
+    for (int64_t b = slab * per + t; b < last; b += kListThreads * kListIlp) {
+        int2 p[kListIlp];
+        int pos[kListIlp];
 #pragma unroll
-        for (int u = 0; u < kScatterIlp; ++u) {
-            const int64_t e = b + (int64_t)u * blockDim.x + threadIdx.x;
-            valid[u] = e < count;
-            p[u] = valid[u] ? s.accepted[e] : make_int2(-1 - lane, 0);
-        }
-        // lanes with the same tile take consecutive slots with one atomic
-        unsigned grp[kScatterIlp];
-        int base[kScatterIlp];
-#pragma unroll
-        for (int u = 0; u < kScatterIlp; ++u) {
-            grp[u] = __match_any_sync(0xffffffffu, p[u].x);
-            base[u] = 0;
-            if (valid[u] && lane == __ffs(grp[u]) - 1) base[u] = atomicAdd(&s.fill[p[u].x], __popc(grp[u]));
+        for (int u = 0; u < kListIlp; ++u) {
+            const int64_t e = b + u * kListThreads;
+            p[u] = e < last ? s.accepted[e] : make_int2(-1, 0);
         }
 #pragma unroll
-        for (int u = 0; u < kScatterIlp; ++u) {
-            base[u] = __shfl_sync(0xffffffffu, base[u], __ffs(grp[u]) - 1);
-            if (!valid[u]) continue;
-            const int pos = base[u] + __popc(grp[u] & ((1u << lane) - 1u));
-            const int id = s.chunk_base[p[u].x] + pos / kChunk;
-            if (pos / kChunk < s.pool.max_chunks && id < s.pool.num_chunks && pos < s.pool.counts[p[u].x])
-                s.pool.entries[(size_t)id * kChunk + pos % kChunk] = p[u].y;
+        for (int u = 0; u < kListIlp; ++u) {
+            const bool in = p[u].x >= lo && p[u].x < lo + width;
+            pos[u] = in ? atomicAdd(&s_slot[p[u].x - lo], 1) : -1;
         }
+        if (!SCATTER) continue;
+#pragma unroll
+        for (int u = 0; u < kListIlp; ++u) {
+            if (pos[u] < 0) continue;
+            const int id = s.chunk_base[p[u].x] + pos[u] / kChunk;
+            if (pos[u] / kChunk < s.pool.max_chunks && id < s.pool.num_chunks && pos[u] < s.pool.counts[p[u].x])
+                s.pool.entries[(size_t)id * kChunk + pos[u] % kChunk] = p[u].y;
+        }
+    }
+    if (SCATTER) return;
+    __syncthreads();
+    for (int j = t; j < width; j += kListThreads) row[j] = s_slot[j];
+}
+
+// Exclusive sums of every tile's counts over the slabs, in place, and the tile's total: 32 tiles per
+// block, the slabs split over its 8 warps.
+__global__ void __launch_bounds__(256) list_bases(ListArgs s) {
+    __shared__ int part[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tile = blockIdx.x * 32 + lane;
+    const int per = (s.slabs + 7) / 8;
+    const int first = min(w * per, s.slabs), last = min(first + per, s.slabs);
+    int sum = 0;
+    if (tile < s.tiles) {
+#pragma unroll 8
+        for (int i = first; i < last; ++i) sum += s.slab_counts[(size_t)i * s.tiles + tile];
+    }
+    part[w][lane] = sum;
+    __syncthreads();
+    if (tile >= s.tiles) return;
+    int base = 0;
+    for (int i = 0; i < w; ++i) base += part[i][lane];
+    if (w == 7) s.tile_counts[tile] = base + sum;
+#pragma unroll 8
+    for (int i = first; i < last; ++i) {
+        int* c = s.slab_counts + (size_t)i * s.tiles + tile;
+        const int x = *c;
+        *c = base;
+        base += x;
     }
 }
 
@@ -854,7 +899,7 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     const int acc_cap = (int)std::min<int64_t>((int64_t)pool.num_chunks * kChunk, (int64_t)INT32_MAX);
     int2 *fa, *fb;
     int2* accepted;
-    int *counters, *tile_counts, *chunk_base, *fill;
+    int *counters, *tile_counts, *chunk_base, *slab_counts;
     ARC_TRY(arena_get(ctx, "lc_front_a", cap, &fa));
     ARC_TRY(arena_get(ctx, "lc_front_b", cap, &fb));
     ARC_TRY(arena_get(ctx, "lc_accepted", acc_cap, &accepted));
@@ -868,10 +913,7 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     ARC_TRY(arena_get(ctx, "lc_counters", kSlots, &counters));
     ARC_TRY(arena_get(ctx, "lc_tile_counts", tiles, &tile_counts));
     ARC_TRY(arena_get(ctx, "lc_chunk_base", tiles, &chunk_base));
-    ARC_TRY(arena_get(ctx, "lc_fill", tiles, &fill));
     ARC_TRY_CUDA(cudaMemsetAsync(counters, 0, sizeof(int) * kSlots, st));
-    ARC_TRY_CUDA(cudaMemsetAsync(tile_counts, 0, sizeof(int) * tiles, st));
-    ARC_TRY_CUDA(cudaMemsetAsync(fill, 0, sizeof(int) * tiles, st));
 
     const float p = cp->mlp_threshold;
     LevelArgs la{};
@@ -897,7 +939,6 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     la.accepted = accepted;
     la.acc_count = counters + 3;
     la.acc_capacity = acc_cap;
-    la.tile_counts = tile_counts;
     la.band = cp->mlp_band > 0.0f ? cp->mlp_band : INFINITY;
     la.clamp2 = gp->dist_clamp > 0.0f ? gp->dist_clamp * gp->dist_clamp : 0.0f;
     la.cos_thr = fmaxf(cosf(gp->cone_half_angle), 0.001f);
@@ -947,20 +988,34 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     // the accepted pairs grouped by tile into the cut pool, timed as a stage of its own
     stage_begin(ctx, "cut_lists");
     kernels = 0;
-    ScatterArgs sa;
+    ListArgs sa{};
     sa.accepted = accepted;
     sa.acc_count = counters + 3;
     sa.acc_capacity = acc_cap;
+    sa.tiles = tiles;
+    sa.groups = std::max((tiles + kListMaxTiles - 1) / kListMaxTiles,
+                         std::min((tiles + kListTiles - 1) / kListTiles, kListGroups));
+    sa.group_tiles = (tiles + sa.groups - 1) / sa.groups;
+    sa.slabs = ctx->sm_count * kListSlabsPerSm;
+    const size_t list_smem = sizeof(int) * (size_t)sa.group_tiles;
+    ARC_TRY(arena_get(ctx, "lc_slab_counts", (size_t)sa.slabs * tiles, &slab_counts));
+    sa.slab_counts = slab_counts;
     sa.tile_counts = tile_counts;
     sa.chunk_base = chunk_base;
-    sa.fill = fill;
     sa.pool = pool;
     sa.total_chunks = counters + 4;
     sa.err = ctx->d_error;
+    ARC_TRY_CUDA(cudaFuncSetAttribute(list_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(sizeof(int) * kListMaxTiles)));
+    ARC_TRY_CUDA(cudaFuncSetAttribute(list_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(sizeof(int) * kListMaxTiles)));
+    const int list_grid = sa.slabs * sa.groups;
+    list_pass<false><<<list_grid, kListThreads, list_smem, st>>>(sa);
+    list_bases<<<(tiles + 31) / 32, 256, 0, st>>>(sa);
     tile_chunk_scan<<<1, 1024, 0, st>>>(tile_counts, tiles, chunk_base, counters + 4, pool.max_chunks, ctx->d_error);
     scatter_tables<<<(tiles + 255) / 256, 256, 0, st>>>(sa, tiles);
-    scatter_nodes<<<grid, 256, 0, st>>>(sa);
-    kernels += 3;
+    list_pass<true><<<list_grid, kListThreads, list_smem, st>>>(sa);
+    kernels += 5;
     ARC_TRY_CUDA(cudaMemcpyAsync(pool.next, counters + 4, sizeof(int), cudaMemcpyDeviceToDevice, st));
     stage_end(ctx, kernels);
     ARC_TRY_CUDA(cudaGetLastError());
