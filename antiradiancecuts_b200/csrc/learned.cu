@@ -577,12 +577,13 @@ __global__ void scatter_tables(ListArgs s, int tiles) {
 // consecutive nodes), not by the slots: the first form (one global counter per tile, incremented by
 // learned_level and again by the scatter) took 14.4 ms here and 6 ms more in learned_level for the
 // 640M pairs of 1920x1080 x 1,048,576, and 230 us for 1,024 tiles, whose counters are 32 lines.
-// Now 10.3 ms (the counting pass 0.76 ms, 5 GB) and 200 us.  What matters is how many sectors are open
-// at once: one CTA per SM with 8 pairs per thread and trip 10.3 ms, two CTAs with 4 pairs 12.2 to
-// 14.9 ms; two slabs per SM 10.3 ms, a quarter as many 13.6 ms, eight times as many 10.9 ms.  Up to
-// kListGroups groups of about kListTiles tiles: 1 group 13.6 ms, 2: 10.7, 4: 10.3, 8: 12.2 (every
-// group reads all pairs); larger frames only take more groups where shared memory asks for it.
-constexpr int kListIlp = 8;
+// Now 9.9 ms (the counting pass 0.76 ms, 5 GB) and 200 us.  What matters is how many sectors are open
+// at once (figures with the counting pass in as many groups, 1.5 ms in 4): one CTA per SM with 8 pairs
+// per thread and trip 10.3 ms, two CTAs with 4 pairs 12.2 to
+// 14.9 ms; two slabs per SM 10.3 ms, a quarter as many 13.6 ms, eight times as many 10.9 ms.  The
+// scatter takes up to kListGroups groups of about kListTiles tiles: 1 group 13.6 ms, 2: 10.7, 4: 10.3,
+// 8: 12.2 (every group reads all pairs); larger frames only take more groups where shared memory asks
+// for it.  The counting pass stores nothing per pair: as few groups as fit (1: 0.76 ms, 4: 1.5 ms).
 constexpr int kListThreads = 1024;
 constexpr int kListTiles = 8192;
 constexpr int kListGroups = 4;
@@ -590,7 +591,8 @@ constexpr int kListMaxTiles = 50176;  // 196 KB of shared memory
 constexpr int kListSlabsPerSm = 2;
 
 template <bool SCATTER>
-__global__ void __launch_bounds__(kListThreads, 1) list_pass(ListArgs s) {
+__global__ void __launch_bounds__(kListThreads, SCATTER ? 1 : 2) list_pass(ListArgs s) {
+    constexpr int kListIlp = SCATTER ? 8 : 4;
     extern __shared__ int s_slot[];
     const int t = threadIdx.x;
     const int slab = blockIdx.x / s.groups, lo = (blockIdx.x % s.groups) * s.group_tiles;
@@ -993,11 +995,7 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     sa.acc_count = counters + 3;
     sa.acc_capacity = acc_cap;
     sa.tiles = tiles;
-    sa.groups = std::max((tiles + kListMaxTiles - 1) / kListMaxTiles,
-                         std::min((tiles + kListTiles - 1) / kListTiles, kListGroups));
-    sa.group_tiles = (tiles + sa.groups - 1) / sa.groups;
     sa.slabs = ctx->sm_count * kListSlabsPerSm;
-    const size_t list_smem = sizeof(int) * (size_t)sa.group_tiles;
     ARC_TRY(arena_get(ctx, "lc_slab_counts", (size_t)sa.slabs * tiles, &slab_counts));
     sa.slab_counts = slab_counts;
     sa.tile_counts = tile_counts;
@@ -1009,12 +1007,19 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
                                       (int)(sizeof(int) * kListMaxTiles)));
     ARC_TRY_CUDA(cudaFuncSetAttribute(list_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(sizeof(int) * kListMaxTiles)));
-    const int list_grid = sa.slabs * sa.groups;
-    list_pass<false><<<list_grid, kListThreads, list_smem, st>>>(sa);
+    const auto split = [&](int groups) {
+        sa.groups = groups;
+        sa.group_tiles = (tiles + groups - 1) / groups;
+        return sizeof(int) * (size_t)sa.group_tiles;
+    };
+    const int min_groups = (tiles + kListMaxTiles - 1) / kListMaxTiles;
+    size_t list_smem = split(min_groups);
+    list_pass<false><<<sa.slabs * sa.groups, kListThreads, list_smem, st>>>(sa);
     list_bases<<<(tiles + 31) / 32, 256, 0, st>>>(sa);
     tile_chunk_scan<<<1, 1024, 0, st>>>(tile_counts, tiles, chunk_base, counters + 4, pool.max_chunks, ctx->d_error);
     scatter_tables<<<(tiles + 255) / 256, 256, 0, st>>>(sa, tiles);
-    list_pass<true><<<list_grid, kListThreads, list_smem, st>>>(sa);
+    list_smem = split(std::max(min_groups, std::min((tiles + kListTiles - 1) / kListTiles, kListGroups)));
+    list_pass<true><<<sa.slabs * sa.groups, kListThreads, list_smem, st>>>(sa);
     kernels += 5;
     ARC_TRY_CUDA(cudaMemcpyAsync(pool.next, counters + 4, sizeof(int), cudaMemcpyDeviceToDevice, st));
     stage_end(ctx, kernels);
