@@ -124,19 +124,9 @@ __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
     const int rows = kThreads / kTileW;  // 16
     const int ybase = blockIdx.y * rows * PX + ty;
 
-    const int nchunks = (k.n + k.chunk - 1) / k.chunk;
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-        for (int c = 0; c < kStages && c < nchunks; ++c) {
-            const int cnt = min(k.chunk, k.n - c * k.chunk);
-            mbar_arrive_expect_tx(&bars[c], (uint32_t)cnt * 64u);
-            bulk_g2s(stage + (size_t)c * k.chunk * 4, k.records + (size_t)c * k.chunk * 4, (uint32_t)cnt * 64u,
-                     &bars[c]);
-        }
     }
 
     Pixel<T> pix[PX];
@@ -177,6 +167,23 @@ __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
         for (int c = 0; c < 6; ++c) sc[j][c] = ss[j][c] = 0.0f;
     }
 
+    // A warp without a surface pixel skips the pairs, a block without one the records as well (known
+    // before the first copy, so that none is in flight when it ends): 960 x 540 x 131,072, half of it
+    // background, per-term Kahan 129.5 -> 75.1 ms, naive 91.7 -> 51.8 ms, the same sums.
+    bool live = false;
+#pragma unroll
+    for (int j = 0; j < PX; ++j) live |= valid[j];
+    live = __any_sync(0xffffffffu, live);
+    const int nchunks = __syncthreads_or(live) ? (k.n + k.chunk - 1) / k.chunk : 0;
+    if (tid == 0) {
+        for (int c = 0; c < kStages && c < nchunks; ++c) {
+            const int cnt = min(k.chunk, k.n - c * k.chunk);
+            mbar_arrive_expect_tx(&bars[c], (uint32_t)cnt * 64u);
+            bulk_g2s(stage + (size_t)c * k.chunk * 4, k.records + (size_t)c * k.chunk * 4, (uint32_t)cnt * 64u,
+                     &bars[c]);
+        }
+    }
+
     bool ok = true;
     int fail_c = -1;  // first chunk whose wait gave up
     for (int c = 0; c < nchunks; ++c) {
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) gather_bf_kernel(BfArgs k) {
             ok = mbar_wait_bounded(&bars[s], parity, k.err);
             if (!ok) fail_c = c;
         }
-        if (ok) {
+        if (ok && live) {
             const int cnt = min(k.chunk, k.n - c * k.chunk);
             const float4* rec = stage + (size_t)s * k.chunk * 4;
 #pragma unroll 2
