@@ -1,6 +1,7 @@
 // Cut gathers over the LBVH.
 //
-// ARC_CUT_SOLID_ANGLE: the lightcut of kernel_bvh (cudaGather.cu:316-444), one thread per pixel:
+// ARC_CUT_SOLID_ANGLE: the lightcut of kernel_bvh (cudaGather.cu:316-444), one thread per pixel, a
+//   warp sharing the walk:
 //   DFS from the root; a leaf adds its exact radiance; an inner node is skipped when both of its
 //   box corners lie behind the receiver (cudaGather.cu:405-408), used whole when the solid angle
 //   2 pi (1 - d / sqrt(r^2 + d^2)) of its bounding sphere seen from the representative is below
@@ -8,8 +9,8 @@
 //   overflows for large trees); overflow paints the reference's magenta pixel and sets
 //   ARC_DEVERR_STACK_OVERFLOW.  Antiradiance comes from the brute-force pass, as in the
 //   reference's non-clustered run() path.
-// ARC_CUT_ERROR_BOUND: one cut per 8x8 pixel tile, chosen by one warp that walks the tree
-//   cooperatively (32 nodes per step, ballot/popc compaction of accepted nodes and of the
+// ARC_CUT_ERROR_BOUND: one cut per 8x8 pixel tile, chosen by one block that walks the tree
+//   cooperatively (128 nodes per step, ballot/popc compaction of accepted nodes and of the
 //   children to push).  A node is refined while an upper bound of its contribution to any pixel
 //   of the tile exceeds eps times the tile's coarse radiance estimate.  Every pixel of the tile
 //   then evaluates the same node list, so the evaluation is fully coherent.
