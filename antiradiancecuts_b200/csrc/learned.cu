@@ -589,6 +589,7 @@ constexpr int kListTiles = 8192;
 constexpr int kListGroups = 4;
 constexpr int kListMaxTiles = 50176;  // 196 KB of shared memory
 constexpr int kListSlabsPerSm = 2;
+constexpr int64_t kListCounts = (int64_t)1 << 26;  // counts of all slabs, 256 MB: fewer slabs above 226,719 tiles
 
 template <bool SCATTER>
 __global__ void __launch_bounds__(kListThreads, SCATTER ? 1 : 2) list_pass(ListArgs s) {
@@ -995,7 +996,7 @@ arc_status launch_cut_select_learned(arc_context* ctx, const arc_lbvh* bvh, cons
     sa.acc_count = counters + 3;
     sa.acc_capacity = acc_cap;
     sa.tiles = tiles;
-    sa.slabs = ctx->sm_count * kListSlabsPerSm;
+    sa.slabs = (int)std::max<int64_t>(1, std::min<int64_t>(ctx->sm_count * kListSlabsPerSm, kListCounts / tiles));
     ARC_TRY(arena_get(ctx, "lc_slab_counts", (size_t)sa.slabs * tiles, &slab_counts));
     sa.slab_counts = slab_counts;
     sa.tile_counts = tile_counts;
