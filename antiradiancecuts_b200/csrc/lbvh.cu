@@ -454,10 +454,12 @@ struct BlockArgs {
     ArcFloat3* sorted_pos;
     ArcFloat3* sorted_nrm;
     // the nodes that reach over a block's leaves, and the nodes below them
-    float4* state;         // [2N-1][8]: NodeState of a block's roots and of the nodes above them
-    int32_t* visit;        // [N-1] arrivals
+    float4* state;         // [cap][8]: NodeState of the blocks' roots from the front, of the top nodes from the end
+    int32_t cap;           // >= roots + top nodes
+    int32_t* visit;        // [N-1] of a top node: 1 + the state of the child that arrived first
     int32_t* roots;        // record indices of every block's roots
     int32_t* top;          // inner nodes above them
+    int32_t* top_slot;     // [N-1] of a top node: its place in top
     int32_t* counts;       // roots, top nodes
 };
 
@@ -816,27 +818,49 @@ __global__ void __launch_bounds__(kBlockLeaves) lbvh_blocks(BlockArgs b) {
     __syncthreads();
     if (j < 2) s_base[j] = atomicAdd(&b.counts[j], s_count[j]);
     __syncthreads();
+    // (all within cap in a valid tree, see state_capacity)
+    bool fits = true;
     if (leaf_root) {
-        b.roots[s_base[0] + slot[0]] = i;
-        store_state(b.state, i, get(j));
+        const int q = s_base[0] + slot[0];
+        fits = q < b.cap;
+        if (fits) {
+            b.roots[q] = i;
+            store_state(b.state, q, get(j));
+        }
     }
     if (node_root) {
-        b.roots[s_base[0] + slot[1]] = n + i;
-        store_state(b.state, n + i, s);
+        const int q = s_base[0] + slot[1];
+        fits = fits && q < b.cap;
+        if (q < b.cap) {
+            b.roots[q] = n + i;
+            store_state(b.state, q, s);
+        }
     }
     if (above) {
-        b.top[s_base[1] + slot[2]] = i;
+        const int q = s_base[1] + slot[2];
+        fits = fits && q < b.cap;
+        if (q < b.cap) b.top[q] = i;
+        b.top_slot[i] = q;
         b.visit[i] = 0;
     }
+    if (!fits) set_error(b.err, ARC_DEVERR_BAD_NODE);
+}
+
+// States that a tree of `blocks` blocks keeps: a node over a boundary between two blocks is one of a chain of at
+// most kMaxHeight such nodes, T of them in all; they have T + 1 roots below them.  (126 B per leaf; a state
+// for every node would take 256.)
+inline int32_t state_capacity(int32_t n, int blocks) {
+    return (int32_t)std::min<int64_t>(2 * (int64_t)n - 1, 2 * (int64_t)kMaxHeight * (blocks - 1) + 1);
 }
 
 // From every block root towards the tree's root: at each inner node above the blocks the first thread to
-// arrive stops and the second merges the two children's states.
+// arrive leaves its state's place and stops, and the second merges the two states.
 __global__ void __launch_bounds__(128) lbvh_climb(BlockArgs b) {
     if (*b.abort != 0u) return;
-    const int n = b.n, roots = b.counts[0];
+    const int n = b.n, roots = min(b.counts[0], b.cap);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < roots; q += gridDim.x * blockDim.x) {
-        int parent = b.parents[b.roots[q]];
+        int node = b.roots[q], own = q;
+        int parent = b.parents[node];
         // a valid tree reaches the root within n - 1 steps; the bound guards against a corrupt one
         for (int steps = 0; parent >= 0; ++steps) {
             if (steps >= n || parent >= n - 1) {
@@ -844,19 +868,27 @@ __global__ void __launch_bounds__(128) lbvh_climb(BlockArgs b) {
                 break;
             }
             const int k = parent;
-            const int lc = b.left[k], rc = b.right[k];
+            const int lc = b.left[k], slot = b.top_slot[k];
             parent = b.parents[n + k];
             __threadfence();  // release this thread's state of the child
-            if (atomicAdd(&b.visit[k], 1) == 0) break;
+            const int other = atomicExch(&b.visit[k], own + 1) - 1;
+            if (other < 0) break;
             __threadfence();  // acquire the sibling's
-            const NodeState l = load_state(b.state, lc >= 0 ? lc : n - (lc + 1)),
-                            r = load_state(b.state, rc >= 0 ? rc : n - (rc + 1));
+            if (other >= b.cap || (unsigned)slot >= (unsigned)b.cap) {
+                set_error(b.err, ARC_DEVERR_BAD_NODE);
+                break;
+            }
+            const bool is_left = (lc >= 0 ? lc : n - (lc + 1)) == node;
+            const NodeState l = load_state(b.state, is_left ? own : other),
+                            r = load_state(b.state, is_left ? other : own);
             float rnd;
             NodeState o;
             merge_sums(o, l, r, b.seed, n + k, &rnd);
             o.cn = cone_union(l.cn, r.cn);
             o.cw = cone_union(l.cw, r.cw);
-            store_state(b.state, n + k, o);
+            node = n + k;
+            own = b.cap - 1 - slot;
+            store_state(b.state, own, o);
         }
     }
 }
@@ -864,10 +896,10 @@ __global__ void __launch_bounds__(128) lbvh_climb(BlockArgs b) {
 // Outputs of the nodes above the blocks, one thread each.
 __global__ void __launch_bounds__(128) lbvh_top_nodes(BlockArgs b) {
     if (*b.abort != 0u) return;
-    const int n = b.n, count = b.counts[1];
+    const int n = b.n, count = min(b.counts[1], b.cap);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
         const int k = b.top[q];
-        const NodeState s = load_state(b.state, n + k);
+        const NodeState s = load_state(b.state, b.cap - 1 - q);
         const float4* r = b.records + 4 * (size_t)s.rep;
         const float4* ra = b.records + 4 * (size_t)s.arep;
         const float4 q0 = r[0], q1 = r[1], a1 = ra[1];
@@ -932,12 +964,15 @@ arc_status launch_lbvh_build(arc_lbvh* bvh, const ArcAvplsGpuParam* avpls, const
     ARC_TRY(get(bvh, "parents", total, &parents));
     ARC_TRY(get(bvh, "range", 2 * (n - 1), &range));
     ARC_TRY(get(bvh, "visit", n - 1, &bu.visit));
-    ARC_TRY(get(bvh, "roots", total, &bu.roots));
-    ARC_TRY(get(bvh, "top", n - 1, &bu.top));
+    const int blocks = (n + kBlockLeaves - 1) / kBlockLeaves;
+    bu.cap = state_capacity(n, blocks);
+    ARC_TRY(get(bvh, "roots", bu.cap, &bu.roots));
+    ARC_TRY(get(bvh, "top", bu.cap, &bu.top));
+    ARC_TRY(get(bvh, "top_slot", n - 1, &bu.top_slot));
     ARC_TRY(get(bvh, "records", (size_t)4 * total, &records));
     ARC_TRY(get(bvh, "dirstat", total, &dirstat));
     ARC_TRY(get(bvh, "bounds", (size_t)4 * (n - 1), &bounds));
-    ARC_TRY(get(bvh, "state", (size_t)8 * total, &bu.state));
+    ARC_TRY(get(bvh, "state", (size_t)8 * bu.cap, &bu.state));
     ArcAvplBvhNodeDataParam nd;
     ARC_TRY(get(bvh, "nd_size", total, &nd.size));
     ARC_TRY(get(bvh, "nd_mat", total, &nd.materialIndex));
@@ -1040,11 +1075,10 @@ arc_status launch_lbvh_build(arc_lbvh* bvh, const ArcAvplsGpuParam* avpls, const
     bu.sorted_pos = bvh->sorted_positions;
     bu.sorted_nrm = bvh->sorted_normals;
     stage_begin(ctx, "lbvh_bottom_up");
-    const int blocks = (n + kBlockLeaves - 1) / kBlockLeaves;
     ARC_TRY_CUDA(cudaFuncSetAttribute(lbvh_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockSmem));
     lbvh_blocks<<<blocks, kBlockLeaves, kBlockSmem, st>>>(bu);
-    // One block settles its whole tree: nothing is left to climb (128 leaves 67 us, 129 with the two
-    // launches 92 us).
+    // One block settles its whole tree: nothing is left to climb (128 leaves 64 us, 129 with the two
+    // launches 90 us).
     if (blocks > 1) {
         // (a block has about ten roots)
         const int top_blocks = std::min(blocks, ctx->sm_count * 8);
