@@ -576,14 +576,14 @@ __global__ void scatter_tables(ListArgs s, int tiles) {
 // Bound by the scattered 4-byte stores (a sector each; a tile's consecutive entries come from
 // consecutive nodes), not by the slots: the first form (one global counter per tile, incremented by
 // learned_level and again by the scatter) took 14.4 ms here and 6 ms more in learned_level for the
-// 640M pairs of 1920x1080 x 1,048,576, and 230 us for 1,024 tiles, whose counters are 32 lines.
-// Now 9.9 ms (the counting pass 0.76 ms, 5 GB) and 200 us.  What matters is how many sectors are open
-// at once (figures with the counting pass in as many groups, 1.5 ms in 4): one CTA per SM with 8 pairs
-// per thread and trip 10.3 ms, two CTAs with 4 pairs 12.2 to
-// 14.9 ms; two slabs per SM 10.3 ms, a quarter as many 13.6 ms, eight times as many 10.9 ms.  The
-// scatter takes up to kListGroups groups of about kListTiles tiles: 1 group 13.6 ms, 2: 10.7, 4: 10.3,
-// 8: 12.2 (every group reads all pairs); larger frames only take more groups where shared memory asks
-// for it.  The counting pass stores nothing per pair: as few groups as fit (1: 0.76 ms, 4: 1.5 ms).
+// 640M pairs of 1920x1080 x 1,048,576, and 210 us for 1,024 tiles.  Now 9.9 ms (the counting pass 0.76 ms,
+// 5 GB) and 198 us.  What matters is how many sectors are open at once (the figures below with the
+// counting pass in as many groups as the scatter, 1.5 ms in 4).  One CTA per SM with 8 pairs per thread and
+// trip: 10.3 ms, two CTAs with 4 pairs 12.2 to 15.5 ms.  In 4 groups 37 slabs 13.6 ms, 74: 12.5, 148: 10.9,
+// 296 (two per SM): 10.3, 592: 10.5, 1,184: 10.9.  With 8 blocks per SM 1 group 13.6 ms, 2: 10.7, 4: 10.3,
+// 8: 12.2 (every group reads all pairs), so the scatter takes up to kListGroups groups of about kListTiles
+// tiles, and more only where shared memory asks for it.  The counting pass stores nothing per pair: as
+// few groups as fit (1: 0.76 ms, 4: 1.5 ms).
 constexpr int kListThreads = 1024;
 constexpr int kListTiles = 8192;
 constexpr int kListGroups = 4;
