@@ -106,8 +106,9 @@ __global__ void __launch_bounds__(kStep) disk_rays(const float4* records, int n,
     }
 }
 
-// Whether the ray from r0 along the unit vector r1 can pass within `radius` of a point of the sphere
-// (c, rho); the margin covers the rounding of the hit point in pair_terms (a few ulp of the distance).
+// Whether the ray from r0 along the unit vector r1 can enter the sphere (c, rho); the margin covers the
+// rounding of the hit point here and in pair_terms, which both start from a difference of positions (a
+// few ulp of the distance).
 __device__ __forceinline__ bool ray_near(float4 r0, float4 r1, float cx, float cy, float cz, float rho) {
     const float vx = cx - r0.x, vy = cy - r0.y, vz = cz - r0.z;
     const float s = fmaxf(0.0f, vx * r1.x + vy * r1.y + vz * r1.z);
@@ -186,12 +187,15 @@ __global__ void __launch_bounds__(kThreads, PX == 1 ? 3 : 2) disk_antiradiance(D
         __syncthreads();
         PixelBounds tb = s_box[0];
         for (int q = 1; q < kWarps; ++q) tb.merge(s_box[q]);
-        // bounding sphere of a box, grown by the disk radius (radius -1: empty)
+        // bounding sphere of a box, grown by the disk radius (radius -1: empty).  The half extents are taken
+        // from the centre as it is rounded, which far from the origin is off by more than the disk radius.
         auto sphere = [&](const PixelBounds& b) {
-            const float ex = b.pmax[0] - b.pmin[0], ey = b.pmax[1] - b.pmin[1], ez = b.pmax[2] - b.pmin[2];
-            return make_float4(0.5f * (b.pmin[0] + b.pmax[0]), 0.5f * (b.pmin[1] + b.pmax[1]),
-                               0.5f * (b.pmin[2] + b.pmax[2]),
-                               b.pmin[0] <= b.pmax[0] ? 0.5001f * sqrtf(ex * ex + ey * ey + ez * ez) + a.radius : -1.0f);
+            const float cx = 0.5f * (b.pmin[0] + b.pmax[0]), cy = 0.5f * (b.pmin[1] + b.pmax[1]),
+                        cz = 0.5f * (b.pmin[2] + b.pmax[2]);
+            const float ex = fmaxf(b.pmax[0] - cx, cx - b.pmin[0]), ey = fmaxf(b.pmax[1] - cy, cy - b.pmin[1]),
+                        ez = fmaxf(b.pmax[2] - cz, cz - b.pmin[2]);
+            return make_float4(cx, cy, cz,
+                               b.pmin[0] <= b.pmax[0] ? 1.0001f * sqrtf(ex * ex + ey * ey + ez * ez) + a.radius : -1.0f);
         };
         // the warp's pixels on one side of the middle of a box's longest axis
         auto half = [&](const PixelBounds& whole, int side) {
