@@ -553,12 +553,11 @@ __global__ void __launch_bounds__(kThreads, PX <= 2 ? 3 : 1) gather_bf_culled_ke
                             const T a = (nx_[j] * dx + ny_[j] * dy + nz_[j] * dz) * r;
                             const T cw = -(d[3] * dx + d[4] * dy + d[5] * dz) * r;
                             const T rr = r * r;
-                            if (cw > (T)cos_thr && a > (T)eps) {
-                                const T ga = a * (rr < clampi ? rr : clampi);
-                                sum[j][3] += d[6] * ga;
-                                sum[j][4] += d[7] * ga;
-                                sum[j][5] += d[8] * ga;
-                            }
+                            // (outside the cone 0 times the antiradiance is added: it may not be finite)
+                            const T ga = cw > (T)cos_thr && a > (T)eps ? a * (rr < clampi ? rr : clampi) : (T)0;
+                            sum[j][3] += d[6] * ga;
+                            sum[j][4] += d[7] * ga;
+                            sum[j][5] += d[8] * ga;
                         }
                     }
                 }
