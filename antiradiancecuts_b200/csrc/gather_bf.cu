@@ -789,11 +789,25 @@ constexpr int kBlocksPerSm = 24;
 constexpr int kMinChunks = 2;
 constexpr int64_t kPartialBytes = (int64_t)1 << 30;
 
+// The most records per stage of the tile shapes with PX pixels per thread.  A kernel's limit of dynamic
+// shared memory belongs to the device: it is set to what the largest of its shapes needs, the same value
+// from every call, so that a call of another context or thread cannot lower it before this one's launch.
+template <int PX>
+constexpr int max_chunk() {
+    int most = 0;
+    for (const TileShape& t : kTileShapes)
+        if (t.px == PX && t.chunk > most) most = t.chunk;
+    return most;
+}
+
+constexpr int fast_smem(int chunk) { return kStages * chunk * 64 + kStages * (int)sizeof(uint64_t); }
+
 template <int AR, int PREC, int PX>
 arc_status launch_fast(const BfArgs& a, cudaStream_t st) {
-    const size_t smem = (size_t)kStages * a.chunk * 64 + kStages * sizeof(uint64_t);
+    const int smem = fast_smem(a.chunk);
     auto fn = gather_bf_kernel<AR, PREC, PX>;
-    if (smem > 48 * 1024) ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024)
+        ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, fast_smem(max_chunk<PX>())));
     dim3 grid((a.width + kTileW - 1) / kTileW, (a.height + 16 * PX - 1) / (16 * PX));
     fn<<<grid, kThreads, smem, st>>>(a);
     ARC_TRY_CUDA(cudaGetLastError());
@@ -820,7 +834,8 @@ template <int AR, typename T, int PX, bool RAD>
 arc_status launch_culled_kernel(const BfArgs& a, int segments, cudaStream_t st) {
     const int smem = culled_smem<T, PX>(a.chunk);
     auto fn = gather_bf_culled_kernel<AR, T, PX, RAD>;
-    ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    constexpr int most = culled_smem<T, PX>(sizeof(T) == 8 ? kFp64Chunk : max_chunk<PX>());
+    ARC_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     dim3 grid = tile_grid(a, PX);
     grid.z = (unsigned)segments;
     fn<<<grid, kThreads, smem, st>>>(a);
