@@ -27,11 +27,11 @@ __device__ __forceinline__ float rn_sqrt_z(float a) {
     const float r = __fsqrt_rn(a == 0.0f ? 1.0f : a);
     return a == 0.0f ? a : r;
 }
-// a / b for a >= 0, b >= 0 (0 / 0 is not a number)
+// a / b for a >= 0, b >= 0 and what is not a number (0 / 0 is not a number, nor is 0 by one)
 __device__ __forceinline__ float rn_div_z(float a, float b) {
     const bool zero = a == 0.0f || b == 0.0f;
     const float r = __fdiv_rn(zero ? 1.0f : a, zero ? 1.0f : b);
-    return !zero ? r : b != 0.0f ? a : a != 0.0f ? __int_as_float(0x7f800000) : __int_as_float(0x7fffffff);
+    return !zero ? r : b > 0.0f ? a : a > 0.0f ? __int_as_float(0x7f800000) : __int_as_float(0x7fffffff);
 }
 __device__ __forceinline__ float rn_dot(float ax, float ay, float az, float bx, float by, float bz) {
     return rn_add(rn_add(rn_mul(ax, bx), rn_mul(ay, by)), rn_mul(az, bz));
