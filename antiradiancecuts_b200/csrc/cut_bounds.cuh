@@ -286,16 +286,21 @@ __device__ __forceinline__ FastBound node_bound_fast(const TileInfo& t, float4 b
     }
     float id2;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(id2) : "f"(g.d2c));
-    float m = ne.Ls * (g.cos1 * g.cos2) * id2;
-    float e = ne.Ls * (g.cos1 + g.cos2 + kCosErr) * id2;
+    // (the sums and the caller's factor may be negative, and the two terms may cancel: the radius takes
+    // magnitudes)
+    const float Ls = fabsf(ne.Ls), As = fabsf(ne.As);
+    float m = ne.Ls * (g.cos1 * g.cos2) * id2, a = Ls * (g.cos1 * g.cos2) * id2;
+    float e = Ls * (g.cos1 + g.cos2 + kCosErr) * id2;
     if (bp.ar_kind == ARC_AR_CONE) {
         m += ne.As * (g.ar_ok * g.cos1) * id2;
-        e += ne.As * g.ar_ok * id2;
+        a += As * fabsf(g.ar_ok * g.cos1) * id2;
+        e += As * fabsf(g.ar_ok) * id2;
     } else if (bp.ar_kind == ARC_AR_DISK) {
         m += ne.As * bp.disk_scale;
+        a += As * bp.disk_scale;
     }
     f.m = t.kdl * m;
-    f.err = t.kdl * (kCosErr * e) + 1e-5f * f.m;
+    f.err = t.kdl * (kCosErr * e + 1e-5f * a);
     return f;
 }
 
