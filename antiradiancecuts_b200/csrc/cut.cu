@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(kSolidThreads) cut_solid_angle_kernel(SolidArg
         const float kd[3] = {kOneOverPi * d.x, kOneOverPi * d.y, kOneOverPi * d.z};
         for (int q = 0; q < 3; ++q) r[q] = surface ? r[q] * (double)kd[q] : 0.0;
     }
-    if (failed >> lane & 1u) {
+    // (a walk whose budget ran out was its warp's: what its other pixels still had to visit is not known)
+    if ((failed >> lane & 1u) || (surface && budget < 0)) {
         r[0] = 100000.0;
         r[1] = 0.0;
         r[2] = 100000.0;
