@@ -12,8 +12,9 @@
 //   * The default and the all-FP64 precision (no or cone antiradiance) test each staged record once
 //     against the tile's bounds and evaluate only the records that can add something to it
 //     (gather_bf_culled_kernel, pair_cull.cuh), and the default precision's disk antiradiance is a
-//     culled pass of its own (disk_ar.cu); the other precisions, and every disk gather of the
-//     allocation-free entry point, evaluate every pair (gather_bf_kernel).
+//     culled pass of its own (disk_ar.cu); the other precisions, every disk gather of the
+//     allocation-free entry point, and gathers of few AVPLs (few_avpls) evaluate every pair
+//     (gather_bf_kernel).
 //   * Radiance and antiradiance go to separate compensated sums (per-chunk FP32 partials folded
 //     into Kahan sums, or per-term Kahan) and are combined in FP64.
 // General path (specular materials or geometry-term limits): one thread per pixel evaluating the
@@ -902,9 +903,21 @@ arc_status launch_fast_px(const BfArgs& a, int px, cudaStream_t st) {
     return launch_fast<AR, PREC, 4>(a, st);
 }
 
+// Few AVPLs: one launch of the kernel that evaluates every pair takes less than the culled kernel's
+// barriers and list tests (all FP64), or than the culled radiance, disk pass and combination (default
+// precision, disk).  Microseconds, culled / every pair:
+//   disk    1 x 1 x 1: 41 / 17, 192 x 192 x 64: 44 / 41, 512 x 512 x 16: 67 / 32, 1920 x 1080 x 16: 201 / 105
+//   FP64    1 x 1 x 1: 25 / 16, 192 x 192 x 64: 30 / 30, 512 x 512 x 16: 49 / 37, 1920 x 1080 x 16: 166 / 128
+// and beyond the line culled is ahead: 512 x 512 x 128 84 / 131 and 97 / 176, 1920 x 1080 x 64 217 / 438 and
+// 228 / 647.
+bool few_avpls(int n, int64_t pixels) {
+    return n <= 16 || (n <= 64 && n * pixels <= (int64_t)1 << 23);
+}
+
 // the culled kernel serves the default and the all-FP64 precision with no or cone antiradiance
-bool use_culled(const ArcGatherParams& p) {
-    return p.ar_kind != ARC_AR_DISK && (p.precision == ARC_PREC_KAHAN || p.precision == ARC_PREC_FP64);
+bool use_culled(const ArcGatherParams& p, int n, int64_t pixels) {
+    if (p.ar_kind == ARC_AR_DISK) return false;
+    return p.precision == ARC_PREC_KAHAN || (p.precision == ARC_PREC_FP64 && !few_avpls(n, pixels));
 }
 
 dim3 tile_grid(const BfArgs& a, int px) {
@@ -976,6 +989,8 @@ arc_status launch_fast_path(const BfArgs& a, const ArcGatherParams& p, int px, c
         if (p.precision == ARC_PREC_FP64) return launch_fast<1, 3, 1>(a, st);
         return launch_fast_prec<1>(a, p.precision, px, st);
     }
+    if (p.precision == ARC_PREC_FP64)
+        return p.ar_kind == ARC_AR_NONE ? launch_fast<0, 3, 1>(a, st) : launch_fast<2, 3, 1>(a, st);
     return p.ar_kind == ARC_AR_NONE ? launch_fast_prec<0>(a, p.precision, px, st)
                                     : launch_fast_prec<2>(a, p.precision, px, st);
 }
@@ -1026,8 +1041,9 @@ arc_status launch_gather_bruteforce(arc_context* ctx, const GatherLaunch& g) {
     }
     ARC_TRY(pack_records(ctx, g, a));
     const int chosen = p.tile_config >= 0 ? p.tile_config : ctx->bf_tile_config;
-    if (use_culled(p)) return run_culled(ctx, a, p, chosen, true);
-    if (p.ar_kind == ARC_AR_DISK && p.precision == ARC_PREC_KAHAN) {
+    const int64_t pixels = (int64_t)gb.width * gb.height;
+    if (use_culled(p, a.n, pixels)) return run_culled(ctx, a, p, chosen, true);
+    if (p.ar_kind == ARC_AR_DISK && p.precision == ARC_PREC_KAHAN && !few_avpls(a.n, pixels)) {
         // the radiance by the culled gather, the antiradiance by the culled disk pass
         double *rad64 = nullptr, *ar64 = nullptr;
         const size_t bytes = (size_t)gb.height * out.pitch * 3 * sizeof(double);
@@ -1340,7 +1356,7 @@ extern "C" arc_status arc_gather_bruteforce_noalloc(void* cuda_stream, const Arc
             pack_bf_records<<<(a.n + 255) / 256, 256, 0, st>>>(*avpls, mats, num_materials, records, err);
             ARC_TRY_CUDA(cudaGetLastError());
         }
-        if (use_culled(p)) {  // one segment: there is no room for partial sums
+        if (use_culled(p, a.n, (int64_t)gb.width * gb.height)) {  // one segment: there is no room for partial sums
             CulledPlan c = culled_plan(a, p, p.tile_config, 1);
             c.segments = 1;
             ARC_TRY(launch_culled(a, p, c, st));
