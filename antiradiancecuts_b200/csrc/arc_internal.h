@@ -172,10 +172,11 @@ arc_status launch_run_clustered_antiradiance(arc_context* ctx, const ArcAvplsGpu
                                              const ArcClusterParams* cl, const ArcGatherParams* gp,
                                              const ArcOutputView* out);
 // disk antiradiance over every AVPL into out_ar (float4) and / or out_ar64 (3 doubles per pixel);
-// clustered: surface pixels and bad materials as arc_antiradiance_clustered treats them
-arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* avpls, const ArcGBufferView* gb,
-                                    const ArcGatherParams* gp, bool clustered, float* out_ar, double* out_ar64,
-                                    int64_t opitch);
+// clustered: surface pixels and bad materials as arc_antiradiance_clustered treats them; records: the
+// AVPLs' (launch_pack_records), packed here if NULL
+arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* avpls, const float4* records,
+                                    const ArcGBufferView* gb, const ArcGatherParams* gp, bool clustered, float* out_ar,
+                                    double* out_ar64, int64_t opitch);
 // result = radiance - antiradiance in FP64 (planes of 3 doubles per pixel at out's pitch) into out's
 // result, antiradiance and FP64 result planes; ar64 may be NULL
 arc_status launch_combine(arc_context* ctx, const double* rad64, const double* ar64, int width, int height,

@@ -353,8 +353,8 @@ extern "C" arc_status arc_antiradiance_clustered(arc_context* ctx, const ArcAvpl
     const int64_t slots = (int64_t)tiles * kCThreads;
     ARC_CHECK_ARG(slots < INT32_MAX, "image too large for the cluster slots");
     if (!info)  // nobody reads the clusters and their lists: the culled pass sums the same pairs
-        return launch_disk_antiradiance(ctx, avpls, gbuffer, params, true, out->antiradiance, out->result_fp64,
-                                        out->pitch);
+        return launch_disk_antiradiance(ctx, avpls, nullptr, gbuffer, params, true, out->antiradiance,
+                                        out->result_fp64, out->pitch);
     int *pixel_cluster, *tile_count, *counts, *offsets, *block_sums, *total;
     float4* box;
     ARC_TRY(ctx->arena.get("cl_pixel", (size_t)W * H * sizeof(int), reinterpret_cast<void**>(&pixel_cluster)));

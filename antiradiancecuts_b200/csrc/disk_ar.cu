@@ -399,11 +399,10 @@ __global__ void __launch_bounds__(kThreads) disk_combine(DiskArgs a, int segment
 
 }  // namespace
 
-arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* avpls, const ArcGBufferView* gb,
-                                    const ArcGatherParams* gp, bool clustered, float* out_ar, double* out_ar64,
-                                    int64_t opitch) {
-    const float4* records = nullptr;
-    ARC_TRY(launch_pack_records(ctx, avpls, &records));
+arc_status launch_disk_antiradiance(arc_context* ctx, const ArcAvplsGpuParam* avpls, const float4* records,
+                                    const ArcGBufferView* gb, const ArcGatherParams* gp, bool clustered, float* out_ar,
+                                    double* out_ar64, int64_t opitch) {
+    if (!records) ARC_TRY(launch_pack_records(ctx, avpls, &records));
     DiskArgs a{};
     a.records = records;
     a.n = avpls->numAvpls;

@@ -1054,7 +1054,7 @@ arc_status launch_gather_bruteforce(arc_context* ctx, const GatherLaunch& g) {
         a.out_res = a.out_ar = nullptr;
         a.out_res64 = rad64;
         ARC_TRY(run_culled(ctx, a, q, chosen, true));
-        ARC_TRY(launch_disk_antiradiance(ctx, g.avpls, &gb, &p, false, nullptr, ar64, out.pitch));
+        ARC_TRY(launch_disk_antiradiance(ctx, g.avpls, a.records, &gb, &p, false, nullptr, ar64, out.pitch));
         return launch_combine(ctx, rad64, ar64, gb.width, gb.height, &out);
     }
     const TileShape ts = kTileShapes[chosen >= 0 ? chosen : kDefaultTileShape];
@@ -1083,7 +1083,7 @@ arc_status launch_pack_records(arc_context* ctx, const ArcAvplsGpuParam* avpls, 
 arc_status launch_antiradiance_only(arc_context* ctx, const GatherLaunch& g, double* ar64) {
     const ArcGatherParams& p = *g.params;
     if (p.ar_kind == ARC_AR_DISK)
-        return launch_disk_antiradiance(ctx, g.avpls, g.gbuffer, &p, false, nullptr, ar64, g.out->pitch);
+        return launch_disk_antiradiance(ctx, g.avpls, nullptr, g.gbuffer, &p, false, nullptr, ar64, g.out->pitch);
     BfArgs a = make_args(ctx, g);
     a.out_res = nullptr;
     a.out_rad = nullptr;
