@@ -474,8 +474,10 @@ typedef struct ArcRunConfig {
     float mlp_threshold;
     float mlp_band;
     int64_t cut_pool_entries;
-    /* useClusteredDeferred (cudaGather.cu:948-1031): the disk antiradiance through screen clusters
-     * (arc_antiradiance_clustered) instead of brute force; with ar_kind ARC_AR_DISK only */
+    /* useClusteredDeferred (cudaGather.cu:948-1031): the disk antiradiance from
+     * arc_antiradiance_clustered without cluster arrays, in a pass after the radiance; with ar_kind
+     * ARC_AR_DISK only.  No cluster is built: cluster_z_near and cluster_theta are checked and do not
+     * change the image */
     int32_t useClusteredDeferred;
     float cluster_z_near; /* ArcClusterParams.z_near */
     float cluster_theta;  /* ArcClusterParams.theta */
@@ -550,8 +552,8 @@ typedef struct ArcClusterParams {
     float theta;  /* cameraTheta: half the vertical field of view, radians */
 } ArcClusterParams;
 
-/* Device arrays of the last arc_antiradiance_clustered call on the context (valid until the
- * next call): pixel_cluster[height * width] (cluster slot or -1: no surface); box[slot][8]
+/* Device arrays of the last arc_antiradiance_clustered call on the context that asked for them
+ * (info not NULL; valid until the next such call): pixel_cluster[height * width] (cluster slot or -1: no surface); box[slot][8]
  * ({min, 0}, {max, 0}); tile_count[tile] (clusters of the tile, in slots tile * slots_per_tile
  * ...); counts[slot] (AVPLs in the cluster's list) and lists (every list in slot order, each in
  * AVPL order: the list of slot s starts at the sum of counts[0 .. s-1]). */
@@ -566,13 +568,16 @@ typedef struct ArcClusterInfo {
     int64_t list_entries;
 } ArcClusterInfo;
 
-/* Disk antiradiance through screen clusters and their light lists (kernel_gather_cluster_lights +
- * kernel_antiradiance_clusterred, cudaGather.cu:605-748): the AVPLs of a pixel's cluster are
- * those whose ray (position, incDirection) meets the cluster box grown by twice the disk radius,
- * which holds every AVPL whose disk antiradiance reaches the cluster's pixels, so the result is
- * the brute-force disk antiradiance up to summation order.  Writes out->antiradiance (float4,
- * w = 1) and, when set, out->result_fp64 (3 doubles per pixel: the antiradiance in FP64); other
- * planes are untouched.  params: ar_kind ARC_AR_DISK with disk_radius > 0.  info may be NULL. */
+/* Disk antiradiance of clustered deferred shading (kernel_gather_cluster_lights +
+ * kernel_antiradiance_clusterred, cudaGather.cu:605-748).  With info: through screen clusters and
+ * their light lists, which info then names; the AVPLs of a pixel's cluster are those whose ray
+ * (position, incDirection) meets the cluster box grown by twice the disk radius, which holds every
+ * AVPL whose disk antiradiance reaches the cluster's pixels, so the result is the brute-force disk
+ * antiradiance up to summation order.  With info NULL: the same sums without clusters, from a pass
+ * that culls the AVPLs per pixel tile; cparams is checked as with info and otherwise unused.  Writes
+ * out->antiradiance (float4, w = 1) and, when set, out->result_fp64 (3 doubles per pixel: the
+ * antiradiance in FP64); other planes are untouched.  params: ar_kind ARC_AR_DISK with
+ * disk_radius > 0. */
 arc_status arc_antiradiance_clustered(arc_context* ctx, const ArcAvplsGpuParam* avpls, const ArcGBufferView* gbuffer,
                                       ArcFloat3 camera_position, const ArcClusterParams* cparams,
                                       const ArcGatherParams* params, const ArcOutputView* out, ArcClusterInfo* info);
