@@ -39,9 +39,10 @@ static_assert(kCounts <= 32, "one lane per count in the block's prefix sum");
 // 32 x 32 tiles when they make at least this many blocks per SM (a quarter of the ray tests; 1280 x 720 x
 // 65,536: 0.55 against 0.99 ms), else 16 x 16 (more, smaller blocks).
 constexpr int64_t kBigTilesPerSm = 2;
-// Segments: blocks per SM at which the AVPLs are no longer split (512 x 512 x 32,768 / 1280 x 720 x 65,536:
-// 0.28 / 0.64 ms at 8 per SM, 0.28 / 0.55 ms at 16, 0.29 / 0.51 ms at 32: the blocks' set-up against their
-// balance), partial sums within kPartialBytes.
+// Segments: blocks per SM at which the AVPLs are no longer split, the blocks' set-up against their balance
+// (512 x 512 x 32,768 / 1280 x 720 x 65,536 / 1920 x 1080 x 65,536 in ms: 0.284 / 0.640 / 1.143 at 8 per SM,
+// 0.285 / 0.560 / 0.948 at 16, 0.290 / 0.533 / 0.948 at 24, 0.298 / 0.527 / 0.910 at 32, 0.319 / 0.538 / 0.916 at
+// 48), partial sums within kPartialBytes.
 constexpr int64_t kBlocksPerSm = 24;
 constexpr int64_t kPartialBytes = (int64_t)1 << 30;
 

@@ -15,8 +15,8 @@
 //     culled pass of its own (disk_ar.cu); the other precisions, every disk gather of the
 //     allocation-free entry point, and gathers of few AVPLs (few_avpls) evaluate every pair
 //     (gather_bf_kernel).
-//   * Radiance and antiradiance go to separate compensated sums (per-chunk FP32 partials folded
-//     into Kahan sums, or per-term Kahan) and are combined in FP64.
+//   * Radiance and antiradiance go to separate sums (culled: per-chunk FP32 partials folded into
+//     FP64; every pair: into Kahan sums, or per-term Kahan) and are combined in FP64.
 // General path (specular materials or geometry-term limits): one thread per pixel evaluating the
 // full f_r on both sides of every pair.
 #include <algorithm>
@@ -343,13 +343,14 @@ __device__ __forceinline__ void write_pixel(const BfArgs& k, int x, int y, int m
 // the warps that hold some run the pair loops, and where they are half of the block's warps or fewer the
 // rest take the same pixels over every second, fourth or eighth pair of records (the block adds their sums
 // in FP64).  With all pixels evaluated a tile costs the same whatever its surface: 960 x 540 x 131,072 AVPLs
-// with 1%, 5%, 20% and 50% of scattered surface pixels 42.9, 50.3, 50.9 and 51.1 ms, now 5.2, 6.1, 15.6 and
-// 39.5 ms (a kernel over a list of the surface pixels that tests no records: 12.2, 12.2, 23.9 and 47.4 ms).
+// with 1%, 5%, 20% and 50% of scattered surface pixels 42.9, 50.3, 50.9 and 51.1 ms, now 5.2, 6.2, 15.7 and
+// 39.9 ms (a kernel over a list of the surface pixels that tests no records: 12.2, 12.2, 23.9 and 47.4 ms).
 // Above half the tile's two pixels per thread share each record's loads.
 //
-// Bound by the FMA pipe: 18 packed FP32x2 operations per two radiance pairs (70% of the pipe's cycles,
-// 16.3 instructions per evaluated pair).  1920 x 1080 x 262,144 AVPLs, cone 60 degrees: 138 ms, 352 ms for
-// the kernel that evaluated every pair; all FP64, 637 x 359 x 16,381: 3.6 against 20.3 ms.
+// Bound by the FMA pipe: 18 packed FP32x2 operations per two radiance pairs (69% of the pipe's cycles,
+// 16.3 instructions per evaluated pair).  1920 x 1080 x 262,144 AVPLs, cone 60 degrees: 133 ms (138 ms before
+// the warps without a surface pixel left the pairs out), 352 ms for the kernel that evaluated every pair;
+// all FP64, 637 x 359 x 16,381: 3.5 against 20.3 ms.
 // ---------------------------------------------------------------------------------------
 // staged records | the two lists | FP32: the threads' FP64 sums (their registers hold the pixels and
 // the pair loop's operands instead) | mbarrier
@@ -866,7 +867,11 @@ constexpr int kFp64Chunk = 256;
 // Segments of the culled gather: enough blocks for several waves of resident ones (a grid of one
 // partial wave leaves SMs idle: 64 x 64 x 4,096 takes 269 us in one segment and 59 us split, 640 x 360 x
 // 16,384 2.14 and 1.30 ms), each segment at least kMinChunks chunks long (a block's set-up -- pixel
-// loads, tile bounds -- costs about a chunk), partial sums within kPartialBytes.
+// loads, tile bounds -- costs about a chunk), partial sums within kPartialBytes.  Measured:
+//   blocks per SM 6 / 12 / 24 / 48: 640 x 360 x 16,384 1.39 / 1.17 / 1.10 / 1.10 ms, 1280 x 720 x 65,536 16.5 /
+//     16.7 / 15.1 / 14.4 ms, 1920 x 1080 x 262,144 123.0 / 123.1 / 122.7 / 120.2 ms, smaller ones the same;
+//   chunks per segment 1 / 2 / 4: 64 x 64 x 4,096 60 / 71 / 103 us, 256 x 256 x 4,096 204 / 196 / 218 us, larger
+//     ones the same.
 constexpr int kBlocksPerSm = 24;
 constexpr int kMinChunks = 2;
 constexpr int64_t kPartialBytes = (int64_t)1 << 30;
